@@ -26,6 +26,7 @@
 // Nothing is read back to the host inside a step.
 #include "lare_solver.cuh"
 #include "lare_ops.cuh"
+#include "lare_march.cuh"
 #include "lare_bc.cuh"
 #include "lare_geom_host.h"
 
@@ -56,447 +57,71 @@ __global__ void __launch_bounds__(kThreads, (MinBlocks<Op, P2>::value)) k_op(Ctx
     for (int i = lo[0] + (int)blockIdx.y; i <= hi[0]; i += gridDim.y) Op::template run<GEO, P2>(c, arg, i, j, k);
 }
 
-// The z sweep's stages S6, S7 and S8 (ops::SweepFused<2>) over whole z
-// lines: a block holds kZThreads / (nz + 4) lines of (i, j) in 0..nx x
-// 0..ny, one thread per k = -2..nz+1 of each.
-constexpr int kZThreads = ops::kZLineThreads;
+// The fused kernels (bodies in lare_march.cuh), one block of the phase per
+// CUDA block.
+using march::kMThreads;
+using march::kRP;
+using march::kZThreads;
+using march::MarchTile;
+using march::PrepMarch;
+using march::VolMarch;
+using march::WinTile;
+using march::ZTile;
 
-// ct_arg >= 0: each point of 0..n also takes the z sweep's CT update of B
-// (SweepCTUpd<2> with that argument), which nothing else in the kernel reads
-// or writes.
+template <bool GEO, bool P2, int CW>
+__global__ void __launch_bounds__(kMThreads, 3) k_pred_march(Ctx c, MarchTile m, int resistive, double *pe_out, double *pi_out)
+{
+    extern __shared__ double ring[];
+    march::pred<GEO, P2, CW>(c, m, (int)blockIdx.x, resistive, pe_out, pi_out, ring);
+}
+
+template <class P, bool GEO, bool P2, int CW>
+__global__ void __launch_bounds__(kMThreads, P::kMinBlocks) k_cellnode_march(Ctx c, MarchTile m, int arg)
+{
+    extern __shared__ double ring[];
+    march::cellnode<P, GEO, P2, CW>(c, m, (int)blockIdx.x, arg, ring);
+}
+
+template <bool GEO, bool P2, int CW>
+__global__ void __launch_bounds__(kMThreads, march::kHeatMinBlocks) k_heat_march(Ctx c, MarchTile m)
+{
+    extern __shared__ double ring[];
+    march::heat_edges<GEO, P2, CW>(c, m, (int)blockIdx.x, ring);
+}
+
+template <bool GEO, bool P2, int CW>
+__global__ void __launch_bounds__(kMThreads, 5) k_resist_march(Ctx c, MarchTile m, double *nbx, double *nby, double *nbz)
+{
+    extern __shared__ double ring[];
+    march::resist<GEO, P2, CW>(c, m, (int)blockIdx.x, nbx, nby, nbz, ring);
+}
+
+template <int DIR, bool GEO>
+__global__ void __launch_bounds__(ops::kWinThreads, 5) k_ctmass(Ctx c, WinTile w, int scale, int images)  // cap tuned on B200
+{
+    extern __shared__ double csm[];
+    march::ctmass<DIR, GEO>(c, w, (int)blockIdx.x, scale, images, csm);
+}
+
+template <bool GEO>
+__global__ void __launch_bounds__(march::kZCtThreads, 4) k_ctmass_z(Ctx c, ZTile z, int images)
+{
+    __shared__ double zsm[ops::SweepCTMass<2>::NARR * march::kZCtThreads];
+    march::ctmass_z<GEO>(c, z, (int)blockIdx.x, images, zsm);
+}
+
+template <int DIR, bool GEO>
+__global__ void __launch_bounds__(ops::kWinThreads, 4) k_psweep(Ctx c, WinTile wt, ops::SweepOut w, int ct_arg)  // window shape and cap tuned on B200
+{
+    extern __shared__ double psm[];
+    march::psweep<DIR, GEO>(c, wt, (int)blockIdx.x, w, ct_arg, psm);
+}
+
 template <bool GEO>
 __global__ void __launch_bounds__(kZThreads, 5) k_zsweep(Ctx c, int ct_arg)  // 5 blocks per SM, tuned on B200
 {
-    using F = ops::SweepFused<2>;
     extern __shared__ double zsm[];
-    static_assert(!F::kSharedFluxSlots, "the z passes of stage B run without a barrier between them");
-    const Geom &g = c.g;
-    const int W = g.nz + 4, lines = kZThreads / W, S = lines * W;
-    const int line = (int)threadIdx.x / W, k = (int)threadIdx.x % W - 2;
-    const long long q = (long long)blockIdx.x * lines + line;
-    const bool on = line < lines && q < (long long)(g.nx + 1) * (g.ny + 1);
-    const int i = on ? (int)(q / (g.ny + 1)) : 0, j = on ? (int)(q % (g.ny + 1)) : 0;
-    const ops::LineStore st{zsm, S, line * W + k + 2};
-    const ops::SweepOut w = ops::sweep_in_place(c);
-    if (on) F::stage_a<GEO>(c, i, j, k, st, w, true);
-    __syncthreads();
-    if (on && k >= 1 && k <= g.nz) F::stage_b_energy(c, i, j, k, st, w);
-    if (on && k >= -1 && k <= g.nz) F::stage_b_mom<GEO>(c, i, j, k, st);  // its own slots: no barrier between
-    __syncthreads();
-    if (on && k >= 0 && k <= g.nz) F::stage_c(c, i, j, k, st, w);
-    if (ct_arg >= 0 && on && k >= 0 && k <= g.nz) ops::SweepCTUpd<2>::run<GEO, false>(c, ct_arg, i, j, k);
-}
-
-// The x or y sweep's stages (ops::SweepFused<DIR>) out of place, over
-// windows of kWinK adjacent k in 0..nz times kWinS own points along DIR, for
-// one value of the third index (j for x, i for y) in 0..n.  The solve's
-// state arrays are only read; the new rho, energies and velocities go to w.
-// Halo points recompute stage A (two before, one after) and stage B (one
-// before) without writing the state.  ct_arg >= 0: each own point (0..n in
-// every dimension) also takes the sweep's CT update of B (SweepCTUpd<DIR>
-// with that argument); no stage reads B.
-template <int DIR, bool GEO>
-__global__ void __launch_bounds__(ops::kWinThreads, 4) k_psweep(Ctx c, ops::SweepOut w, int ct_arg)  // window shape and cap tuned on B200
-{
-    using F = ops::SweepFused<DIR>;
-    constexpr int TK = ops::kWinK, TS = ops::kWinThreads / ops::kWinK;
-    extern __shared__ double psm[];
-    const Geom &g = c.g;
-    const int nd = DIR == 0 ? g.nx : g.ny;
-    const int nkt = (g.nz + TK) / TK, nwin = (nd + ops::kWinS) / ops::kWinS;
-    const int b = (int)blockIdx.x;
-    const int win = b % nwin, kt = (b / nwin) % nkt, a = b / (nwin * nkt);
-    const int s0 = win * ops::kWinS, s1 = min(s0 + ops::kWinS - 1, nd);  // own points
-    const int kc = (int)threadIdx.x % TK, sl = (int)threadIdx.x / TK;
-    const int k = kt * TK + kc;
-    const bool on = k <= g.nz;
-    auto at = [&](int s) { return ops::WinStore{psm, s - s0 + 2, kc}; };
-    const int a_lo = max(s0 - 2, -2), a_hi = min(s1 + 1, nd + 1);
-    for (int s = a_lo + sl; s <= a_hi; s += TS)
-        if (on) F::template stage_a<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), w, s >= s0 && s <= s1);
-    __syncthreads();
-    for (int s = s0 + sl; s <= s1; s += TS)
-        if (on) F::stage_b_energy(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), w);
-    __syncthreads();
-    const int b_lo = max(s0 - 1, -1);
-    for (int s = b_lo + sl; s <= s1; s += TS)
-        if (on) F::template stage_b_mom<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s));
-    __syncthreads();
-    for (int s = s0 + sl; s <= s1; s += TS)
-        if (on) F::stage_c(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), w);
-    if (ct_arg >= 0)
-        for (int s = s0 + sl; s <= s1; s += TS)
-            if (on) ops::SweepCTUpd<DIR>::template run<GEO, false>(c, ct_arg, DIR == 0 ? s : a, DIR == 0 ? a : s, k);
-}
-
-// The predictor (ops::Pred1 then ops::Pred2) in one kernel.  A block owns
-// kMK x kMJ nodes of a y-z plane (k fastest) and a chunk of kMI planes along
-// x, and marches along x: for each plane i it computes Pred1 for the cells of
-// plane i+1 that its nodes read (its kMJ+1 x kMK+1 cells: the +1 halo in y
-// and z is recomputed by the neighbouring block too) into a ring of three
-// planes in shared memory, then Pred2 for its nodes of plane i from the
-// ring.  cv1 and the half-step B never go to global memory.  The half-step
-// p_e and p_i of the block's own cells go to pe_out / pi_out: in resistive
-// runs Pred1 reads the step-start p_e / p_i at cells that other blocks own,
-// so those arrays cannot be overwritten in place.
-// The ring plane is (kMK+1) x (kMJ+1) cells, one per thread of a block of
-// kMThreads: 32 x 9, nine full warps, so the producer is one pass; the
-// consumer maps thread t to (t / (kMK+1), t % (kMK+1)) and leaves the last
-// lane of each row and the last row idle.
-constexpr int kMK = 31, kMJ = 8, kMI = 16;
-constexpr int kRP = (kMK + 1) * (kMJ + 1);  // cells of one ring plane
-constexpr int kMThreads = (kRP + 31) / 32 * 32;
-
-struct RingSrc {
-    const double *ring;
-    __device__ double operator()(int arr, int q) const { return ring[arr * 3 * kRP + q]; }
-};
-// The predictor's ring: Pred1's outputs with p_e + p_i in the PE slot (Pred2
-// reads only that sum), five arrays.
-struct PredRingSrc {
-    static constexpr bool kPressureSum = true;
-    static constexpr int NR = ops::Pred1::PI;  // CV1, B1X, B1Y, B1Z, PE (= p_e + p_i)
-    const double *ring;
-    __device__ double operator()(int arr, int q) const { return ring[arr * 3 * kRP + q]; }
-};
-
-template <bool GEO, bool P2>
-__global__ void __launch_bounds__(kMThreads, 3) k_pred_march(Ctx c, int resistive, double *pe_out, double *pi_out)
-{
-    using P1 = ops::Pred1;
-    extern __shared__ double ring[];  // [PredRingSrc::NR][3 planes][kRP]
-    const Geom &g = c.g;
-    const int nkt = (g.nz + kMK) / kMK, njt = (g.ny + kMJ) / kMJ;  // tiles over nodes 0..n
-    int b = (int)blockIdx.x;
-    const int tk = b % nkt;
-    b /= nkt;
-    const int tj = b % njt;
-    const int i0 = (b / njt) * kMI, i1 = min(i0 + kMI - 1, g.nx);
-    const int k0 = tk * kMK, j0 = tj * kMJ;
-    const int t = (int)threadIdx.x;
-    // Pred1 at the block's cells of plane i (cells 0..n+1: what Pred2 reads)
-    auto produce = [&](int i) {
-        const int slot = i % 3;
-        for (int p = t; p < kRP; p += kMThreads) {
-            const int pj = p / (kMK + 1), pk = p - pj * (kMK + 1);
-            const int j = j0 + pj, k = k0 + pk;
-            if (j > g.ny + 1 || k > g.nz + 1) continue;
-            double out[P1::NOUT];
-            bool half_p;
-            P1::compute<GEO, P2>(c, resistive, i, j, k, out, half_p);
-#pragma unroll
-            for (int a = 0; a < P1::PE; ++a) ring[(a * 3 + slot) * kRP + p] = out[a];
-            ring[(P1::PE * 3 + slot) * kRP + p] = out[P1::PE] + out[P1::PI];
-            if (pj < kMJ && pk < kMK && i <= i1 && j <= g.ny && k <= g.nz) {
-                const int o = box_off(g, i, j, k);
-                pe_out[o] = out[P1::PE];
-                pi_out[o] = out[P1::PI];
-            }
-        }
-    };
-    const int kc = t % (kMK + 1), jc = t / (kMK + 1);
-    const int j = j0 + jc, k = k0 + kc;
-    const bool on = kc < kMK && jc < kMJ && j <= g.ny && k <= g.nz;
-    const PredRingSrc src{ring};
-    produce(i0);
-    for (int i = i0; i <= i1; ++i) {
-        produce(i + 1);
-        __syncthreads();  // the ring's planes i and i+1 are complete
-        if (on) {
-            const int s0 = i % 3, s1 = (i + 1) % 3;
-            ops::Pred2::run_src<GEO, P2>(c, i, j, k, src, s0 * kRP + jc * (kMK + 1) + kc, (s1 - s0) * kRP, kMK + 1, 1);
-        }
-        // three ring planes: the next iteration's producer writes the plane
-        // this one read as i-1, which no thread reads after this barrier
-    }
-}
-
-// A cell op feeding a node op that reads it at the node's eight cells, in
-// one kernel: the same march as k_pred_march over nodes -1..n+1 of every
-// dimension, with the cell op over cells -1..n+2.  P::produce computes a
-// cell's ring values (P::NR of them) and, where `own`, stores its outputs
-// (each cell is owned by one block: a chunk, row or column holds its own
-// cells and, at the grid's upper end, the +1 halo cell too);
-// P::consume runs the node op from the ring.
-template <class P, bool GEO, bool P2>
-__global__ void __launch_bounds__(kMThreads, P::kMinBlocks) k_cellnode_march(Ctx c, int arg)
-{
-    extern __shared__ double ring[];  // [P::NR][3 planes][kRP]
-    const Geom &g = c.g;
-    const int nkt = (g.nz + 2 + kMK) / kMK, njt = (g.ny + 2 + kMJ) / kMJ;  // tiles over nodes -1..n+1
-    int b = (int)blockIdx.x;
-    const int tk = b % nkt;
-    b /= nkt;
-    const int tj = b % njt;
-    const int i0 = -1 + (b / njt) * kMI, i1 = min(i0 + kMI - 1, g.nx + 1);
-    const int k0 = -1 + tk * kMK, j0 = -1 + tj * kMJ;
-    const int t = (int)threadIdx.x;
-    auto produce = [&](int i) {
-        const int slot = (i + 3) % 3;
-        for (int p = t; p < kRP; p += kMThreads) {
-            const int pj = p / (kMK + 1), pk = p - pj * (kMK + 1);
-            const int j = j0 + pj, k = k0 + pk;
-            if (j > g.ny + 2 || k > g.nz + 2) continue;
-            const bool own = (pj < kMJ || j == g.ny + 2) && (pk < kMK || k == g.nz + 2) && (i <= i1 || i == g.nx + 2);
-            double out[P::NR];
-            P::template produce<GEO, P2>(c, arg, i, j, k, own, out);
-#pragma unroll
-            for (int a = 0; a < P::NR; ++a) ring[(a * 3 + slot) * kRP + p] = out[a];
-        }
-    };
-    const int kc = t % (kMK + 1), jc = t / (kMK + 1);
-    const int j = j0 + jc, k = k0 + kc;
-    const bool on = kc < kMK && jc < kMJ && j <= g.ny + 1 && k <= g.nz + 1;
-    const RingSrc src{ring};
-    produce(i0);
-    for (int i = i0; i <= i1; ++i) {
-        produce(i + 1);
-        __syncthreads();  // the ring's planes i and i+1 are complete
-        if (on) {
-            const int s0 = (i + 3) % 3, s1 = (i + 4) % 3;
-            P::template consume<GEO, P2>(c, arg, i, j, k, src, s0 * kRP + jc * (kMK + 1) + kc, (s1 - s0) * kRP,
-                                         kMK + 1, 1);
-        }
-    }
-}
-
-// CellPrep + NodePrep: each cell's rho and sound speed go into the ring for
-// the node averages, so cs never goes to global memory; in resistive runs
-// (arg 1) the cell's step-start p_e, p_i are stored.
-struct PrepMarch {
-    static constexpr int NR = 2, kMinBlocks = 5;  // register cap tuned on B200
-    template <bool GEO, bool P2>
-    __device__ static void produce(const Ctx &c, int resistive, int i, int j, int k, bool own, double *out)
-    {
-        const int o = box_off(c.g, i, j, k);
-        double pe, pi;
-        out[1] = ops::CellPrep::sound_speed(c, o, out[0], pe, pi);
-        if (resistive && own) {
-            c.s[S_PE][o] = pe;
-            c.s[S_PI][o] = pi;
-        }
-    }
-    template <bool GEO, bool P2, class S>
-    __device__ static void consume(const Ctx &c, int, int i, int j, int k, const S &src, int q0, int QX, int QY, int QZ)
-    {
-        ops::NodePrep::run_src<GEO, P2>(c, i, j, k, src, q0, QX, QY, QZ);
-    }
-};
-
-// SweepVol + SweepCvc of one sweep: cv1 goes into the ring for the node
-// volumes cvc1.
-template <int DIR>
-struct VolMarch {
-    static constexpr int NR = 1, kMinBlocks = DIR == 2 ? 5 : 4;  // register cap tuned on B200
-    template <bool GEO, bool P2>
-    __device__ static void produce(const Ctx &c, int arg, int i, int j, int k, bool own, double *out)
-    {
-        out[0] = ops::SweepVol<DIR>::template compute<GEO, P2>(c, arg, i, j, k, own);
-    }
-    template <bool GEO, bool P2, class S>
-    __device__ static void consume(const Ctx &c, int, int i, int j, int k, const S &src, int q0, int QX, int QY, int QZ)
-    {
-        ops::SweepCvc::node(c, box_off(c.g, i, j, k), src, q0, QX, QY, QZ);
-    }
-};
-
-// An edge term feeding a cell op that reads it on twelve edges around the
-// cell, in one kernel (used for the shock heating, whose twelve products of
-// velocity jumps per cell, lagran.cpp:888-979, are terms of the edges
-// between the cell's corner nodes).  Each term is formed once, at the node
-// where its edge ends, instead of once for each of the four cells that share
-// the edge.  The march of k_pred_march over cells 0..n+1: for each plane i
-// the block forms the x, y and z edge terms of the nodes of plane i that its
-// cells read (rows j0-1 .. j0+kMJ-1, kMK+1 columns from k0 + P::KOFF) into a
-// ring of three planes in shared memory, then runs the cell op for its cells
-// of plane i from the ring's planes i-1 and i.
-template <class P, bool GEO, bool P2>
-__global__ void __launch_bounds__(kMThreads, (P2 ? P::kMinBlocksP2 : P::kMinBlocks)) k_edge_march(Ctx c)
-{
-    extern __shared__ double ring[];  // [3 edge directions][3 planes][kRP]
-    const Geom &g = c.g;
-    const int nkt = (g.nz + 1 + kMK) / kMK, njt = (g.ny + 1 + kMJ) / kMJ;  // tiles over cells 0..n+1
-    int b = (int)blockIdx.x;
-    const int tk = b % nkt;
-    b /= nkt;
-    const int tj = b % njt;
-    const int i0 = (b / njt) * kMI, i1 = min(i0 + kMI - 1, g.nx + 1);
-    const int k0 = tk * kMK, j0 = tj * kMJ;
-    const int t = (int)threadIdx.x;
-    const int kmax = g.nz + 2 + P::KOFF;  // last node column the cells read
-    auto produce = [&](int i) {
-        const int slot = (i + 3) % 3;
-        for (int p = t; p < kRP; p += kMThreads) {
-            const int pj = p / (kMK + 1), pk = p - pj * (kMK + 1);
-            const int j = j0 - 1 + pj, k = k0 + P::KOFF + pk;
-            if (j > g.ny + 1 || k > kmax) continue;
-            double e[3];
-            P::Op::node_edges(c, box_off(g, i, j, k), e);
-#pragma unroll
-            for (int a = 0; a < 3; ++a) ring[(a * 3 + slot) * kRP + p] = e[a];
-        }
-    };
-    const int kc = t % (kMK + 1), jc = t / (kMK + 1);
-    const int j = j0 + jc, k = k0 + kc;
-    const bool on = kc < kMK && jc < kMJ && j <= g.ny + 1 && k <= g.nz + 1;
-    const RingSrc src{ring};
-    produce(i0 - 1);
-    for (int i = i0; i <= i1; ++i) {
-        produce(i);
-        __syncthreads();  // the ring's planes i-1 and i are complete
-        if (on) {
-            const int s0 = (i + 3) % 3, sm = (i + 2) % 3;
-            double a[12];
-            P::Op::ring_edges(src, s0 * kRP + (jc + 1) * (kMK + 1) + (kc - P::KOFF), (s0 - sm) * kRP, kMK + 1, a);
-            P::template finish<GEO, P2>(c, i, j, k, a);
-        }
-        // three ring planes: the next iteration's producer writes the plane
-        // this one read as i-2, which no thread reads any more
-    }
-}
-
-// Corr1 from the ring of products of velocity jumps: the shock heating.
-// (Corr2's energy and density update folded in here, with only its velocity
-// update left as a kernel, measured slower on B200: 0.83 + 0.25 ms against
-// 0.43 + 0.60.)
-struct HeatEdges {
-    using Op = ops::Corr1;
-    static constexpr int KOFF = 0, kMinBlocks = 4, kMinBlocksP2 = 4;  // register cap tuned on B200
-    template <bool GEO, bool P2>
-    __device__ static void finish(const Ctx &c, int i, int j, int k, const double *a)
-    {
-        c.s[S_VH][box_off(c.g, i, j, k)] = Op::heating_finish<GEO, P2>(c, i, j, k, a);
-    }
-};
-
-// One resistive sub-step (ops::ResistRK then ops::ResistB) in one kernel,
-// out of place for B.  A block owns kMK x kMJ points of a y-z plane of the
-// whole box (-2..n+2) and a chunk of kMI planes along x, and marches along x:
-// ResistRK for the cells of plane i that its points read (the -1 halo in y
-// and z is recomputed by the neighbouring block) goes into a ring of three
-// planes in shared memory, then ResistB for its points of plane i reads the
-// ring's planes i-1 and i.  ResistRK reads B at +1 neighbours that other
-// blocks update, so the new B goes to nbx/nby/nbz (every box point: updated
-// or copied); the electron energy is updated in place (nothing else reads
-// it here).
-template <bool GEO, bool P2>
-__global__ void __launch_bounds__(kMThreads, 5) k_resist_march(Ctx c, double *nbx, double *nby, double *nbz)
-{
-    using RK = ops::ResistRK;
-    extern __shared__ double ring[];  // [RK::NOUT][3 planes][kRP]
-    const Geom &g = c.g;
-    const int nkt = (g.nz + 4 + kMK) / kMK, njt = (g.ny + 4 + kMJ) / kMJ;  // tiles over -2..n+2
-    int b = (int)blockIdx.x;
-    const int tk = b % nkt;
-    b /= nkt;
-    const int tj = b % njt;
-    const int i0 = -2 + (b / njt) * kMI, i1 = min(i0 + kMI - 1, g.nx + 2);
-    const int k0 = -2 + tk * kMK, j0 = -2 + tj * kMJ;
-    const int t = (int)threadIdx.x;
-    // ResistRK at the block's cells of plane i (ring index (j - j0 + 1, k - k0 + 1)),
-    // where it is defined (0..n)
-    auto produce = [&](int i) {
-        if (i < 0 || i > g.nx) return;
-        const int slot = (i + 6) % 3;
-        for (int p = t; p < kRP; p += kMThreads) {
-            const int pj = p / (kMK + 1), pk = p - pj * (kMK + 1);
-            const int j = j0 - 1 + pj, k = k0 - 1 + pk;
-            if (j < 0 || j > g.ny || k < 0 || k > g.nz) continue;
-            double out[RK::NOUT];
-            RK::compute<GEO, P2>(c, i, j, k, out);
-#pragma unroll
-            for (int a = 0; a < RK::NOUT; ++a) ring[(a * 3 + slot) * kRP + p] = out[a];
-        }
-    };
-    const int kc = t % (kMK + 1), jc = t / (kMK + 1);
-    const int j = j0 + jc, k = k0 + kc;
-    const bool on = kc < kMK && jc < kMJ && j <= g.ny + 2 && k <= g.nz + 2;
-    const RingSrc src{ring};
-    produce(i0 - 1);
-    for (int i = i0; i <= i1; ++i) {
-        produce(i);
-        __syncthreads();  // the ring's planes i-1 and i are complete
-        if (on) {
-            const int s0 = (i + 6) % 3, sm = (i + 5) % 3;
-            ops::ResistB::run_src<P2>(c, i, j, k, src, s0 * kRP + (jc + 1) * (kMK + 1) + (kc + 1), (s0 - sm) * kRP,
-                                      kMK + 1, 1, nbx, nby, nbz);
-        }
-    }
-}
-
-// SweepCT + SweepMass of the x or y sweep (ops::SweepCTMass<DIR>) over
-// windows of kWinK adjacent k times kWinS own points along DIR, for one value
-// a of the third index (j for x, i for y).  The CT quotients of the window's
-// points and of a halo of one before and two after go to shared memory first.
-// CT fluxes where a and k are in 0..n, mass fluxes where they are in 0..n+1.
-constexpr int kCtS = 21;              // own points of a window along the sweep (tuned on B200)
-constexpr int kCtP = kCtS + 3;         // with the quotient halo (one before, two after)
-struct CtStore {
-    double *sm;
-    int at, kc;
-    __device__ double get(int a, int ds) const { return sm[(a * kCtP + at + ds) * ops::kWinK + kc]; }
-    __device__ void put(int a, double v) const { sm[(a * kCtP + at) * ops::kWinK + kc] = v; }
-};
-
-template <int DIR, bool GEO>
-__global__ void __launch_bounds__(ops::kWinThreads, 5) k_ctmass(Ctx c, int scale, int images)  // cap tuned on B200
-{
-    using F = ops::SweepCTMass<DIR>;
-    constexpr int TK = ops::kWinK, TS = ops::kWinThreads / ops::kWinK;
-    extern __shared__ double csm[];
-    const Geom &g = c.g;
-    const int nd = DIR == 0 ? g.nx : g.ny, na = DIR == 0 ? g.ny : g.nx;
-    const int nkt = (g.nz + 1 + TK) / TK, nwin = (nd + kCtS) / kCtS;
-    const int b = (int)blockIdx.x;
-    const int win = b % nwin, kt = (b / nwin) % nkt, a = b / (nwin * nkt);
-    const int s0 = win * kCtS, s1 = min(s0 + kCtS - 1, nd);
-    const int kc = (int)threadIdx.x % TK, sl = (int)threadIdx.x / TK;
-    const int k = kt * TK + kc;
-    const bool ct = a <= na && k <= g.nz, mass = k <= g.nz + 1;
-    auto at = [&](int s) { return CtStore{csm, s - s0 + 1, kc}; };
-    if (ct)
-        for (int s = s0 - 1 + sl; s <= s1 + 2; s += TS)
-            F::template quot<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), scale != 0);
-    __syncthreads();
-    if (mass)
-        for (int s = s0 + sl; s <= s1; s += TS)
-            F::template fluxes<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), ct, images != 0);
-}
-
-// SweepCT + SweepMass of the z sweep: kZRows lines (i, j) in 0..nx+1 x
-// 0..ny+1 per block (CT fluxes on the lines in 0..n), 32 own k in 0..nz each;
-// the quotients of k0-1 .. k0+34 (up to nz+2) of each line go to shared
-// memory first.
-constexpr int kZRows = 8, kZOwn = 64, kZSpan = kZOwn + 3;
-struct ZRowStore {
-    double *sm;
-    int at;
-    __device__ double get(int a, int ds) const { return sm[a * (kZRows * kZSpan) + at + ds]; }
-    __device__ void put(int a, double v) const { sm[a * (kZRows * kZSpan) + at] = v; }
-};
-
-template <bool GEO>
-__global__ void __launch_bounds__(256, 5) k_ctmass_z(Ctx c, int images)  // cap tuned on B200
-{
-    using F = ops::SweepCTMass<2>;
-    __shared__ double zsm[F::NARR * kZRows * kZSpan];
-    const Geom &g = c.g;
-    const int r = (int)threadIdx.x / 32, kc = (int)threadIdx.x % 32;
-    const long long line = (long long)blockIdx.x * kZRows + r;
-    const bool on = line < (long long)(g.nx + 2) * (g.ny + 2);
-    const int i = on ? (int)(line / (g.ny + 2)) : 0, j = on ? (int)(line % (g.ny + 2)) : 0;
-    const int k0 = (int)blockIdx.y * kZOwn;
-    const bool ct = on && i <= g.nx && j <= g.ny;
-    if (ct)
-        for (int kk = kc; kk < kZSpan; kk += 32) {
-            const int k = k0 - 1 + kk;
-            if (k <= g.nz + 2) F::quot<GEO>(c, i, j, k, ZRowStore{zsm, r * kZSpan + kk}, false);
-        }
-    __syncthreads();
-    for (int kk = kc; kk < kZOwn; kk += 32) {
-        const int k = k0 + kk;  // along the sweep: 0..nz for both fluxes
-        if (on && k <= g.nz) F::fluxes<GEO>(c, i, j, k, ZRowStore{zsm, r * kZSpan + kk + 1}, ct, images != 0);
-    }
+    march::zsweep<GEO>(c, (int)blockIdx.x, ct_arg, zsm);
 }
 
 // The points of the out-of-place sweep's arrays it does not compute (rho and
@@ -719,7 +344,7 @@ long long Solver::bytes_for(const sams_lare_params &p)
     return (narr * nelem + staging + axes) * (long long)sizeof(double) + (long long)sizeof(Scalars) + 4096;
 }
 
-bool Solver::fused_path(const sams_lare_params &p) { return lanes_full(p.nz + 1, kMK); }
+bool Solver::fused_path(const sams_lare_params &p) { return lanes_full(p.nz + 1, 31); }
 
 Solver::~Solver() { free_all(); }
 
@@ -877,7 +502,6 @@ int Solver::init_impl(const sams_lare_params &p, const sams_lare_bcs &bcs, int d
     if ((rc = check(cudaMemcpy(sc_, &s0, sizeof(s0), cudaMemcpyHostToDevice), "scalars upload"))) return rc;
     ctx_.sc = sc_;
     bytes_ = (long long)abytes + (long long)(packed.size() * sizeof(double)) + (long long)sizeof(Scalars);
-    if ((rc = setup_psweep())) return rc;
     return check(cudaStreamSynchronize(stream_), "init sync");
 }
 
@@ -901,10 +525,7 @@ int Solver::init_borrowed(const sams_lare_params &p, const sams_lare_bcs &bcs, c
     ctx_ = ctx;
     sc_ = ctx.sc;  // borrowed: release_borrowed() must clear it before destruction
     stream_ = stream;
-    int rc;
-    if ((rc = check(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device), "sm count")))
-        return rc;
-    return setup_psweep();
+    return check(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device), "sm count");
 }
 
 void Solver::release_borrowed()
@@ -1008,17 +629,17 @@ void Solver::launch_psweep(int ct_arg)
     const Geom &g = ctx_.g;
     const ops::SweepOut w{ctx_.s[kOut[0]], ctx_.s[kOut[1]], ctx_.s[kOut[2]],
                           ctx_.s[kOut[3]], ctx_.s[kOut[4]], ctx_.s[kOut[5]]};
-    const int nd = DIR == 0 ? g.nx : g.ny, na = (DIR == 0 ? g.ny : g.nx) + 1;
-    const long long blocks = (long long)na * ((g.nz + ops::kWinK) / ops::kWinK) * ((nd + ops::kWinS) / ops::kWinS);
+    const int nd = DIR == 0 ? g.nx : g.ny, na = DIR == 0 ? g.ny : g.nx;
+    const WinTile wt = march::win_tile(nd + 1, (long long)(na + 1) * (g.nz + 1), 3, 4 * sm_count_);
     const size_t smem = (size_t)ops::SweepFused<DIR>::NARR * ops::WinStore::P * ops::kWinK * sizeof(double);
     // rho1 (rho before the sweep) is rho itself here: the sweep writes the new
     // rho elsewhere (SweepVol skipped the copy)
     Ctx cc = ctx_;
     cc.s[S_R_RHO1] = ctx_.f[SAMS_F_RHO];
     if (ctx_.p.geometry)
-        k_psweep<DIR, true><<<(unsigned)blocks, ops::kWinThreads, smem, stream_>>>(cc, w, ct_arg);
+        k_psweep<DIR, true><<<(unsigned)wt.blocks, ops::kWinThreads, smem, stream_>>>(cc, wt, w, ct_arg);
     else
-        k_psweep<DIR, false><<<(unsigned)blocks, ops::kWinThreads, smem, stream_>>>(cc, w, ct_arg);
+        k_psweep<DIR, false><<<(unsigned)wt.blocks, ops::kWinThreads, smem, stream_>>>(cc, wt, w, ct_arg);
     ++launches_;
     // The points the sweep does not compute are ghost points of each array;
     // the fill that follows the sweep rewrites all of them from domain values
@@ -1033,60 +654,38 @@ void Solver::launch_psweep(int ct_arg)
     for (int q = 0; q < 6; ++q) std::swap(ctx_.f[kState[q]], ctx_.s[kOut[q]]);
 }
 
-// Whether the fused x / y sweep runs for this solve (its windows must be at
-// least three quarters full of k values), and its shared memory: allow the
-// device's opt-in maximum (the attribute belongs to the kernel, so it is
-// the same for every solve).
-int Solver::setup_psweep()
-{
-    int maxsm = 0, rc;
-    if ((rc = check(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_), "smem limit")))
-        return rc;
-    const size_t need = (size_t)ops::SweepFused<0>::NARR * ops::WinStore::P * ops::kWinK * sizeof(double);
-    // a window holds kWinK adjacent k; thin grids would leave most lanes idle
-    const int kw = ops::kWinK, nk = ctx_.g.nz + 1;
-    const bool lanes_full = 4 * nk >= 3 * kw * ((nk + kw - 1) / kw);
-    psweep_ok_ = need <= (size_t)maxsm && lanes_full;
-    if (!psweep_ok_) return SAMS_OK;
-    const void *fn[4] = {(const void *)k_psweep<0, false>, (const void *)k_psweep<0, true>,
-                         (const void *)k_psweep<1, false>, (const void *)k_psweep<1, true>};
-    for (const void *f : fn)
-        if ((rc = check(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm), "psweep smem")))
-            return rc;
-    return SAMS_OK;
-}
-
 // A cell op + node op pair (k_cellnode_march) over the whole box.
 template <class P>
 void Solver::launch_cellnode(int arg)
 {
     const Geom &g = ctx_.g;
-    const long long blocks =
-        (long long)((g.nz + 2 + kMK) / kMK) * ((g.ny + 2 + kMJ) / kMJ) * ((g.nx + 2 + kMI) / kMI);
+    const MarchTile m = march::march_tile(g.nz + 3, g.ny + 3, g.nx + 3, P::kMinBlocks * sm_count_);
     const size_t smem = (size_t)P::NR * 3 * kRP * sizeof(double);
+    auto run = [&](auto kernel) { kernel<<<(unsigned)m.blocks, kMThreads, smem, stream_>>>(ctx_, m, arg); };
+    const bool wide = march::march_wide(m);
     if (ctx_.p.geometry)
-        k_cellnode_march<P, true, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, arg);
+        run(k_cellnode_march<P, true, false, 0>);
     else if (ctx_.p.pow2)
-        k_cellnode_march<P, false, true><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, arg);
+        wide ? run(k_cellnode_march<P, false, true, march::kWideW>) : run(k_cellnode_march<P, false, true, 0>);
     else
-        k_cellnode_march<P, false, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, arg);
+        wide ? run(k_cellnode_march<P, false, false, march::kWideW>) : run(k_cellnode_march<P, false, false, 0>);
     ++launches_;
 }
 
-// A marching edge-term kernel (k_edge_march) over cells 0..n+1.
-template <class P>
-void Solver::launch_edges()
+// The shock heating (k_heat_march) over cells 0..n+1.
+void Solver::launch_heat()
 {
     const Geom &g = ctx_.g;
-    const long long blocks =
-        (long long)((g.nz + 1 + kMK) / kMK) * ((g.ny + 1 + kMJ) / kMJ) * ((g.nx + 1 + kMI) / kMI);
+    const MarchTile m = march::march_tile(g.nz + 2, g.ny + 2, g.nx + 2, march::kHeatMinBlocks * sm_count_);
     const size_t smem = (size_t)3 * 3 * kRP * sizeof(double);
+    auto run = [&](auto kernel) { kernel<<<(unsigned)m.blocks, kMThreads, smem, stream_>>>(ctx_, m); };
+    const bool wide = march::march_wide(m);
     if (ctx_.p.geometry)
-        k_edge_march<P, true, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_);
+        run(k_heat_march<true, false, 0>);
     else if (ctx_.p.pow2)
-        k_edge_march<P, false, true><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_);
+        wide ? run(k_heat_march<false, true, march::kWideW>) : run(k_heat_march<false, true, 0>);
     else
-        k_edge_march<P, false, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_);
+        wide ? run(k_heat_march<false, false, march::kWideW>) : run(k_heat_march<false, false, 0>);
     ++launches_;
 }
 
@@ -1096,21 +695,23 @@ void Solver::launch_edges()
 void Solver::launch_pred(int resistive)
 {
     const Geom &g = ctx_.g;
-    const long long blocks = (long long)((g.nz + kMK) / kMK) * ((g.ny + kMJ) / kMJ) * ((g.nx + kMI) / kMI);
-    const size_t smem = (size_t)PredRingSrc::NR * 3 * kRP * sizeof(double);
+    const MarchTile m = march::march_tile(g.nz + 1, g.ny + 1, g.nx + 1, 3 * sm_count_);
+    const size_t smem = (size_t)march::PredRingSrc::NR * 3 * kRP * sizeof(double);
     double *pe = ctx_.s[S_CS], *pi = ctx_.s[S_CSV];
+    auto run = [&](auto kernel) { kernel<<<(unsigned)m.blocks, kMThreads, smem, stream_>>>(ctx_, m, resistive, pe, pi); };
+    const bool wide = march::march_wide(m);
     if (ctx_.p.geometry)
-        k_pred_march<true, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, resistive, pe, pi);
+        run(k_pred_march<true, false, 0>);
     else if (ctx_.p.pow2)
-        k_pred_march<false, true><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, resistive, pe, pi);
+        wide ? run(k_pred_march<false, true, march::kWideW>) : run(k_pred_march<false, true, 0>);
     else
-        k_pred_march<false, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, resistive, pe, pi);
+        wide ? run(k_pred_march<false, false, march::kWideW>) : run(k_pred_march<false, false, 0>);
     ++launches_;
     std::swap(ctx_.s[S_PE], ctx_.s[S_CS]);
     std::swap(ctx_.s[S_PI], ctx_.s[S_CSV]);
 }
 
-// One resistive sub-step fused (k_resist_march): the new B goes to the
+// One resistive sub-step fused (k_resist_march); the new B goes to the
 // S_CS / S_CSV / S_CV1 arrays (free during the sub-steps), whose slots then
 // swap with the field's, so after the two sub-steps B is back in its own
 // arrays and those three slots hold B as it was at the start of the last
@@ -1118,16 +719,17 @@ void Solver::launch_pred(int resistive)
 void Solver::launch_resist(bool last)
 {
     const Geom &g = ctx_.g;
-    const long long blocks =
-        (long long)((g.nz + 4 + kMK) / kMK) * ((g.ny + 4 + kMJ) / kMJ) * ((g.nx + 4 + kMI) / kMI);
+    const MarchTile m = march::march_tile(g.nz + 5, g.ny + 5, g.nx + 5, 5 * sm_count_);
     const size_t smem = (size_t)ops::ResistRK::NOUT * 3 * kRP * sizeof(double);
     double *nb[3] = {ctx_.s[S_CS], ctx_.s[S_CSV], ctx_.s[S_CV1]};
+    auto run = [&](auto kernel) { kernel<<<(unsigned)m.blocks, kMThreads, smem, stream_>>>(ctx_, m, nb[0], nb[1], nb[2]); };
+    const bool wide = march::march_wide(m);
     if (ctx_.p.geometry)
-        k_resist_march<true, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, nb[0], nb[1], nb[2]);
+        run(k_resist_march<true, false, 0>);
     else if (ctx_.p.pow2)
-        k_resist_march<false, true><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, nb[0], nb[1], nb[2]);
+        wide ? run(k_resist_march<false, true, march::kWideW>) : run(k_resist_march<false, true, 0>);
     else
-        k_resist_march<false, false><<<(unsigned)blocks, kMThreads, smem, stream_>>>(ctx_, nb[0], nb[1], nb[2]);
+        wide ? run(k_resist_march<false, false, march::kWideW>) : run(k_resist_march<false, false, 0>);
     ++launches_;
     std::swap(ctx_.f[SAMS_F_BX], ctx_.s[S_CS]);
     std::swap(ctx_.f[SAMS_F_BY], ctx_.s[S_CSV]);
@@ -1144,35 +746,25 @@ template <int DIR>
 bool Solver::launch_ctmass(int scale)
 {
     const Geom &g = ctx_.g;
-    // windows over k (x, y: kWinK lanes over 0..nz+1; z: kZOwn own k per
-    // line): on thin grids the separate kernels keep more lanes busy
-    const bool window = DIR == 2 ? lanes_full(g.nz + 1, kZOwn) : lanes_full(g.nz + 2, ops::kWinK);
-    if (!window) {  // (the solver folds the B scaling in only where the x window runs: scale == 0 here)
-        launch<ops::SweepCT<DIR>>(0);
-        launch<ops::SweepMass<DIR>>(0);
-        return false;
-    }
     // dm's periodic fill along the sweep folded into the kernel (the slabs'
     // x fill is an exchange between slabs and stays)
     const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
     const int images = !(halo_ && DIR == 0) && nd >= kBcSequentialBelow &&
                        bc_.kind[SAMS_F_DM][DIR][0] == SAMS_BC_PERIODIC && bc_.kind[SAMS_F_DM][DIR][1] == SAMS_BC_PERIODIC;
     if (DIR == 2) {
-        const long long lines = (long long)(g.nx + 2) * (g.ny + 2);
-        dim3 grid((unsigned)ceil_div(lines, kZRows), (unsigned)ceil_div(g.nz + 1, kZOwn));
+        const ZTile z = march::z_tile(g.nz, (long long)(g.nx + 2) * (g.ny + 2));
         if (ctx_.p.geometry)
-            k_ctmass_z<true><<<grid, 256, 0, stream_>>>(ctx_, images);
+            k_ctmass_z<true><<<(unsigned)z.blocks, march::kZCtThreads, 0, stream_>>>(ctx_, z, images);
         else
-            k_ctmass_z<false><<<grid, 256, 0, stream_>>>(ctx_, images);
+            k_ctmass_z<false><<<(unsigned)z.blocks, march::kZCtThreads, 0, stream_>>>(ctx_, z, images);
     } else {
         const int na = DIR == 0 ? g.ny : g.nx;
-        const long long blocks = (long long)(na + 2) * ((g.nz + 1 + ops::kWinK) / ops::kWinK) *
-                                 ((nd + kCtS) / kCtS);
-        const size_t smem = (size_t)ops::SweepCTMass<DIR>::NARR * kCtP * ops::kWinK * sizeof(double);
+        const WinTile w = march::win_tile(nd + 1, (long long)(na + 2) * (g.nz + 2), 3, 5 * sm_count_);
+        const size_t smem = (size_t)ops::SweepCTMass<DIR>::NARR * march::kCtP * ops::kWinK * sizeof(double);
         if (ctx_.p.geometry)
-            k_ctmass<DIR, true><<<(unsigned)blocks, ops::kWinThreads, smem, stream_>>>(ctx_, scale, images);
+            k_ctmass<DIR, true><<<(unsigned)w.blocks, ops::kWinThreads, smem, stream_>>>(ctx_, w, scale, images);
         else
-            k_ctmass<DIR, false><<<(unsigned)blocks, ops::kWinThreads, smem, stream_>>>(ctx_, scale, images);
+            k_ctmass<DIR, false><<<(unsigned)w.blocks, ops::kWinThreads, smem, stream_>>>(ctx_, w, scale, images);
     }
     ++launches_;
     return images != 0;
@@ -1278,15 +870,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     };
     mark(0);
     // ---- Lagrangian predictor ----
-    // the marching kernels tile k by kMK: on thin grids the separate kernels
-    // (one thread per (j, k) of a plane) keep more lanes busy
-    const bool march = lanes_full(ctx_.g.nz + 1, kMK);
-    if (march) {
-        launch_cellnode<PrepMarch>(resistive);
-    } else {
-        launch<ops::CellPrep>(resistive);
-        launch<ops::NodePrep>(0);
-    }
+    launch_cellnode<PrepMarch>(resistive);
     launch<ops::Alpha>(0);
     {
         // Visc with two threads per cell (k_visc_split): 1.21 -> 1.12 ms at
@@ -1309,31 +893,18 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     ++launches_;
     if (resistive) {
         for (int sub = 0; sub < 2; ++sub) {
-            if (march) {
-                launch_resist(sub == 1);
-            } else {
-                launch<ops::ResistRK>(0);
-                launch<ops::ResistB>(sub == 1 ? 1 : 0);
-            }
+            launch_resist(sub == 1);
             bc_fill(FM_BFIELD | FM_ENERGY);
         }
     }
-    if (march) {
-        launch_pred(resistive);
-    } else {
-        launch<ops::Pred1>(resistive);
-        launch<ops::Pred2>(0);
-    }
+    launch_pred(resistive);
     bc_fill(FM_REMAPV);
     mark(1);
     // ---- corrector ----
     // (Corr1 and Corr2 as one pass, with the velocities written out of place,
     // was measured slower on B200: Corr2 runs at 6 blocks per SM alone, at
     // Corr1's 2 when fused.)
-    if (march)
-        launch_edges<HeatEdges>();
-    else
-        launch<ops::Corr1>(0);
+    launch_heat();
     launch<ops::Corr2>(0);
     bc_fill(FM_VELOCITY | FM_ENERGY | FM_DENSITY);
     mark(2);
@@ -1343,17 +914,11 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     // the z sweep then unscales 0..n only, and the final B fill sets the
     // ghosts from those values, as it does after BScale's pass over the
     // whole box.
-    // The x-sweep half of the fold forms b * area inside k_ctmass, so it also
-    // needs that window kernel (not used on thin grids).
-    const bool b_fill_all = ghosts_refilled(FM_BFIELD) && lanes_full(ctx_.g.nz + 2, ops::kWinK);
+    const bool b_fill_all = ghosts_refilled(FM_BFIELD);
+    const bool fused_xy = !p_.rke;  // k_psweep runs the x and y stages
     if (p_.rke) launch<ops::RkeZero>(0);
     if (!b_fill_all) launch<ops::BScale>(0);
-    if (march) {
-        launch_cellnode<VolMarch<0>>(!p_.rke && psweep_ok_ ? 1 : 0);
-    } else {
-        launch<ops::SweepVol<0>>(!p_.rke && psweep_ok_ ? 1 : 0);
-        launch<ops::SweepCvc>(0);
-    }
+    launch_cellnode<VolMarch<0>>(fused_xy ? 1 : 0);
     const bool dm_x = launch_ctmass<0>(b_fill_all ? 1 : 0);
     // The CT update changes only B, which the dm fill and the stages S6-S8
     // do not read, so the y and z sweeps' fused stages take it at their
@@ -1361,7 +926,6 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     // folded in, it stays a kernel of its own: inside k_psweep it measured
     // slower on B200 (14 us per step), in the y and z sweeps faster (13 and
     // 40 us).
-    const bool fused_xy = !p_.rke && psweep_ok_;  // k_psweep runs the x and y stages
     launch<ops::SweepCTUpd<0>>(b_fill_all ? 1 : 0);
     if (!dm_x) bc_fill_dim(FM_DM, 0);
     if (fused_xy) {
@@ -1377,12 +941,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     }
     bc_fill(FM_ALL9);
     mark(3);
-    if (march) {
-        launch_cellnode<VolMarch<1>>(!p_.rke && psweep_ok_ ? 1 : 0);
-    } else {
-        launch<ops::SweepVol<1>>(!p_.rke && psweep_ok_ ? 1 : 0);
-        launch<ops::SweepCvc>(0);
-    }
+    launch_cellnode<VolMarch<1>>(fused_xy ? 1 : 0);
     const bool dm_y = launch_ctmass<1>(0);
     if (!fused_xy) launch<ops::SweepCTUpd<1>>(0);
     if (!dm_y) bc_fill_dim(FM_DM, 1);
@@ -1399,12 +958,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     }
     bc_fill(FM_ALL9);
     mark(4);
-    if (march) {
-        launch_cellnode<VolMarch<2>>(0);
-    } else {
-        launch<ops::SweepVol<2>>(0);
-        launch<ops::SweepCvc>(0);
-    }
+    launch_cellnode<VolMarch<2>>(0);
     const bool dm_z = launch_ctmass<2>(0);
     const bool zfused = !p_.rke && ctx_.g.nz + 4 <= kZThreads;
     if (!zfused) launch<ops::SweepCTUpd<2>>(b_fill_all ? 2 : 0);

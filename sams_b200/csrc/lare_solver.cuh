@@ -112,12 +112,11 @@ private:
     template <class Op> void launch(int arg);
     template <int DIR> void launch_psweep(int ct_arg);
     template <class P> void launch_cellnode(int arg);
-    template <class P> void launch_edges();
+    void launch_heat();
     void launch_pred(int resistive);
     void launch_resist(bool last);
     // true when the kernel also wrote dm's periodic ghost images along DIR
     template <int DIR> bool launch_ctmass(int scale);
-    int setup_psweep();
     int staging(double **out);
     void free_all();
 
@@ -126,7 +125,6 @@ private:
     sams_lare_params p_{};
     BcTable bc_{};
     Halo *halo_ = nullptr;
-    bool psweep_ok_ = false;  // the fused x / y sweep's shared memory fits this device
     int device_ = 0;
     int sm_count_ = 148;  // multiprocessors of device_ (grid sizing)
     cudaStream_t own_stream_ = nullptr;
