@@ -107,7 +107,7 @@ __host__ __device__ inline BcEdge bc_edge_slab(const Geom &g, int f, int d, int 
 
 // Value the condition writes at ghost point q (q[d] in glo..ghi), from the
 // array's current contents.
-__device__ __forceinline__ double bc_edge_value(const double *a, const Geom &g, const BcEdge &s, int kind,
+__host__ __device__ __forceinline__ double bc_edge_value(const double *a, const Geom &g, const BcEdge &s, int kind,
                                                 double clamp_value, int d, int e, const int *q)
 {
     const int gq = q[d];
@@ -139,7 +139,7 @@ __device__ __forceinline__ double bc_edge_value(const double *a, const Geom &g, 
 // cells) the whole ghost line through q when q is its first layer.  A LARE
 // BC_OTHER slot writes q only if its plane is one the slot's operations
 // write; those operations are independent, so every point is one thread.
-__device__ __forceinline__ void bc_edge_apply(double *a, const Geom &g, const BcEdge &s, const BcTable &bt, int f,
+__host__ __device__ __forceinline__ void bc_edge_apply(double *a, const Geom &g, const BcEdge &s, const BcTable &bt, int f,
                                               int d, int e, int *q)
 {
     const int kind = bt.kind[f][d][e];
@@ -172,5 +172,108 @@ __device__ __forceinline__ void bc_edge_apply(double *a, const Geom &g, const Bc
         a[box_off(g, q[0], q[1], q[2])] = v;
     }
 }
+
+// Host: whether the conditions of field f can be applied in one pass over its
+// ghost shell (bc_compose_value): every ghost point's final value is then a
+// function of points that the fill leaves as they are, so no thread reads
+// what another writes.  That needs three or more cells in the dimension and,
+// for a half-cell field, whose boundary index (0 or n) is a ghost and a
+// domain point at once, conditions that leave the boundary index they read
+// unchanged: both edges periodic (index 0 takes index n, which keeps its
+// value), or zero-gradient, clamp or none on either.  The plane operations of
+// SAMS_BC_LARE_OTHER stay with the edge by edge fill.
+inline bool bc_composable(const BcTable &t, int f, const int n[3])
+{
+    for (int d = 0; d < 3; ++d) {
+        const int l = t.kind[f][d][0], u = t.kind[f][d][1];
+        if (n[d] < kBcSequentialBelow || l == SAMS_BC_LARE_OTHER || u == SAMS_BC_LARE_OTHER) return false;
+        if (!field_half(f, d)) continue;
+        if ((l == SAMS_BC_PERIODIC) != (u == SAMS_BC_PERIODIC) || l == SAMS_BC_MIRROR || u == SAMS_BC_MIRROR) return false;
+    }
+    return true;
+}
+
+// Value at point q of field f after the conditions of dimensions 0..D, lower
+// edge then upper in each, from the array as it was before the fill: the last
+// dimension in which q is a ghost decides, reading what the earlier
+// dimensions leave at its source (the reference's order, row by row copies of
+// bc_edge_value).
+template <int D>
+__host__ __device__ inline double bc_compose_value(const double *a, const Geom &g, const BcTable &bt, int f, int q0,
+                                                   int q1, int q2)
+{
+    if constexpr (D < 0) {
+        return a[box_off(g, q0, q1, q2)];
+    } else {
+        const int n = D == 0 ? g.nx : (D == 1 ? g.ny : g.nz);
+        const int q = D == 0 ? q0 : (D == 1 ? q1 : q2);
+        const bool half = field_half(f, D) != 0;
+        auto raw = [&](int p) {
+            return bc_compose_value<D - 1>(a, g, bt, f, D == 0 ? p : q0, D == 1 ? p : q1, D == 2 ? p : q2);
+        };
+        const int e = q >= (half ? n : n + 1) ? 1 : 0;
+        if (e == 0 && q > 0) return raw(q);
+        switch (bt.kind[f][D][e]) {
+        case SAMS_BC_NONE:
+            return raw(q);
+        case SAMS_BC_PERIODIC:  // (a half-cell upper copy of index 0 reads what the lower edge put there, index n)
+            return raw(e == 0 ? q + n : (half && q == n ? n : q - n));
+        case SAMS_BC_ZERO_GRADIENT:
+            return raw(e == 0 ? (half ? 0 : 1) : n);
+        case SAMS_BC_MIRROR: {
+            const double av = raw(e == 0 ? 1 : n);
+            const double bv = (av + av) / 2.0;
+            const double delta = raw(e == 0 ? 1 - q : 2 * n + 1 - q) - bv;
+            return bv - delta;
+        }
+        default:  // SAMS_BC_CLAMP
+            return bt.value[f][D][e];
+        }
+    }
+}
+
+// The points of field f's range that are ghosts in some dimension (-1 or -2
+// to 0, and n+1 or, half-cell, n and up), one per t in 0 .. count-1.
+struct BcShell {
+    int lb[3], ext[3], nin[3], gh[3];  // first index, points, inner points 1.., ghosts per dimension
+    __host__ __device__ BcShell(const Geom &g, int f)
+    {
+        const int n[3] = {g.nx, g.ny, g.nz};
+        for (int d = 0; d < 3; ++d) {
+            const int h = field_half(f, d);
+            lb[d] = h ? -2 : -1;
+            ext[d] = n[d] + 3 - lb[d];
+            nin[d] = n[d] - h;
+            gh[d] = ext[d] - nin[d];
+        }
+    }
+    __host__ __device__ int ghost(int d, int t) const { return t < 1 - lb[d] ? lb[d] + t : nin[d] + 1 + (t - (1 - lb[d])); }
+    __host__ __device__ bool point(int t, int &i, int &j, int &k) const
+    {
+        const int A = gh[0] * ext[1] * ext[2], B = nin[0] * gh[1] * ext[2], C = nin[0] * nin[1] * gh[2];
+        if (t < A) {
+            const int pl = ext[1] * ext[2], x = t / pl, r = t - x * pl;
+            i = ghost(0, x);
+            j = lb[1] + r / ext[2];
+            k = lb[2] + r % ext[2];
+            return true;
+        }
+        if ((t -= A) < B) {
+            const int pl = gh[1] * ext[2], x = t / pl, r = t - x * pl, y = r / ext[2];
+            i = 1 + x;
+            j = ghost(1, y);
+            k = lb[2] + (r - y * ext[2]);
+            return true;
+        }
+        if ((t -= B) < C) {
+            const int pl = nin[1] * gh[2], x = t / pl, r = t - x * pl, y = r / gh[2];
+            i = 1 + x;
+            j = 1 + y;
+            k = ghost(2, r - y * gh[2]);
+            return true;
+        }
+        return false;
+    }
+};
 
 }  // namespace sams

@@ -1252,6 +1252,9 @@ struct SweepMass {
     }
 };
 
+// What SweepCTMass writes into dm's ghosts along the sweep.
+enum { kNoImages = 0, kPeriodicImages, kCopyImages };
+
 // SweepCT and SweepMass of one sweep in one kernel (k_ctmass): every
 // quotient b/db of the CT fluxes is formed once per point into a window store
 // and read by the four fluxes along the sweep that use it (the separate
@@ -1292,12 +1295,14 @@ struct SweepCTMass {
     }
     // CT fluxes where `ct` ((i, j, k) in 0..n), the mass flux everywhere it
     // is called (0..n along the sweep, 0..n+1 across).  With `images` (dm
-    // periodic along the sweep, at least three cells) the mass flux also goes
-    // to the ghost points that the periodic fill along the sweep would copy it
-    // to (sweep index n-1, n -> -1, 0 and 1, 2 -> n+1, n+2), and index 0,
-    // which that fill overwrites, is left alone, so the fill is not needed.
+    // periodic, or zero-gradient at both edges, along the sweep, at least three
+    // cells) the mass flux also goes to the ghost points that the fill along
+    // the sweep would copy it to (periodic: sweep index n-1, n -> -1, 0 and
+    // 1, 2 -> n+1, n+2; zero-gradient: 1 -> -1, 0 and n -> n+1, n+2), and
+    // index 0, which that fill overwrites, is left alone, so the fill is not
+    // needed.
     template <bool GEO, class A>
-    __device__ static void fluxes(const Ctx &c, int i, int j, int k, A st, bool ct, bool images = false)
+    __device__ static void fluxes(const Ctx &c, int i, int j, int k, A st, bool ct, int images)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
@@ -1319,13 +1324,18 @@ struct SweepCTMass {
         const double m = mass_flux(face_velocity<DIR>(c, o), dt, face_area<DIR, GEO>(c, i, j, k), rho[o - d],
                                    rho[o], rho[o + d], rho[o + 2 * d], dci, dcm, dcp, cvi, cvp);
         double *dm = c.f[SAMS_F_DM];
-        if (!images) {
+        if (images == kNoImages) {
             dm[o] = m;
             return;
         }
         const int s = DIR == 0 ? i : (DIR == 1 ? j : k);
         const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
         if (s >= 1) dm[o] = m;
+        if (images == kCopyImages) {
+            if (s == 1) dm[o - d] = dm[o - 2 * d] = m;
+            if (s == nd) dm[o + d] = dm[o + 2 * d] = m;
+            return;
+        }
         if (s >= nd - 1) dm[o - nd * d] = m;
         if (s >= 1 && s <= 2) dm[o + nd * d] = m;
     }

@@ -315,6 +315,20 @@ __global__ void __launch_bounds__(kThreads) k_bc_edge(Ctx c, FieldList fl, BcTab
     bc_edge_apply(c.f[f], g, sl, bt, f, d, e, q);
 }
 
+// All conditions of the given fields in one pass over each field's ghost
+// shell, where they compose (bc_composable): the six edge launches of a fill
+// with walls become one.
+__global__ void __launch_bounds__(kThreads) k_bc_compose(Ctx c, FieldList fl, BcTable bt)
+{
+    const int f = fl.id[blockIdx.y];
+    const BcShell sh(c.g, f);
+    int i, j, k;
+    if (!sh.point((int)(blockIdx.x * blockDim.x + threadIdx.x), i, j, k)) return;
+    double *a = c.f[f];
+    const double v = bc_compose_value<2>(a, c.g, bt, f, i, j, k);
+    a[box_off(c.g, i, j, k)] = v;
+}
+
 FieldList make_list(unsigned mask)
 {
     FieldList fl{};
@@ -746,11 +760,14 @@ template <int DIR>
 bool Solver::launch_ctmass(int scale)
 {
     const Geom &g = ctx_.g;
-    // dm's periodic fill along the sweep folded into the kernel (the slabs'
+    // dm's periodic or zero-gradient fill along the sweep folded into the kernel (the slabs'
     // x fill is an exchange between slabs and stays)
     const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
-    const int images = !(halo_ && DIR == 0) && nd >= kBcSequentialBelow &&
-                       bc_.kind[SAMS_F_DM][DIR][0] == SAMS_BC_PERIODIC && bc_.kind[SAMS_F_DM][DIR][1] == SAMS_BC_PERIODIC;
+    int images = ops::kNoImages;
+    if (!(halo_ && DIR == 0) && nd >= kBcSequentialBelow && bc_.kind[SAMS_F_DM][DIR][0] == bc_.kind[SAMS_F_DM][DIR][1]) {
+        if (bc_.kind[SAMS_F_DM][DIR][0] == SAMS_BC_PERIODIC) images = ops::kPeriodicImages;
+        if (bc_.kind[SAMS_F_DM][DIR][0] == SAMS_BC_ZERO_GRADIENT) images = ops::kCopyImages;
+    }
     if (DIR == 2) {
         const ZTile z = march::z_tile(g.nz, (long long)(g.nx + 2) * (g.ny + 2));
         if (ctx_.p.geometry)
@@ -767,7 +784,7 @@ bool Solver::launch_ctmass(int scale)
             k_ctmass<DIR, false><<<(unsigned)w.blocks, ops::kWinThreads, smem, stream_>>>(ctx_, w, scale, images);
     }
     ++launches_;
-    return images != 0;
+    return images != ops::kNoImages;
 }
 
 template <class Op>
@@ -834,6 +851,17 @@ void Solver::bc_fill(unsigned mask)
         k_bc_periodic<<<grid, kThreads, 0, stream_>>>(ctx_, fl);
         ++launches_;
         (void)e0;
+        return;
+    }
+    const int n[3] = {g.nx, g.ny, g.nz};
+    bool compose = true;
+    for (int q = 0; q < fl.n; ++q) compose = compose && bc_composable(bc_, fl.id[q], n);
+    if (compose) {
+        const long long e1 = g.ny + 5, e2 = g.nz + 5;
+        const long long cnt = 6 * e1 * e2 + (long long)g.nx * 6 * e2 + (long long)g.nx * g.ny * 6;  // the largest shell
+        dim3 grid((unsigned)ceil_div(cnt, kThreads), (unsigned)fl.n);
+        k_bc_compose<<<grid, kThreads, 0, stream_>>>(ctx_, fl, bc_);
+        ++launches_;
         return;
     }
     for (int d = 0; d < 3; ++d) bc_fill_dim(mask, d);
