@@ -25,7 +25,11 @@ struct Geom {
     int sx, sy;        // element strides of i and j (k stride is 1)
     int zoff;          // k + zoff is the position of index k in its row
     long long nelem;   // doubles per field allocation
+    int far;           // the solves in hand outgrow L2 (far_from_l2): fused kernels prefetch
 };
+// Whether arrays of this many doubles (summed over the solves stepped
+// together) outgrow L2 during a phase, which reads a dozen of them.
+inline int far_from_l2(long long nelem) { return nelem * 8 * 12 > 126000000LL; }
 
 // Host/device helpers for the box geometry.
 // Offsets are 32-bit: the 32 arrays of a solve must fit one GPU, so a single

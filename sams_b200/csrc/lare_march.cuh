@@ -103,6 +103,18 @@ __host__ __device__ __forceinline__ MarchAt march_at(const MarchTile &m, int b, 
     return a;
 }
 
+// Ask L2 for the line at offset o of an array (no register waits for it).
+// These kernels wait on memory first (8 to 16 of the 14 to 24 cycles between
+// a warp's instructions), and where the arrays outgrow L2 half of those waits
+// go to DRAM, one after another as each stage reaches its arrays.  So each
+// block asks at its start, or a plane ahead, for what its later stages read:
+// 256^3 x and y stages 1.33 -> 1.24 and 1.47 -> 1.36 ms, predictor 1.52 -> 1.46,
+// resistive sub-step 0.41 -> 0.37, heating 0.46 -> 0.42.  On grids that stay in
+// L2 (96^3) the cell-to-node marches lost 7% with it: Geom::far draws the line
+// at twelve arrays, what a phase reads, against L2's 126 MB.  (Asking for the
+// next wave's block instead was 4% slower over the step than none at all.)
+__device__ __forceinline__ void prefetch(const double *a, int o) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a + o)); }
+
 struct RingSrc {
     const double *ring;
     __device__ double operator()(int arr, int q) const { return ring[arr * 3 * kRP + q]; }
@@ -157,6 +169,31 @@ __device__ __forceinline__ void pred(const Ctx &c, const MarchTile &m, int b, in
     const PredRingSrc src{ring};
     produce(i0);
     for (int i = i0; i <= i1; ++i) {
+        if (g.far && cell && i < i1) {
+            const int o = box_off(g, i + 2, j, k);
+            prefetch(c.f[SAMS_F_VX], o);
+            prefetch(c.f[SAMS_F_VY], o);
+            prefetch(c.f[SAMS_F_VZ], o);
+            prefetch(c.f[SAMS_F_RHO], o);
+            prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+            prefetch(c.f[SAMS_F_ENERGY_ION], o);
+            prefetch(c.s[S_VH], o);
+            if (resistive) {
+                prefetch(c.s[S_B1X], o);
+                prefetch(c.s[S_B1Y], o);
+                prefetch(c.s[S_B1Z], o);
+                prefetch(c.s[S_PE], o);
+                prefetch(c.s[S_PI], o);
+            } else {
+                prefetch(c.f[SAMS_F_BX], o);
+                prefetch(c.f[SAMS_F_BY], o);
+                prefetch(c.f[SAMS_F_BZ], o);
+            }
+            prefetch(c.s[S_FXV], o - g.sx);
+            prefetch(c.s[S_FYV], o - g.sx);
+            prefetch(c.s[S_FZV], o - g.sx);
+            prefetch(c.s[S_RHOV], o - g.sx);
+        }
         produce(i + 1);
         __syncthreads();  // the ring's planes i and i+1 are complete
         if (on) {
@@ -198,6 +235,7 @@ __device__ __forceinline__ void cellnode(const Ctx &c, const MarchTile &m, int b
     const RingSrc src{ring};
     produce(i0);
     for (int i = i0; i <= i1; ++i) {
+        if (g.far && cell && i < i1) P::prefetch_cell(c, box_off(g, i + 2, j, k));
         produce(i + 1);
         __syncthreads();  // the ring's planes i and i+1 are complete
         if (on) {
@@ -211,6 +249,15 @@ __device__ __forceinline__ void cellnode(const Ctx &c, const MarchTile &m, int b
 // the node averages, so cs never goes to global memory; in resistive runs
 // (arg 1) the cell's step-start p_e, p_i are stored.
 struct PrepMarch {
+    __device__ static void prefetch_cell(const Ctx &c, int o)
+    {
+        prefetch(c.f[SAMS_F_RHO], o);
+        prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+        prefetch(c.f[SAMS_F_ENERGY_ION], o);
+        prefetch(c.f[SAMS_F_BX], o);
+        prefetch(c.f[SAMS_F_BY], o);
+        prefetch(c.f[SAMS_F_BZ], o);
+    }
     static constexpr int NR = 2, kMinBlocks = 5;  // register cap tuned on B200
     template <bool GEO, bool P2>
     __device__ static void produce(const Ctx &c, int resistive, int i, int j, int k, bool own, double *out)
@@ -234,6 +281,12 @@ struct PrepMarch {
 // volumes cvc1.
 template <int DIR>
 struct VolMarch {
+    __device__ static void prefetch_cell(const Ctx &c, int o)
+    {
+        if (DIR == 0) prefetch(c.f[SAMS_F_VX1], o);
+        if (DIR <= 1) prefetch(c.f[SAMS_F_VY1], o);
+        prefetch(c.f[SAMS_F_VZ1], o);
+    }
     static constexpr int NR = 1, kMinBlocks = DIR == 2 ? 5 : 4;  // register cap tuned on B200
     template <bool GEO, bool P2>
     __device__ static void produce(const Ctx &c, int arg, int i, int j, int k, bool own, double *out)
@@ -280,6 +333,18 @@ __device__ __forceinline__ void heat_edges(const Ctx &c, const MarchTile &m, int
     const RingSrc src{ring};
     produce(i0 - 1);
     for (int i = i0; i <= i1; ++i) {
+        if (g.far && node && i < i1) {
+            const int o = box_off(g, i + 1, jn, k);
+            prefetch(c.f[SAMS_F_VX], o);
+            prefetch(c.f[SAMS_F_VY], o);
+            prefetch(c.f[SAMS_F_VZ], o);
+            prefetch(c.f[SAMS_F_VX1], o);
+            prefetch(c.f[SAMS_F_VY1], o);
+            prefetch(c.f[SAMS_F_VZ1], o);
+            prefetch(c.s[S_A1], o);
+            prefetch(c.s[S_A2], o);
+            prefetch(c.s[S_A3], o);
+        }
         produce(i);
         __syncthreads();  // the ring's planes i-1 and i are complete
         if (on) {
@@ -327,6 +392,14 @@ __device__ __forceinline__ void resist(const Ctx &c, const MarchTile &m, int b, 
     const RingSrc src{ring};
     produce(i0 - 1);
     for (int i = i0; i <= i1; ++i) {
+        if (g.far && on && i < i1) {
+            const int o = box_off(g, i + 1, j, k), ob = i < g.nx ? o + g.sx : o;  // ResistRK reads B at +1
+            prefetch(c.f[SAMS_F_BX], ob);
+            prefetch(c.f[SAMS_F_BY], ob);
+            prefetch(c.f[SAMS_F_BZ], ob);
+            prefetch(c.f[SAMS_F_RHO], o);
+            prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+        }
         produce(i);
         __syncthreads();  // the ring's planes i-1 and i are complete
         if (on) {
@@ -424,6 +497,14 @@ __device__ __forceinline__ void ctmass(const Ctx &c, const WinTile &w, int b, in
     const int s0 = p.s0, s1 = p.s1, kc = p.kc, sl = p.sl, a = p.a, k = p.k;
     const bool mass = a <= na + 1, ct = a <= na && k <= g.nz;
     auto at = [&](int s) { return CtStore{csm, s - s0 + 1, kc}; };
+    if (g.far && mass)
+        for (int s = s0 + sl; s <= s1; s += TS) {
+            const int o = box_off(g, DIR == 0 ? s : a, DIR == 0 ? a : s, k);
+            prefetch(c.f[SAMS_F_VX1 + DIR], o);
+            prefetch(c.s[S_R_CV1], o);
+            prefetch(c.s[S_R_CVC1], o);
+            prefetch(c.f[SAMS_F_RHO], o);
+        }
     if (ct)
         for (int s = s0 - 1 + sl; s <= s1 + 2; s += TS)
             F::template quot<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), scale != 0);
@@ -525,6 +606,22 @@ __device__ __forceinline__ void psweep(const Ctx &c, const WinTile &wt, int b, c
     const bool on = a <= na;
     auto at = [&](int s) { return ops::WinStore{psm, s - s0 + 2, kc}; };
     const int a_lo = max(s0 - 2, -2), a_hi = min(s1 + 1, nd + 1);
+    if (g.far && on) {
+        for (int s = a_lo + sl; s <= a_hi; s += TS) {
+            const int o = box_off(g, DIR == 0 ? s : a, DIR == 0 ? a : s, k);
+            prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+            prefetch(c.f[SAMS_F_ENERGY_ION], o);
+            prefetch(c.s[S_R_CV1], o);
+            prefetch(c.s[S_R_CVC1], o);
+            prefetch(c.s[S_R_RHO1], o);
+            prefetch(c.f[SAMS_F_DM], o);
+            prefetch(c.f[SAMS_F_VX1 + DIR], o);
+            prefetch(c.s[S_R_CV2], o);
+            prefetch(c.f[SAMS_F_VX], o);
+            prefetch(c.f[SAMS_F_VY], o);
+            prefetch(c.f[SAMS_F_VZ], o);
+        }
+    }
     for (int s = a_lo + sl; s <= a_hi; s += TS)
         if (on) F::template stage_a<GEO>(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), w, s >= s0 && s <= s1);
     __syncthreads();
@@ -561,6 +658,23 @@ __device__ __forceinline__ void zsweep(const Ctx &c, int b, int ct_arg, double *
     const int i = on ? (int)(q / (g.ny + 1)) : 0, j = on ? (int)(q % (g.ny + 1)) : 0;
     const ops::LineStore st{zsm, S, line * W + k + 2};
     const ops::SweepOut w = ops::sweep_in_place(c);
+    if (g.far && on) {
+        const int o = box_off(g, i, j, k);
+        prefetch(c.f[SAMS_F_VX], o);
+        prefetch(c.f[SAMS_F_VY], o);
+        prefetch(c.f[SAMS_F_VZ], o);
+        prefetch(c.s[S_R_CV2], o);
+        prefetch(c.f[SAMS_F_DM], o);
+        prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+        prefetch(c.f[SAMS_F_ENERGY_ION], o);
+        if (ct_arg >= 0) {
+            prefetch(c.f[SAMS_F_BX], o);
+            prefetch(c.f[SAMS_F_BY], o);
+            prefetch(c.f[SAMS_F_BZ], o);
+            prefetch(c.s[S_R_CT1], o);
+            prefetch(c.s[S_R_CT2], o);
+        }
+    }
     if (on) F::stage_a<GEO>(c, i, j, k, st, w, true);
     __syncthreads();
     if (on && k >= 1 && k <= g.nz) F::stage_b_energy(c, i, j, k, st, w);

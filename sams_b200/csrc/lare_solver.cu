@@ -175,6 +175,24 @@ __global__ void __launch_bounds__(kThreads, 4) k_visc_split(Ctx c)  // 4 blocks 
         const int j = lo[1] + (int)(t / nk);
         const int k = lo[2] + (int)(t % nk);
         for (int i = lo[0] + (int)blockIdx.y; i <= hi[0]; i += gridDim.y) {
+            if (c.g.far && i + (int)gridDim.y <= hi[0]) {  // the plane this thread walks to next
+                const int o = box_off(c.g, i + (int)gridDim.y, j, k);
+                if (half == 0) {
+                    march::prefetch(c.f[SAMS_F_VX], o);
+                    march::prefetch(c.f[SAMS_F_VY], o);
+                    march::prefetch(c.f[SAMS_F_VZ], o);
+                    march::prefetch(c.s[S_A1], o);
+                    march::prefetch(c.s[S_A2], o);
+                    march::prefetch(c.s[S_A3], o);
+                } else {
+                    march::prefetch(c.f[SAMS_F_BX], o);
+                    march::prefetch(c.f[SAMS_F_BY], o);
+                    march::prefetch(c.f[SAMS_F_BZ], o);
+                    march::prefetch(c.f[SAMS_F_RHO], o);
+                    march::prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
+                    march::prefetch(c.f[SAMS_F_ENERGY_ION], o);
+                }
+            }
             if (half == 0)
                 ops::Visc::heat_forces<GEO, P2>(c, i, j, k, bad);
             else if (i <= c.g.nx && j <= c.g.ny && k <= c.g.nz)
@@ -456,6 +474,7 @@ int Solver::init_impl(const sams_lare_params &p, const sams_lare_bcs &bcs, int d
     g.sy = (int)zrow;
     g.sx = (int)sx;
     g.nelem = (long long)(p.nx + 5) * sx;
+    g.far = far_from_l2(g.nelem);
     // the rke correction keeps one more array (delta_ke) across the sweeps
     const long long narr = SAMS_NFIELDS + NSCRATCH + (p.rke ? 1 : 0);
     const size_t abytes = (size_t)narr * (size_t)g.nelem * sizeof(double);
