@@ -3,12 +3,14 @@
 // The per-point work is the same sams::ops code as the single-solve path;
 // what changes is the launcher: a persistent grid strides over a worklist of
 // tiles from every live solve, loading each tile's solve context (pointers,
-// geometry, parameters) into shared memory.  Boundary fills walk a flattened
-// index over the ghost shells of all solves.  One batched step is the same
-// phase sequence as Solver::enqueue_step, each phase a single launch for the
-// whole batch.
+// geometry, parameters) into shared memory.  The fused kernels run the same
+// bodies as the single solve's (lare_march.cuh), their worklist the blocks of
+// every solve's own tiling; boundary fills walk the ghost shells of all
+// solves.  One batched step is the same phase sequence as
+// Solver::enqueue_step, each phase a single launch for the whole batch.
 #include "lare_batch.cuh"
 #include "lare_ops.cuh"
+#include "lare_march.cuh"
 #include "lare_bc.cuh"
 #include "lare_geom_host.h"
 
@@ -20,10 +22,62 @@ namespace sams {
 namespace {
 
 constexpr int kT = 256;
+constexpr int kFillPoints = kT;  // shell points per entry of the fill's block list
 
-__device__ __forceinline__ void load_ctx(Ctx &dst, const Ctx *src)
+// Where the x and y sweeps write the six state fields (launch_psweep of the
+// single solve), and those fields.
+__constant__ const int kSweepOut[6] = {S_FX, S_FY, S_FZ, S_VH, S_FXV, S_FYV};
+
+// Points of the shell that kb_bc_fill walks, and point t of it.
+__host__ __device__ inline int fill_points(const Geom &g)
 {
-    const int nw = (int)(sizeof(Ctx) / sizeof(int));
+    return 6 * (g.ny + 5) * (g.nz + 5) + (g.nx - 1) * 6 * (g.nz + 5) + (g.nx - 1) * (g.ny - 1) * 6;
+}
+__device__ __forceinline__ int shell_index(int n, int t) { return t < 3 ? t - 2 : n + t - 3; }  // -2, -1, 0, n .. n+2
+__device__ __forceinline__ bool fill_point(const Geom &g, int t, int &q0, int &q1, int &q2)
+{
+    const int E1 = g.ny + 5, E2 = g.nz + 5;
+    const int A = 6 * E1 * E2, B = (g.nx - 1) * 6 * E2, C = (g.nx - 1) * (g.ny - 1) * 6;
+    if (t < A) {
+        const int x = t / (E1 * E2), r = t - x * (E1 * E2), y = r / E2;
+        q0 = shell_index(g.nx, x);
+        q1 = y - 2;
+        q2 = r - y * E2 - 2;
+        return true;
+    }
+    if ((t -= A) < B) {
+        const int i = t / (6 * E2), r = t - i * (6 * E2), y = r / E2;
+        q0 = 1 + i;
+        q1 = shell_index(g.ny, y);
+        q2 = r - y * E2 - 2;
+        return true;
+    }
+    if ((t -= B) < C) {
+        const int i = t / ((g.ny - 1) * 6), r = t - i * ((g.ny - 1) * 6), j = r / 6;
+        q0 = 1 + i;
+        q1 = 1 + j;
+        q2 = shell_index(g.nz, r - j * 6);
+        return true;
+    }
+    return false;
+}
+// Whether field f's own range holds the point and has it as a ghost.
+__device__ __forceinline__ bool field_ghost(const Geom &g, int f, int q0, int q1, int q2)
+{
+    const int q[3] = {q0, q1, q2}, n[3] = {g.nx, g.ny, g.nz};
+    bool ghost = false;
+    for (int d = 0; d < 3; ++d) {
+        const int h = field_half(f, d);
+        if (q[d] < (h ? -2 : -1)) return false;
+        ghost = ghost || q[d] <= 0 || q[d] > n[d] - h;
+    }
+    return ghost;
+}
+
+template <class T>
+__device__ __forceinline__ void load_words(T &dst, const T *src)
+{
+    const int nw = (int)(sizeof(T) / sizeof(int));
     const int *s = reinterpret_cast<const int *>(src);
     int *d = reinterpret_cast<int *>(&dst);
     for (int w = threadIdx.x; w < nw; w += blockDim.x) d[w] = s[w];
@@ -33,8 +87,7 @@ __device__ __forceinline__ void load_ctx(Ctx &dst, const Ctx *src)
 // used when none is, carries no metric factors).
 template <class Op, bool GEO, bool P2>
 __global__ void __launch_bounds__(kT, (MinBlocksBatch<Op, P2>::value))
-    kb_op(const Ctx *__restrict__ ctxs, const Tile *__restrict__ tiles, int ntiles, int arg, int tile_i,
-          int resistive_only)
+    kb_op(const Ctx *__restrict__ ctxs, const Tile *__restrict__ tiles, int ntiles, int arg, int tile_i)
 {
     __shared__ Ctx c;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -44,21 +97,18 @@ __global__ void __launch_bounds__(kT, (MinBlocksBatch<Op, P2>::value))
         // every op's range is inside them, and a tile past the op's range
         // is skipped before its context is staged (uniform over the block)
         const Ctx *src = ctxs + tl.inst;
-        const int resistive = src->p.resistive;
-        if (resistive_only && !resistive) continue;
-        const int a = arg >= 0 ? arg : resistive;
         int lo[3], hi[3];
-        Op::bounds(src->g, a, lo, hi);
+        Op::bounds(src->g, arg, lo, hi);
         const int nk = hi[2] - lo[2] + 1;
         if (tl.p0 >= (hi[1] - lo[1] + 1) * nk || tl.i0 > hi[0] || tl.i0 + tile_i - 1 < lo[0]) continue;
         __syncthreads();
-        load_ctx(c, src);
+        load_words(c, src);
         __syncthreads();
         const int p = tl.p0 + (int)threadIdx.x;
         if (p >= (hi[1] - lo[1] + 1) * nk) continue;
         const int j = lo[1] + p / nk, k = lo[2] + p % nk;
         const int ia = max(tl.i0, lo[0]), ib = min(tl.i0 + tile_i - 1, hi[0]);
-        for (int i = ia; i <= ib; ++i) Op::template run<GEO, P2>(c, a, i, j, k);
+        for (int i = ia; i <= ib; ++i) Op::template run<GEO, P2>(c, arg, i, j, k);
     }
 }
 
@@ -75,7 +125,7 @@ __global__ void __launch_bounds__(kT, 4)  // the split work at 4 blocks per SM, 
         const int nk = hi[2] - lo[2] + 1;
         if (tl.p0 >= (hi[1] - lo[1] + 1) * nk || tl.i0 > hi[0] || tl.i0 + tile_i - 1 < lo[0]) continue;
         __syncthreads();
-        load_ctx(c, ctxs + tl.inst);
+        load_words(c, ctxs + tl.inst);
         __syncthreads();
         // two threads per cell, as the single-solve k_visc_split: warps 0-3
         // run the heating and forces, warps 4-7 the viscous pressure and CFL
@@ -107,38 +157,114 @@ __global__ void __launch_bounds__(kT, 4)  // the split work at 4 blocks per SM, 
     }
 }
 
-// The z sweep's S6, S7 and S8 as one kernel over whole z lines (the
-// single-solve k_zsweep): each tile is a run of lines of one solve,
-// kThreads / (nz + 4) of them, starting at line p0 of (i, j) in
-// 0..nx x 0..ny.
-template <bool GEO>
-__global__ void __launch_bounds__(ops::kZLineThreads, 4)
-    kb_zsweep(const Ctx *__restrict__ ctxs, const Tile *__restrict__ tiles, int ntiles)
+// The fused phases (bodies in lare_march.cuh) over every live solve's blocks:
+// a persistent grid strides over the phase's block list, staging each block's
+// solve context and tilings in shared memory.
+struct BlockScratch {
+    Ctx c;
+    SolveTiles t;
+};
+template <class F>
+__device__ __forceinline__ void for_blocks(const Ctx *ctxs, const SolveTiles *st, const BlockRef *blocks, int n, F &&run)
 {
-    __shared__ Ctx c;
+    __shared__ BlockScratch sh;
+    for (int q = blockIdx.x; q < n; q += gridDim.x) {
+        const BlockRef r = blocks[q];
+        __syncthreads();
+        load_words(sh.c, ctxs + r.inst);
+        load_words(sh.t, st + r.inst);
+        __syncthreads();
+        run(sh.c, sh.t, r.block);
+    }
+}
+
+#define KB_ARGS const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st, const BlockRef *__restrict__ blocks, int n
+
+template <class P, int WHICH, bool GEO, bool P2>
+__global__ void __launch_bounds__(march::kMThreads, P::kMinBlocks) kb_cellnode(KB_ARGS, int arg)
+{
+    extern __shared__ double ring[];
+    for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
+        march::cellnode<P, GEO, P2>(c, t.cellnode[WHICH], b, arg >= 0 ? arg : c.p.resistive, ring);
+    });
+}
+
+template <bool GEO, bool P2>
+__global__ void __launch_bounds__(march::kMThreads, 3) kb_pred(KB_ARGS)
+{
+    extern __shared__ double ring[];
+    for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
+        march::pred<GEO, P2>(c, t.pred, b, c.p.resistive, c.s[S_CS], c.s[S_CSV], ring);
+    });
+}
+
+template <bool GEO, bool P2>
+__global__ void __launch_bounds__(march::kMThreads, march::kHeatMinBlocks) kb_heat(KB_ARGS)
+{
+    extern __shared__ double ring[];
+    for_blocks(ctxs, st, blocks, n,
+               [&](const Ctx &c, const SolveTiles &t, int b) { march::heat_edges<GEO, P2>(c, t.heat, b, ring); });
+}
+
+template <bool GEO, bool P2>
+__global__ void __launch_bounds__(march::kMThreads, 5) kb_resist(KB_ARGS)
+{
+    extern __shared__ double ring[];
+    for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
+        march::resist<GEO, P2>(c, t.resist, b, c.s[S_CS], c.s[S_CSV], c.s[S_CV1], ring);
+    });
+}
+
+template <int DIR, bool GEO>
+__global__ void __launch_bounds__(ops::kWinThreads, 5) kb_ctmass(KB_ARGS, int scale)
+{
+    extern __shared__ double csm[];
+    for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
+        march::ctmass<DIR, GEO>(c, t.ct[DIR], b, scale, t.images[DIR], csm);
+    });
+}
+
+template <bool GEO>
+__global__ void __launch_bounds__(march::kZCtThreads, 4) kb_ctmass_z(KB_ARGS)
+{
+    __shared__ double zsm[ops::SweepCTMass<2>::NARR * march::kZCtThreads];
+    for_blocks(ctxs, st, blocks, n,
+               [&](const Ctx &c, const SolveTiles &t, int b) { march::ctmass_z<GEO>(c, t.ctz, b, t.images[2], zsm); });
+}
+
+template <int DIR, bool GEO>
+__global__ void __launch_bounds__(ops::kWinThreads, 4) kb_psweep(KB_ARGS, int ct_arg)
+{
+    extern __shared__ double psm[];
+    for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
+        const ops::SweepOut w{c.s[kSweepOut[0]], c.s[kSweepOut[1]], c.s[kSweepOut[2]],
+                              c.s[kSweepOut[3]], c.s[kSweepOut[4]], c.s[kSweepOut[5]]};
+        march::psweep<DIR, GEO>(c, t.stage[DIR], b, w, ct_arg, psm);
+    });
+}
+
+template <bool GEO>
+__global__ void __launch_bounds__(march::kZThreads, 4) kb_zsweep(KB_ARGS, int ct_arg)
+{
     extern __shared__ double zsm[];
-    constexpr int kZT = ops::kZLineThreads;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const Tile tl = tiles[t];
-        __syncthreads();
-        load_ctx(c, ctxs + tl.inst);
-        __syncthreads();
-        const Geom &g = c.g;
-        const int W = g.nz + 4, lines = kZT / W, S = lines * W;
-        const int line = (int)threadIdx.x / W, k = (int)threadIdx.x % W - 2;
-        const long long q = (long long)tl.p0 + line;
-        const bool on = line < lines && q < (long long)(g.nx + 1) * (g.ny + 1);
-        const int i = on ? (int)(q / (g.ny + 1)) : 0, j = on ? (int)(q % (g.ny + 1)) : 0;
-        using F = ops::SweepFused<2>;
-        static_assert(!F::kSharedFluxSlots, "the z passes of stage B run without a barrier between them");
-        const ops::LineStore st{zsm, S, line * W + k + 2};
-        const ops::SweepOut w = ops::sweep_in_place(c);
-        if (on) F::stage_a<GEO>(c, i, j, k, st, w, true);
-        __syncthreads();
-        if (on && k >= 1 && k <= g.nz) F::stage_b_energy(c, i, j, k, st, w);
-        if (on && k >= -1 && k <= g.nz) F::stage_b_mom<GEO>(c, i, j, k, st);  // its own slots: no barrier between
-        __syncthreads();
-        if (on && k >= 0 && k <= g.nz) F::stage_c(c, i, j, k, st, w);
+    for_blocks(ctxs, st, blocks, n,
+               [&](const Ctx &c, const SolveTiles &, int b) { march::zsweep<GEO>(c, b, ct_arg, zsm); });
+}
+#undef KB_ARGS
+
+// The ghost points of the out-of-place sweeps' arrays that no fill rewrites
+// (k_copy_shell of the single solve), for the solves that need it.
+__global__ void __launch_bounds__(kT) kb_copy_shell(const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st,
+                                                    const int *__restrict__ live, int nlive)
+{
+    for (int li = blockIdx.y; li < nlive; li += gridDim.y) {
+        const int inst = live[li];
+        if (st[inst].refilled) continue;
+        const Ctx &c = ctxs[inst];
+        const Geom g = c.g;
+        const ops::SweepOut w{c.s[kSweepOut[0]], c.s[kSweepOut[1]], c.s[kSweepOut[2]],
+                              c.s[kSweepOut[3]], c.s[kSweepOut[4]], c.s[kSweepOut[5]]};
+        ops::copy_shell(c, g, w, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
     }
 }
 
@@ -176,76 +302,69 @@ __device__ __forceinline__ int locate(const long long *off, int n, long long g)
     return lo;
 }
 
-
-// Composite periodic fill (see k_bc_periodic in lare_solver.cu) for every
-// live solve whose fields in `mask` are all-periodic.  The flat index walks
-// the ghost shell of each solve's whole box (-2..n+2 outside the interior
-// 1..n: x slabs, then y slabs inside x, then z slabs inside x and y); a
-// point is decomposed once and then copied for every field whose own range
-// holds it.  The set of points each field receives and their sources are
-// those of the per-field fill.
-__global__ void kb_bc_periodic(const Ctx *__restrict__ ctxs, const int *__restrict__ live,
-                               const unsigned *__restrict__ pfields, const long long *__restrict__ off, int nlive,
-                               long long total, unsigned mask, int resistive_only)
+// Boundary fill of the fields in `mask` for every live solve whose conditions
+// on them can be applied in one pass (SolveTiles::periodic: the composite
+// periodic gather of k_bc_periodic; SolveTiles::compose: bc_compose_value).
+// Each entry of the list is kFillPoints consecutive points of one solve's
+// ghost shell: its whole box -2..n+2 outside 1..n (1..n-1: the half-cell
+// fields' index n is a ghost too), x slabs, then y slabs inside x, then z
+// slabs inside x and y.  A point is decomposed once and then written for every
+// field in whose own range it is a ghost.
+__global__ void __launch_bounds__(kT) kb_bc_fill(const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st,
+                                                 const BcTable *__restrict__ bcs, const BlockRef *__restrict__ blocks, int n,
+                                                 unsigned mask, int resistive_only)
 {
-    for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < total;
-         gi += (long long)gridDim.x * blockDim.x) {
-        const int li = locate(off, nlive, gi);
-        if ((mask & ~pfields[li]) != 0) continue;
-        const Ctx &c = ctxs[live[li]];
+    for (int b = blockIdx.x; b < n; b += gridDim.x) {
+        const BlockRef r = blocks[b];
+        const Ctx &c = ctxs[r.inst];
+        const bool periodic = (mask & ~st[r.inst].periodic) == 0;
+        if (!periodic && (mask & ~st[r.inst].compose) != 0) continue;  // edge by edge (kb_bc_edge)
         if (resistive_only && !c.p.resistive) continue;
         const Geom &g = c.g;
-        const int n0 = g.nx, n1 = g.ny, n2 = g.nz;
-        const int E1 = n1 + 5, E2 = n2 + 5;
-        int t = (int)(gi - off[li]);
         int q0, q1, q2;
-        const int A = 5 * E1 * E2, B = n0 * 5 * E2;
-        if (t < A) {
-            const int gx = t / (E1 * E2), r = t - gx * (E1 * E2);
-            q0 = gx < 3 ? gx - 2 : n0 + gx - 2;
-            q1 = r / E2 - 2;
-            q2 = r - (q1 + 2) * E2 - 2;
-        } else if ((t -= A) < B) {
-            const int i = t / (5 * E2), r = t - i * (5 * E2);
-            const int gy = r / E2;
-            q0 = 1 + i;
-            q1 = gy < 3 ? gy - 2 : n1 + gy - 2;
-            q2 = r - gy * E2 - 2;
-        } else {
-            t -= B;
-            const int i = t / (n1 * 5), r = t - i * (n1 * 5);
-            const int j = r / 5, gz = r - j * 5;
-            q0 = 1 + i;
-            q1 = 1 + j;
-            q2 = gz < 3 ? gz - 2 : n2 + gz - 2;
+        if (!fill_point(g, r.block * kFillPoints + (int)threadIdx.x, q0, q1, q2)) continue;
+        if (periodic) {
+            const int s0 = q0 <= 0 ? q0 + g.nx : (q0 > g.nx ? q0 - g.nx : q0);
+            const int s1 = q1 <= 0 ? q1 + g.ny : (q1 > g.ny ? q1 - g.ny : q1);
+            const int s2 = q2 <= 0 ? q2 + g.nz : (q2 > g.nz ? q2 - g.nz : q2);
+            const int dst = box_off(g, q0, q1, q2), src = box_off(g, s0, s1, s2);
+            if (dst == src) continue;  // (an index n that is no ghost of a centred field, and keeps its value in a half-cell one)
+            for (int f = 0; f < SAMS_NFIELDS; ++f) {
+                if (!(mask & (1u << f))) continue;
+                // centred dimensions start at -1
+                if ((q0 < -1 && !field_half(f, 0)) || (q1 < -1 && !field_half(f, 1)) || (q2 < -1 && !field_half(f, 2)))
+                    continue;
+                double *a = c.f[f];
+                a[dst] = a[src];
+            }
+            continue;
         }
-        const int s0 = q0 <= 0 ? q0 + n0 : (q0 > n0 ? q0 - n0 : q0);
-        const int s1 = q1 <= 0 ? q1 + n1 : (q1 > n1 ? q1 - n1 : q1);
-        const int s2 = q2 <= 0 ? q2 + n2 : (q2 > n2 ? q2 - n2 : q2);
-        const long long dst = box_off(g, q0, q1, q2), src = box_off(g, s0, s1, s2);
+        const BcTable &bt = bcs[r.inst];
         for (int f = 0; f < SAMS_NFIELDS; ++f) {
-            if (!(mask & (1u << f))) continue;
-            // centred dimensions start at -1
-            if ((q0 < -1 && !field_half(f, 0)) || (q1 < -1 && !field_half(f, 1)) || (q2 < -1 && !field_half(f, 2)))
-                continue;
+            if (!(mask & (1u << f)) || !field_ghost(g, f, q0, q1, q2)) continue;
             double *a = c.f[f];
-            a[dst] = a[src];
+            const double v = bc_compose_value<2>(a, g, bt, f, q0, q1, q2);
+            a[box_off(g, q0, q1, q2)] = v;
         }
     }
 }
 
 // One (dimension, edge) of the fields in `mask` for every live solve (those
-// handled by the composite fill are skipped when skip_periodic is set); the
-// point formula and the ordering rule of small dimensions are lare_bc.cuh's.
-__global__ void kb_bc_edge(const Ctx *__restrict__ ctxs, const BcTable *__restrict__ bcs, const int *__restrict__ live,
-                           const unsigned *__restrict__ pfields, const long long *__restrict__ off, int nlive,
-                           long long total, unsigned mask, int d, int e, int skip_periodic, int resistive_only)
+// the one-pass fill, or for dm the CT + mass kernels, have done are skipped);
+// the point formula and the ordering rule of small dimensions are lare_bc.cuh's.
+__global__ void kb_bc_edge(const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st,
+                           const BcTable *__restrict__ bcs, const int *__restrict__ live,
+                           const long long *__restrict__ off, int nlive, long long total, unsigned mask, int d, int e,
+                           int dm_only, int resistive_only)
 {
     for (long long gi = (long long)blockIdx.x * blockDim.x + threadIdx.x; gi < total;
          gi += (long long)gridDim.x * blockDim.x) {
         const int li = locate(off, nlive, gi);
-        if (skip_periodic && (mask & ~pfields[li]) == 0) continue;
         const int inst = live[li];
+        // handled by the CT + mass kernels (dm) or the one-pass fill
+        if (dm_only ? st[inst].images[d] != ops::kNoImages
+                    : (mask & ~st[inst].periodic) == 0 || (mask & ~st[inst].compose) == 0)
+            continue;
         const Ctx &c = ctxs[inst];
         if (resistive_only && !c.p.resistive) continue;
         const BcTable &bt = bcs[inst];
@@ -310,7 +429,7 @@ Batch::~Batch()
     cudaSetDevice(device_);
     drop_graphs();
     for (auto &s : slots_) free_slot(s);
-    cudaFree(d_ctx_);  // one buffer holds every device table
+    cudaFree(d_tables_);
     if (own_stream_) cudaStreamDestroy(own_stream_);
 }
 
@@ -385,13 +504,6 @@ int Batch::add(const sams_lare_params &p, const sams_lare_bcs &bcs, int *id)
     {
         const long long n[3] = {p.nx, p.ny, p.nz};
         if (!bc_table_from(s.bc, bcs, n, &err)) return SAMS_ERR_INVALID;
-    }
-    for (int f = 0; f < SAMS_NFIELDS; ++f) {
-        bool per = true;
-        for (int d = 0; d < 3; ++d)
-            for (int e = 0; e < 2; ++e) per = per && bcs.kind[f][d][e] == SAMS_BC_PERIODIC;
-        // the one-pass periodic gather needs every source inside the domain
-        if (per && std::min(p.nx, std::min(p.ny, p.nz)) >= kBcSequentialBelow) s.periodic_groups |= 1u << f;
     }
     Geom g = batch_geom(p);
     const size_t abytes = (size_t)(SAMS_NFIELDS + NSCRATCH + (p.rke ? 1 : 0)) * (size_t)g.nelem * sizeof(double);
@@ -507,255 +619,391 @@ int Batch::download(int id, int field, double *dst, cudaMemcpyKind kind)
     return check(cudaStreamSynchronize(stream_), "download sync");
 }
 
+// How one solve's phases are cut into blocks and its conditions met.  share:
+// the part of the device that this solve's blocks can count on.
+static SolveTiles solve_tiles(const BatchSlot &s, double share, int sm_count)
+{
+    SolveTiles t{};
+    const Geom &g = s.ctx.g;
+    auto sm = [&](int per_sm) { return std::max(1, (int)(share * per_sm * sm_count)); };
+    t.cellnode[0] = march::march_tile(g.nz + 3, g.ny + 3, g.nx + 3, sm(march::PrepMarch::kMinBlocks));
+    t.pred = march::march_tile(g.nz + 1, g.ny + 1, g.nx + 1, sm(3));
+    t.heat = march::march_tile(g.nz + 2, g.ny + 2, g.nx + 2, sm(march::kHeatMinBlocks));
+    t.resist = march::march_tile(g.nz + 5, g.ny + 5, g.nx + 5, sm(5));
+    for (int d = 0; d < 2; ++d) {
+        const int nd = d == 0 ? g.nx : g.ny, na = d == 0 ? g.ny : g.nx;
+        t.ct[d] = march::win_tile(nd + 1, (long long)(na + 2) * (g.nz + 2), 3, sm(5));
+        t.stage[d] = march::win_tile(nd + 1, (long long)(na + 1) * (g.nz + 1), 3, sm(4));
+    }
+    t.ctz = march::z_tile(g.nz, (long long)(g.nx + 2) * (g.ny + 2));
+    const int n[3] = {g.nx, g.ny, g.nz};
+    const bool three = std::min(n[0], std::min(n[1], n[2])) >= kBcSequentialBelow;
+    t.refilled = three ? 1 : 0;
+    t.b_refilled = three ? 1 : 0;
+    for (int f = 0; f < SAMS_NFIELDS; ++f) {
+        bool per = three, none = false;
+        for (int d = 0; d < 3; ++d)
+            for (int e = 0; e < 2; ++e) {
+                per = per && s.bc.kind[f][d][e] == SAMS_BC_PERIODIC;
+                none = none || s.bc.kind[f][d][e] == SAMS_BC_NONE;
+            }
+        if (per) t.periodic |= 1u << f;
+        if (bc_composable(s.bc, f, n)) t.compose |= 1u << f;
+        // (ghosts_refilled of the single solve)
+        if (none && ((1u << f) & (FM_DENSITY | FM_ENERGY | FM_VELOCITY))) t.refilled = 0;
+        if (none && ((1u << f) & FM_BFIELD)) t.b_refilled = 0;
+    }
+    for (int d = 0; d < 3; ++d) {
+        const int l = s.bc.kind[SAMS_F_DM][d][0], u = s.bc.kind[SAMS_F_DM][d][1];
+        if (n[d] < kBcSequentialBelow || l != u) continue;
+        if (l == SAMS_BC_PERIODIC) t.images[d] = ops::kPeriodicImages;
+        if (l == SAMS_BC_ZERO_GRADIENT) t.images[d] = ops::kCopyImages;
+    }
+    return t;
+}
+
+// The contexts of one solve through a step: scratch arrays and fields trade
+// places after the out-of-place phases exactly as Solver's launches swap them.
+static void solve_contexts(const Ctx &base, bool fused_xy, Ctx out[Batch::NCTX])
+{
+    Ctx c = base;
+    out[Batch::C_START] = c;
+    auto resist_swap = [&] {
+        std::swap(c.f[SAMS_F_BX], c.s[S_CS]);
+        std::swap(c.f[SAMS_F_BY], c.s[S_CSV]);
+        std::swap(c.f[SAMS_F_BZ], c.s[S_CV1]);
+    };
+    if (c.p.resistive) resist_swap();
+    out[Batch::C_SUB] = c;
+    if (c.p.resistive) {
+        resist_swap();
+        std::swap(c.s[S_B1X], c.s[S_CS]);
+        std::swap(c.s[S_B1Y], c.s[S_CSV]);
+        std::swap(c.s[S_B1Z], c.s[S_CV1]);
+    }
+    out[Batch::C_PRED] = c;
+    std::swap(c.s[S_PE], c.s[S_CS]);
+    std::swap(c.s[S_PI], c.s[S_CSV]);
+    out[Batch::C_REMAP] = c;
+    // the out-of-place sweeps read rho itself as rho1
+    static const int kOut[6] = {S_FX, S_FY, S_FZ, S_VH, S_FXV, S_FYV};
+    static const int kState[6] = {SAMS_F_RHO, SAMS_F_ENERGY_ELECTRON, SAMS_F_ENERGY_ION, SAMS_F_VX, SAMS_F_VY, SAMS_F_VZ};
+    out[Batch::C_X] = c;
+    if (fused_xy) {
+        out[Batch::C_X].s[S_R_RHO1] = c.f[SAMS_F_RHO];
+        for (int q = 0; q < 6; ++q) std::swap(c.f[kState[q]], c.s[kOut[q]]);
+    }
+    out[Batch::C_Y] = c;
+    if (fused_xy) out[Batch::C_Y].s[S_R_RHO1] = c.f[SAMS_F_RHO];
+}
+
 int Batch::rebuild()
 {
-    std::vector<Ctx> ctx(slots_.size());
-    std::vector<BcTable> bcs(slots_.size());
+    const size_t nslot = std::max<size_t>(slots_.size(), 1);
+    std::vector<Ctx> ctx(NCTX * nslot);
+    std::vector<BcTable> bcs(nslot);
+    std::vector<SolveTiles> st(nslot);
     std::vector<int> live;
-    std::vector<unsigned> pf;
-    std::vector<long long> shell_off, slab_off[3];
+    std::vector<long long> slab_off[3];
     std::vector<Tile> tiles;
-    long long shell = 0, slab[3] = {0, 0, 0};
-    has_resistive_ = 0;
-    has_rke_ = 0;
-    has_geo_ = 0;
+    std::vector<BlockRef> lists[NPHASE];
+    long long slab[3] = {0, 0, 0};
+    has_resistive_ = has_rke_ = has_geo_ = 0;
     all_pow2_ = 1;
+    fold_ = true;
+    shell_ = edges_ = 0;
+    dm_edges_[0] = dm_edges_[1] = dm_edges_[2] = false;
+    zfuse_ = true;
+    double cells = 0.0;
+    long long elems = 0;
+    for (auto &s : slots_) {
+        if (!s.live) continue;
+        elems += s.ctx.g.nelem;
+        has_rke_ |= s.ctx.p.rke;
+        if (s.ctx.g.nz + 4 > march::kZThreads) zfuse_ = false;
+        cells += (double)(s.p.nx + 5) * (double)(s.p.ny + 5) * (double)(s.p.nz + 5);
+    }
+    fused_xy_ = !has_rke_;
+    zfuse_ = zfuse_ && !has_rke_;
     for (size_t q = 0; q < slots_.size(); ++q) {
-        ctx[q] = slots_[q].ctx;
-        bcs[q] = slots_[q].bc;
-        if (!slots_[q].live) continue;
+        BatchSlot &s = slots_[q];
+        if (!s.live) continue;
+        bcs[q] = s.bc;
+        Ctx cs[NCTX];
+        Ctx base = s.ctx;
+        base.g.far = far_from_l2(elems);
+        solve_contexts(base, fused_xy_, cs);
+        for (int v = 0; v < NCTX; ++v) ctx[(size_t)v * nslot + q] = cs[v];
+        const Geom &g = s.ctx.g;
+        const double share = (double)(s.p.nx + 5) * (double)(s.p.ny + 5) * (double)(s.p.nz + 5) / cells;
+        const SolveTiles t = st[q] = solve_tiles(s, share, sm_count_);
         live.push_back((int)q);
-        pf.push_back(slots_[q].periodic_groups);
-        const Geom &g = slots_[q].ctx.g;
-        has_resistive_ |= slots_[q].ctx.p.resistive;
-        has_rke_ |= slots_[q].ctx.p.rke;
-        has_geo_ |= slots_[q].ctx.p.geometry != 0;
-        all_pow2_ &= slots_[q].ctx.p.pow2;
-        shell_off.push_back(shell);
+        has_resistive_ |= s.ctx.p.resistive;
+        has_geo_ |= s.ctx.p.geometry != 0;
+        all_pow2_ &= s.ctx.p.pow2;
+        fold_ = fold_ && t.b_refilled;
+        if (!t.refilled) shell_ = 1;
+        for (unsigned m : {(unsigned)FM_REMAPV, (unsigned)FM_ALL9})  // (every mask that bc_fill takes is part of one of these)
+            if ((m & ~t.periodic) && (m & ~t.compose)) edges_ = 1;
         const long long e0 = g.nx + 5, e1 = g.ny + 5, e2 = g.nz + 5;
-        shell += 5 * e1 * e2 + (long long)g.nx * 5 * e2 + (long long)g.nx * g.ny * 5;
-        slab_off[0].push_back(slab[0]);
-        slab_off[1].push_back(slab[1]);
-        slab_off[2].push_back(slab[2]);
+        for (int d = 0; d < 3; ++d) {
+            slab_off[d].push_back(slab[d]);
+            if (t.images[d] == ops::kNoImages) dm_edges_[d] = true;
+        }
         slab[0] += 3 * e1 * e2;
         slab[1] += 3 * e0 * e2;
         slab[2] += 3 * e0 * e1;
         const int plane = (int)(e1 * e2);
         for (int i0 = -2; i0 <= g.nx + 2; i0 += tile_i_)
             for (int p0 = 0; p0 < plane; p0 += kT) tiles.push_back(Tile{(int)q, i0, p0, 0});
+        auto blocks = [&](int phase, long long n) {
+            for (long long b = 0; b < n; ++b) lists[phase].push_back(BlockRef{(int)q, (int)b});
+        };
+        blocks(P_CELLNODE, t.cellnode[0].blocks);
+        if (s.ctx.p.resistive) blocks(P_RESIST, t.resist.blocks);
+        blocks(P_PRED, t.pred.blocks);
+        blocks(P_HEAT, t.heat.blocks);
+        blocks(P_CTX, t.ct[0].blocks);
+        blocks(P_CTY, t.ct[1].blocks);
+        blocks(P_CTZ, t.ctz.blocks);
+        blocks(P_STX, t.stage[0].blocks);
+        blocks(P_STY, t.stage[1].blocks);
+        if (zfuse_) {
+            const int lines = march::kZThreads / (g.nz + 4);
+            blocks(P_STZ, ceil_div((long long)(g.nx + 1) * (g.ny + 1), lines));
+        }
+        blocks(P_FILL, ceil_div(fill_points(g), kFillPoints));
     }
     nlive_ = (int)live.size();
     ntiles_ = (int)tiles.size();
-    // z-line tiles of the fused z sweep, after the plane tiles; used when no
-    // solve needs the raw momentum fluxes (rke) and every z line fits a block
-    constexpr int kZT = ops::kZLineThreads;
-    zfuse_ = nlive_ > 0 && !has_rke_;
-    for (int q : live)
-        if (slots_[q].ctx.g.nz + 4 > kZT) zfuse_ = false;
-    if (zfuse_)
-        for (int q : live) {
-            const Geom &g = slots_[q].ctx.g;
-            const int lpb = kZT / (g.nz + 4);
-            const long long nl = (long long)(g.nx + 1) * (g.ny + 1);
-            for (long long first = 0; first < nl; first += lpb) tiles.push_back(Tile{q, 0, (int)first, 0});
-        }
-    nztiles_ = (int)tiles.size() - ntiles_;
-    shell_total_ = shell;
     for (int d = 0; d < 3; ++d) slab_total_[d] = slab[d];
     // one device buffer for all tables
-    const size_t nslot = slots_.size() ? slots_.size() : 1;
-    const size_t need = nslot * sizeof(Ctx) + nslot * sizeof(BcTable) + std::max<size_t>(tiles.size(), 1) * sizeof(Tile) +
-                        (size_t)std::max(nlive_, 1) * (sizeof(int) + sizeof(unsigned) + 4 * sizeof(long long)) + 1024;
+    size_t off = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = off;
+        off += (std::max<size_t>(bytes, 16) + 15) / 16 * 16;
+        return at;
+    };
+    const size_t o_ctx = place(ctx.size() * sizeof(Ctx)), o_bc = place(bcs.size() * sizeof(BcTable));
+    const size_t o_st = place(st.size() * sizeof(SolveTiles)), o_tiles = place(tiles.size() * sizeof(Tile));
+    const size_t o_live = place(live.size() * sizeof(int));
+    const size_t o_slab = place(3 * live.size() * sizeof(long long));
+    size_t o_list[NPHASE];
+    for (int ph = 0; ph < NPHASE; ++ph) o_list[ph] = place(lists[ph].size() * sizeof(BlockRef));
     int rc;
-    if (need > table_cap_bytes_) {
-        cudaFree(d_ctx_);
-        d_ctx_ = nullptr;
-        size_t cap = need * 2;
-        if ((rc = check(cudaMalloc((void **)&d_ctx_, cap), "cudaMalloc(batch tables)"))) return rc;
+    if (off > table_cap_bytes_) {
+        cudaFree(d_tables_);
+        d_tables_ = nullptr;
+        table_cap_bytes_ = 0;
+        const size_t cap = off * 2;
+        if ((rc = check(cudaMalloc((void **)&d_tables_, cap), "cudaMalloc(batch tables)"))) return rc;
         table_cap_bytes_ = cap;
     }
-    char *base = reinterpret_cast<char *>(d_ctx_);
-    size_t o = nslot * sizeof(Ctx);
-    d_bc_ = reinterpret_cast<BcTable *>(base + o);
-    BcTable *d_bc = d_bc_;
-    o += nslot * sizeof(BcTable);
-    o = (o + 15) / 16 * 16;
-    d_tiles_ = reinterpret_cast<Tile *>(base + o);
-    o += std::max<size_t>(tiles.size(), 1) * sizeof(Tile);
-    o = (o + 15) / 16 * 16;
-    d_live_ = reinterpret_cast<int *>(base + o);
-    o += (size_t)std::max(nlive_, 1) * sizeof(int);
-    o = (o + 15) / 16 * 16;
-    d_pf_ = reinterpret_cast<unsigned *>(base + o);
-    unsigned *d_pf = d_pf_;
-    o += (size_t)std::max(nlive_, 1) * sizeof(unsigned);
-    o = (o + 15) / 16 * 16;
-    d_shell_off_ = reinterpret_cast<long long *>(base + o);
-    o += (size_t)std::max(nlive_, 1) * sizeof(long long);
-    d_slab_off_ = reinterpret_cast<long long *>(base + o);
-    (void)d_bc;
-    (void)d_pf;
-    auto cp = [&](void *dst, const void *src, size_t n) {
-        return n ? check(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, stream_), "batch tables") : SAMS_OK;
-    };
-    if ((rc = cp(d_ctx_, ctx.data(), ctx.size() * sizeof(Ctx)))) return rc;
-    if ((rc = cp(d_bc, bcs.data(), bcs.size() * sizeof(BcTable)))) return rc;
-    if ((rc = cp(d_tiles_, tiles.data(), tiles.size() * sizeof(Tile)))) return rc;
-    if ((rc = cp(d_live_, live.data(), live.size() * sizeof(int)))) return rc;
-    if ((rc = cp(d_pf, pf.data(), pf.size() * sizeof(unsigned)))) return rc;
-    if ((rc = cp(d_shell_off_, shell_off.data(), shell_off.size() * sizeof(long long)))) return rc;
-    for (int d = 0; d < 3; ++d)
-        if ((rc = cp(d_slab_off_ + (size_t)d * std::max(nlive_, 1), slab_off[d].data(),
-                     slab_off[d].size() * sizeof(long long))))
-            return rc;
+    std::vector<char> host(off);
+    auto put = [&](size_t at, const void *src, size_t n) { if (n) std::memcpy(host.data() + at, src, n); };
+    put(o_ctx, ctx.data(), ctx.size() * sizeof(Ctx));
+    put(o_bc, bcs.data(), bcs.size() * sizeof(BcTable));
+    put(o_st, st.data(), st.size() * sizeof(SolveTiles));
+    put(o_tiles, tiles.data(), tiles.size() * sizeof(Tile));
+    put(o_live, live.data(), live.size() * sizeof(int));
+    for (int d = 0; d < 3; ++d) put(o_slab + d * live.size() * sizeof(long long), slab_off[d].data(), live.size() * sizeof(long long));
+    for (int v = 0; v < NCTX; ++v) d_ctx_[v] = reinterpret_cast<Ctx *>(d_tables_ + o_ctx) + (size_t)v * nslot;
+    d_bc_ = reinterpret_cast<BcTable *>(d_tables_ + o_bc);
+    d_st_ = reinterpret_cast<SolveTiles *>(d_tables_ + o_st);
+    d_tiles_ = reinterpret_cast<Tile *>(d_tables_ + o_tiles);
+    d_live_ = reinterpret_cast<int *>(d_tables_ + o_live);
+    d_slab_off_ = reinterpret_cast<long long *>(d_tables_ + o_slab);
+    for (int ph = 0; ph < NPHASE; ++ph) {
+        put(o_list[ph], lists[ph].data(), lists[ph].size() * sizeof(BlockRef));
+        d_list_[ph] = reinterpret_cast<BlockRef *>(d_tables_ + o_list[ph]);
+        nlist_[ph] = (int)lists[ph].size();
+    }
+    if ((rc = check(cudaMemcpyAsync(d_tables_, host.data(), off, cudaMemcpyHostToDevice, stream_), "batch tables"))) return rc;
     dirty_ = false;
-    // keep the host-side copies alive until the async copies are done
+    // keep the host-side copy alive until the async copy is done
     return check(cudaStreamSynchronize(stream_), "batch tables sync");
 }
 
 template <class Op>
-void Batch::launch(int arg, bool resistive_only)
+void Batch::launch(int ctx, int arg)
 {
     if (ntiles_ == 0) return;
     const int grid = std::min(ntiles_, sm_count_ * blocks_per_sm_);
-    const int ro = resistive_only ? 1 : 0;
     if (has_geo_)
-        kb_op<Op, true, false><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, arg, tile_i_, ro);
+        kb_op<Op, true, false><<<grid, kT, 0, stream_>>>(d_ctx_[ctx], d_tiles_, ntiles_, arg, tile_i_);
     else if (all_pow2_)
-        kb_op<Op, false, true><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, arg, tile_i_, ro);
+        kb_op<Op, false, true><<<grid, kT, 0, stream_>>>(d_ctx_[ctx], d_tiles_, ntiles_, arg, tile_i_);
     else
-        kb_op<Op, false, false><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, arg, tile_i_, ro);
-}
-
-void Batch::launch_zsweep()
-{
-    if (nztiles_ == 0) return;
-    constexpr int kZT = ops::kZLineThreads;
-    const int grid = std::min(nztiles_, sm_count_ * 4);
-    const size_t smem = (size_t)ops::SweepFused<2>::NARR * kZT * sizeof(double);
-    if (has_geo_)
-        kb_zsweep<true><<<grid, kZT, smem, stream_>>>(d_ctx_, d_tiles_ + ntiles_, nztiles_);
-    else
-        kb_zsweep<false><<<grid, kZT, smem, stream_>>>(d_ctx_, d_tiles_ + ntiles_, nztiles_);
+        kb_op<Op, false, false><<<grid, kT, 0, stream_>>>(d_ctx_[ctx], d_tiles_, ntiles_, arg, tile_i_);
 }
 
 void Batch::launch_visc()
 {
     if (ntiles_ == 0) return;
     const int grid = std::min(ntiles_, sm_count_ * blocks_per_sm_);
+    const Ctx *c = d_ctx_[C_START];
     if (has_geo_)
-        kb_visc<true, false><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, tile_i_);
+        kb_visc<true, false><<<grid, kT, 0, stream_>>>(c, d_tiles_, ntiles_, tile_i_);
     else if (all_pow2_)
-        kb_visc<false, true><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, tile_i_);
+        kb_visc<false, true><<<grid, kT, 0, stream_>>>(c, d_tiles_, ntiles_, tile_i_);
     else
-        kb_visc<false, false><<<grid, kT, 0, stream_>>>(d_ctx_, d_tiles_, ntiles_, tile_i_);
+        kb_visc<false, false><<<grid, kT, 0, stream_>>>(c, d_tiles_, ntiles_, tile_i_);
 }
 
-void Batch::bc_fill(unsigned mask, bool resistive_only)
+// A fused phase over its block list: `per_sm` blocks per SM (the kernel's
+// register cap), each striding over the list.
+#define FUSED_ARGS d_ctx_[ctx], d_st_, d_list_[ph], nlist_[ph]
+#define FUSED_LAUNCH(kernel, per_sm, threads, smem, ...)                                                            \
+    if (nlist_[ph]) kernel<<<std::min(nlist_[ph], sm_count_ * (per_sm)), threads, smem, stream_>>>(FUSED_ARGS, ##__VA_ARGS__)
+#define FUSED_GP(kernel, per_sm, smem, ...)                                                                         \
+    if (has_geo_) { FUSED_LAUNCH((kernel<true, false>), per_sm, march::kMThreads, smem, ##__VA_ARGS__); }           \
+    else if (all_pow2_) { FUSED_LAUNCH((kernel<false, true>), per_sm, march::kMThreads, smem, ##__VA_ARGS__); }     \
+    else { FUSED_LAUNCH((kernel<false, false>), per_sm, march::kMThreads, smem, ##__VA_ARGS__); }
+
+constexpr size_t kPlaneBytes = 3 * march::kRP * sizeof(double);  // one ring array
+
+template <class P>
+void Batch::launch_cellnode(int ctx, int arg)
 {
-    if (nlive_ == 0) return;
-    const BcTable *d_bc = d_bc_;
-    const unsigned *d_pf = d_pf_;
-    const int grid = (int)std::min<long long>(ceil_div(shell_total_, kT), (long long)sm_count_ * 8);
-    kb_bc_periodic<<<grid, kT, 0, stream_>>>(d_ctx_, d_live_, d_pf, d_shell_off_, nlive_, shell_total_, mask,
-                                             resistive_only ? 1 : 0);
-    bool any_general = false;
-    for (auto &s : slots_)
-        if (s.live && (mask & ~s.periodic_groups)) any_general = true;
-    if (!any_general) return;
-    for (int d = 0; d < 3; ++d)
-        for (int e = 0; e < 2; ++e) {
-            const int g2 = (int)std::min<long long>(ceil_div(slab_total_[d], kT), (long long)sm_count_ * 8);
-            kb_bc_edge<<<g2, kT, 0, stream_>>>(d_ctx_, d_bc, d_live_, d_pf, d_slab_off_ + (size_t)d * std::max(nlive_, 1),
-                                               nlive_, slab_total_[d], mask, d, e, 1, resistive_only ? 1 : 0);
-        }
+    const int ph = P_CELLNODE;
+    const size_t smem = P::NR * kPlaneBytes;
+    if (has_geo_) { FUSED_LAUNCH((kb_cellnode<P, 0, true, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
+    else if (all_pow2_) { FUSED_LAUNCH((kb_cellnode<P, 0, false, true>), P::kMinBlocks, march::kMThreads, smem, arg); }
+    else { FUSED_LAUNCH((kb_cellnode<P, 0, false, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
 }
 
-void Batch::bc_fill_dim(unsigned mask, int d, bool resistive_only)
+void Batch::launch_resist(int ctx)
 {
-    if (nlive_ == 0) return;
-    const BcTable *d_bc = d_bc_;
-    const unsigned *d_pf = d_pf_;
+    const int ph = P_RESIST;
+    FUSED_GP(kb_resist, 5, ops::ResistRK::NOUT * kPlaneBytes);
+}
+
+void Batch::launch_pred(int ctx)
+{
+    const int ph = P_PRED;
+    FUSED_GP(kb_pred, 3, march::PredRingSrc::NR * kPlaneBytes);
+}
+
+void Batch::launch_heat(int ctx)
+{
+    const int ph = P_HEAT;
+    FUSED_GP(kb_heat, march::kHeatMinBlocks, 3 * kPlaneBytes);
+}
+
+template <int DIR>
+void Batch::launch_ctmass(int ctx, int scale)
+{
+    const int ph = DIR == 0 ? P_CTX : (DIR == 1 ? P_CTY : P_CTZ);
+    if constexpr (DIR == 2) {
+        (void)scale;
+        if (has_geo_) { FUSED_LAUNCH(kb_ctmass_z<true>, 4, march::kZCtThreads, 0); }
+        else { FUSED_LAUNCH(kb_ctmass_z<false>, 4, march::kZCtThreads, 0); }
+    } else {
+        const size_t smem = (size_t)ops::SweepCTMass<DIR>::NARR * march::kCtP * ops::kWinK * sizeof(double);
+        if (has_geo_) { FUSED_LAUNCH((kb_ctmass<DIR, true>), 5, ops::kWinThreads, smem, scale); }
+        else { FUSED_LAUNCH((kb_ctmass<DIR, false>), 5, ops::kWinThreads, smem, scale); }
+    }
+    if (dm_edges_[DIR]) bc_edges(ctx, FM_DM, DIR, true, false);
+}
+
+template <int DIR>
+void Batch::launch_psweep(int ctx, int ct_arg)
+{
+    const int ph = DIR == 0 ? P_STX : P_STY;
+    const size_t smem = (size_t)ops::SweepFused<DIR>::NARR * ops::WinStore::P * ops::kWinK * sizeof(double);
+    if (has_geo_) { FUSED_LAUNCH((kb_psweep<DIR, true>), 4, ops::kWinThreads, smem, ct_arg); }
+    else { FUSED_LAUNCH((kb_psweep<DIR, false>), 4, ops::kWinThreads, smem, ct_arg); }
+    if (shell_) kb_copy_shell<<<dim3(64, (unsigned)std::min(nlive_, 1024)), kT, 0, stream_>>>(d_ctx_[ctx], d_st_, d_live_, nlive_);
+}
+
+void Batch::launch_zsweep(int ctx, int ct_arg)
+{
+    const int ph = P_STZ;
+    const size_t smem = (size_t)ops::SweepFused<2>::NARR * march::kZThreads * sizeof(double);
+    if (has_geo_) { FUSED_LAUNCH(kb_zsweep<true>, 4, march::kZThreads, smem, ct_arg); }
+    else { FUSED_LAUNCH(kb_zsweep<false>, 4, march::kZThreads, smem, ct_arg); }
+}
+
+void Batch::bc_edges(int ctx, unsigned mask, int d, bool dm_only, bool resistive_only)
+{
     const int g2 = (int)std::min<long long>(ceil_div(slab_total_[d], kT), (long long)sm_count_ * 8);
     for (int e = 0; e < 2; ++e)
-        kb_bc_edge<<<g2, kT, 0, stream_>>>(d_ctx_, d_bc, d_live_, d_pf, d_slab_off_ + (size_t)d * std::max(nlive_, 1),
-                                           nlive_, slab_total_[d], mask, d, e, 0, resistive_only ? 1 : 0);
+        kb_bc_edge<<<g2, kT, 0, stream_>>>(d_ctx_[ctx], d_st_, d_bc_, d_live_, d_slab_off_ + (size_t)d * nlive_, nlive_,
+                                           slab_total_[d], mask, d, e, dm_only ? 1 : 0, resistive_only ? 1 : 0);
 }
 
+void Batch::bc_fill(int ctx, unsigned mask, bool resistive_only)
+{
+    if (nlive_ == 0) return;
+    const int n = nlist_[P_FILL];
+    kb_bc_fill<<<std::min(n, sm_count_ * 8), kT, 0, stream_>>>(d_ctx_[ctx], d_st_, d_bc_, d_list_[P_FILL], n, mask,
+                                                               resistive_only ? 1 : 0);
+    if (edges_)
+        for (int d = 0; d < 3; ++d) bc_edges(ctx, mask, d, false, resistive_only);
+}
+
+// The same phases in the same order as Solver::enqueue_step.
 void Batch::enqueue_step()
 {
+    if (nlive_ == 0) return;
     // ---- Lagrangian predictor ----
-    launch<ops::CellPrep>(-1, false);
-    launch<ops::NodePrep>(0, false);
-    launch<ops::Alpha>(0, false);
+    launch_cellnode<march::PrepMarch>(C_START, -1);
+    launch<ops::Alpha>(C_START, 0);
     launch_visc();
-    if (nlive_) kb_dt_finalize<<<(unsigned)ceil_div(nlive_, 128), 128, 0, stream_>>>(d_ctx_, d_live_, nlive_);
+    kb_dt_finalize<<<(unsigned)ceil_div(nlive_, 128), 128, 0, stream_>>>(d_ctx_[C_START], d_live_, nlive_);
     if (has_resistive_) {
-        for (int sub = 0; sub < 2; ++sub) {
-            launch<ops::ResistRK>(0, true);
-            launch<ops::ResistB>(sub == 1 ? 1 : 0, true);
-            bc_fill(FM_BFIELD | FM_ENERGY, true);
-        }
+        launch_resist(C_START);
+        bc_fill(C_SUB, FM_BFIELD | FM_ENERGY, true);
+        launch_resist(C_SUB);
+        bc_fill(C_PRED, FM_BFIELD | FM_ENERGY, true);
     }
-    launch<ops::Pred1>(-1, false);
-    launch<ops::Pred2>(0, false);
-    bc_fill(FM_REMAPV, false);
+    launch_pred(C_PRED);
+    bc_fill(C_REMAP, FM_REMAPV, false);
     // ---- corrector ----
-    launch<ops::Corr1>(0, false);
-    launch<ops::Corr2>(0, false);
-    bc_fill(FM_VELOCITY | FM_ENERGY | FM_DENSITY, false);
+    launch_heat(C_REMAP);
+    launch<ops::Corr2>(C_REMAP, 0);
+    bc_fill(C_REMAP, FM_VELOCITY | FM_ENERGY | FM_DENSITY, false);
     // ---- remap ----
-    if (has_rke_) launch<ops::RkeZero>(0, false);
-    launch<ops::BScale>(0, false);
-    launch<ops::SweepVol<0>>(0, false);
-    launch<ops::SweepCvc>(0, false);
-    launch<ops::SweepCT<0>>(0, false);
-    launch<ops::SweepCTUpd<0>>(0, false);
-    launch<ops::SweepMass<0>>(0, false);
-    bc_fill_dim(FM_DM, 0, false);
-    launch<ops::SweepS6<0>>(0, false);
-    launch<ops::SweepS7<0>>(0, false);
-    if (has_rke_) {  // solves without rke return at once (Phys::rke)
-        launch<ops::SweepRkeDk<0>>(0, false);
-        launch<ops::SweepRkeGather<0>>(0, false);
+    if (has_rke_) launch<ops::RkeZero>(C_REMAP, 0);
+    if (!fold_) launch<ops::BScale>(C_REMAP, 0);
+    launch_cellnode<march::VolMarch<0>>(C_X, fused_xy_ ? 1 : 0);
+    launch_ctmass<0>(C_X, fold_ ? 1 : 0);
+    launch<ops::SweepCTUpd<0>>(C_X, fold_ ? 1 : 0);
+    stages<0>(C_X, 0, false);
+    bc_fill(C_Y, FM_ALL9, false);
+    launch_cellnode<march::VolMarch<1>>(C_Y, fused_xy_ ? 1 : 0);
+    launch_ctmass<1>(C_Y, 0);
+    stages<1>(C_Y, 0, true);
+    bc_fill(C_REMAP, FM_ALL9, false);
+    launch_cellnode<march::VolMarch<2>>(C_REMAP, 0);
+    launch_ctmass<2>(C_REMAP, 0);
+    stages<2>(C_REMAP, fold_ ? 2 : 0, true);
+    bc_fill(C_REMAP, FM_ALL9, false);
+    if (!fold_) {
+        launch<ops::BScale>(C_REMAP, 1);
+        bc_fill(C_REMAP, FM_BFIELD, false);
     }
-    launch<ops::SweepS8<0>>(0, false);
-    bc_fill(FM_ALL9, false);
-    launch<ops::SweepVol<1>>(0, false);
-    launch<ops::SweepCvc>(0, false);
-    launch<ops::SweepCT<1>>(0, false);
-    launch<ops::SweepCTUpd<1>>(0, false);
-    launch<ops::SweepMass<1>>(0, false);
-    bc_fill_dim(FM_DM, 1, false);
-    launch<ops::SweepS6<1>>(0, false);
-    launch<ops::SweepS7<1>>(0, false);
-    if (has_rke_) {  // solves without rke return at once (Phys::rke)
-        launch<ops::SweepRkeDk<1>>(0, false);
-        launch<ops::SweepRkeGather<1>>(0, false);
-    }
-    launch<ops::SweepS8<1>>(0, false);
-    bc_fill(FM_ALL9, false);
-    launch<ops::SweepVol<2>>(0, false);
-    launch<ops::SweepCvc>(0, false);
-    launch<ops::SweepCT<2>>(0, false);
-    launch<ops::SweepCTUpd<2>>(0, false);
-    launch<ops::SweepMass<2>>(0, false);
-    bc_fill_dim(FM_DM, 2, false);
-    if (zfuse_) {
-        launch_zsweep();
+    if (has_rke_) launch<ops::RkeEnergy>(C_REMAP, 0);
+}
+
+// S6-S8 of one sweep: fused, with the sweep's CT update (where `update` asks
+// for it) at the same points, or the separate kernels.
+template <int DIR>
+void Batch::stages(int ctx, int ct_arg, bool update)
+{
+    if constexpr (DIR == 2) {
+        if (zfuse_) return launch_zsweep(ctx, ct_arg);
     } else {
-        launch<ops::SweepS6<2>>(0, false);
-        launch<ops::SweepS7<2>>(0, false);
-        if (has_rke_) {  // solves without rke return at once (Phys::rke)
-            launch<ops::SweepRkeDk<2>>(0, false);
-            launch<ops::SweepRkeGather<2>>(0, false);
-        }
-        launch<ops::SweepS8<2>>(0, false);
+        if (fused_xy_) return launch_psweep<DIR>(ctx, update ? ct_arg : -1);
     }
-    bc_fill(FM_ALL9, false);
-    launch<ops::BScale>(1, false);
-    bc_fill(FM_BFIELD, false);
-    if (has_rke_) launch<ops::RkeEnergy>(0, false);
+    if (update) launch<ops::SweepCTUpd<DIR>>(ctx, ct_arg);
+    launch<ops::SweepS6<DIR>>(ctx, 0);
+    launch<ops::SweepS7<DIR>>(ctx, 0);
+    if (has_rke_) {  // solves without rke return at once (Phys::rke)
+        launch<ops::SweepRkeDk<DIR>>(ctx, 0);
+        launch<ops::SweepRkeGather<DIR>>(ctx, 0);
+    }
+    launch<ops::SweepS8<DIR>>(ctx, 0);
 }
 
 int Batch::step(long long nsteps)

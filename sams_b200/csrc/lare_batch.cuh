@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "lare_device.cuh"
+#include "lare_march.cuh"
 #include "lare_solver.cuh"
 #include "sams_lare.h"
 
@@ -28,6 +29,21 @@ struct Tile {
     int pad;
 };
 
+// One block of a fused phase: of which solve, and which of its blocks.
+struct BlockRef {
+    int inst, block;
+};
+
+// One solve's tilings of the fused phases and how its ghosts are filled.
+struct SolveTiles {
+    march::MarchTile cellnode[1], pred, heat, resist;
+    march::WinTile ct[2], stage[2];
+    march::ZTile ctz;
+    int images[3];              // what the CT + mass kernels write of dm's ghosts, per sweep
+    int refilled, b_refilled;   // a fill rewrites every ghost of rho, energies and velocities; of B
+    unsigned periodic, compose; // fields that the one-pass fills take (bit per field)
+};
+
 struct BatchSlot {
     bool live = false;
     sams_lare_params p{};
@@ -37,7 +53,6 @@ struct BatchSlot {
     double *axes = nullptr;
     Scalars *sc = nullptr;
     long long bytes = 0;
-    unsigned periodic_groups = 0;  // bit g set: field group g all-periodic
 };
 
 class Batch {
@@ -68,15 +83,27 @@ public:
 
     std::string err;
 
+    // Contexts of a solve through a step (the out-of-place phases trade
+    // arrays): at its start, after the first resistive sub-step, after the
+    // last, from the corrector on, and in the x and y sweeps.
+    enum { C_START, C_SUB, C_PRED, C_REMAP, C_X, C_Y, NCTX };
+
 private:
     int check(cudaError_t e, const char *what);
     int rebuild();
     void enqueue_step();
-    template <class Op> void launch(int arg, bool resistive_only);
+    template <class Op> void launch(int ctx, int arg);
     void launch_visc();
-    void launch_zsweep();
-    void bc_fill(unsigned mask, bool resistive_only);
-    void bc_fill_dim(unsigned mask, int dim, bool resistive_only);
+    template <class P> void launch_cellnode(int ctx, int arg);
+    void launch_resist(int ctx);
+    void launch_pred(int ctx);
+    void launch_heat(int ctx);
+    template <int DIR> void launch_ctmass(int ctx, int scale);
+    template <int DIR> void launch_psweep(int ctx, int ct_arg);
+    void launch_zsweep(int ctx, int ct_arg);
+    template <int DIR> void stages(int ctx, int ct_arg, bool update);
+    void bc_fill(int ctx, unsigned mask, bool resistive_only);
+    void bc_edges(int ctx, unsigned mask, int d, bool dm_only, bool resistive_only);
     void drop_graphs();
     void free_slot(BatchSlot &s);
 
@@ -88,18 +115,25 @@ private:
     int tile_i_ = 2;
     int blocks_per_sm_ = 4;
     int sm_count_ = 148;
-    // device tables (rebuilt when the set of solves changes)
-    Ctx *d_ctx_ = nullptr;
-    Tile *d_tiles_ = nullptr;  // plane tiles, then (when zfuse_) the z-line tiles
+    // device tables, one buffer (rebuilt when the set of solves changes)
+    char *d_tables_ = nullptr;
+    Ctx *d_ctx_[NCTX] = {};
+    Tile *d_tiles_ = nullptr;  // plane tiles of the per-point phases
     int ntiles_ = 0;
-    int nztiles_ = 0;
-    bool zfuse_ = false;  // the z sweep's S6-S8 run as one kernel (kb_zsweep)
+    SolveTiles *d_st_ = nullptr;
+    enum { P_CELLNODE, P_RESIST, P_PRED, P_HEAT, P_CTX, P_CTY, P_CTZ, P_STX, P_STY, P_STZ, P_FILL, NPHASE };
+    BlockRef *d_list_[NPHASE] = {};  // blocks of the fused phases
+    int nlist_[NPHASE] = {};
+    bool fused_xy_ = false;  // the x and y sweeps' S6-S8 run as one kernel (no live solve uses rke)
+    bool zfuse_ = false;     // ... the z sweep's (and every z line fits a block)
+    bool fold_ = false;      // B's scaling is folded into the x and z sweeps' CT updates
+    int shell_ = 0;          // some solve's ghosts outlive a fill: the out-of-place sweeps copy them
+    int edges_ = 0;          // some solve has conditions that no one-pass fill takes
+    bool dm_edges_[3] = {};  // some solve's dm is filled by kb_bc_edge along this dimension
     int *d_live_ = nullptr;
-    unsigned *d_pf_ = nullptr;          // per live solve: fields that are all-periodic
     BcTable *d_bc_ = nullptr;           // per slot boundary conditions
-    long long *d_shell_off_ = nullptr;  // prefix of ghost-shell points per live solve
     long long *d_slab_off_ = nullptr;   // 3 x prefix of one-edge slab points per live solve
-    long long shell_total_ = 0, slab_total_[3] = {0, 0, 0};
+    long long slab_total_[3] = {0, 0, 0};
     int nlive_ = 0;
     int has_resistive_ = 0;
     int has_rke_ = 0;

@@ -1500,6 +1500,32 @@ __device__ __forceinline__ SweepOut sweep_in_place(const Ctx &c)
                     c.f[SAMS_F_VX], c.f[SAMS_F_VY], c.f[SAMS_F_VZ]};
 }
 
+// The ghost points of an out-of-place sweep's arrays (rho and energies
+// outside 1..n, velocities outside 0..n in some dimension), shell points
+// t, t + stride, ..: copied from the solve's arrays, first the rho and energy
+// shell, then the velocity shell.
+__device__ __forceinline__ void copy_shell(const Ctx &c, const Geom &g, const SweepOut &w, long long t, long long stride)
+{
+    const BoxShell cell{{g.nx, g.ny, g.nz}, 1, 0}, node{{g.nx, g.ny, g.nz}, 0, 0};
+    const long long nc = cell.count(), n = nc + node.count();
+    for (; t < n; t += stride) {
+        int i, j, k;
+        if (t < nc) {
+            cell.point(t, i, j, k);
+            const int o = box_off(g, i, j, k);
+            w.rho[o] = c.f[SAMS_F_RHO][o];
+            w.ee[o] = c.f[SAMS_F_ENERGY_ELECTRON][o];
+            w.ei[o] = c.f[SAMS_F_ENERGY_ION][o];
+        } else {
+            node.point(t - nc, i, j, k);
+            const int o = box_off(g, i, j, k);
+            w.ux[o] = c.f[SAMS_F_VX][o];
+            w.uy[o] = c.f[SAMS_F_VY][o];
+            w.uz[o] = c.f[SAMS_F_VZ][o];
+        }
+    }
+}
+
 // SweepS6, SweepS7 and SweepS8 of one sweep as three stages of one kernel.
 // Every value a stage passes to the next (energy fluxes, vertex density,
 // node dm, momentum fluxes) is read only along the sweep direction on the

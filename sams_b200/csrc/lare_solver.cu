@@ -130,26 +130,7 @@ __global__ void __launch_bounds__(kZThreads, 4) k_zsweep(Ctx c, int ct_arg)  // 
 // thread per shell point: the rho / energy shell, then the velocity shell.
 __global__ void __launch_bounds__(kThreads) k_copy_shell(Ctx c, ops::SweepOut w)
 {
-    const Geom &g = c.g;
-    const BoxShell cell{{g.nx, g.ny, g.nz}, 1, 0}, node{{g.nx, g.ny, g.nz}, 0, 0};
-    const long long nc = cell.count(), n = nc + node.count();
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        if (t < nc) {
-            cell.point(t, i, j, k);
-            const int o = box_off(g, i, j, k);
-            w.rho[o] = c.f[SAMS_F_RHO][o];
-            w.ee[o] = c.f[SAMS_F_ENERGY_ELECTRON][o];
-            w.ei[o] = c.f[SAMS_F_ENERGY_ION][o];
-        } else {
-            node.point(t - nc, i, j, k);
-            const int o = box_off(g, i, j, k);
-            w.ux[o] = c.f[SAMS_F_VX][o];
-            w.uy[o] = c.f[SAMS_F_VY][o];
-            w.uz[o] = c.f[SAMS_F_VZ][o];
-        }
-    }
+    ops::copy_shell(c, c.g, w, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
 
 // Visc with two threads per cell: a block holds 128 consecutive (j, k)
