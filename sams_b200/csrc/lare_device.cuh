@@ -16,6 +16,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "lare_div.cuh"
 #include "sams_lare_layout.h"
 
 namespace sams {
@@ -196,19 +197,70 @@ struct RO {
     __device__ __forceinline__ double operator[](int i) const { return __ldg(p + i); }
 };
 
-// x / d, or x * r where the kernel is built for a power-of-two grid (r = 1/d
-// exactly; see Recip).
-template <bool P2>
-__device__ __forceinline__ double div_by(double x, double d, double r)
-{
-    if constexpr (P2) {
-        (void)d;
-        return x * r;
-    } else {
-        (void)r;
-        return x / d;
+// How an op divides.  FastDiv: straight-line (lare_div.cuh); `bad` says that
+// some quotient may not be the IEEE one, and the caller then runs the op again
+// with IeeeDiv before anything it reads has been overwritten.  of() takes a
+// denominator, the call divides by it; pair() is the sum of two quotients of
+// non-negative numerators and fraction() x / d, x not negative, where a result below 2^-600,
+// added to or taken from one or two, may be anything below that.
+//
+// With IEEE divisions throughout, each a branch to its slow path that loads
+// do not move past, against now (us, 256^3 power-of-two grid / 96^3):
+// predictor 1451 / 154 -> 1233 / 129, x stages 1239 / 85 -> 1051 / 71, y stages
+// 1367 / 93 -> 1198 / 81, z stages 1367 / 116 -> 1257 / 86, edge viscosity
+// 866 / 52 -> 767 / 48, corrector 597 / 38 -> 540 / 32; k_visc_split
+// (three blocks per SM) 1090 / 86 -> 1040 / 73.
+struct IeeeDiv {
+    static constexpr bool kFast = false;
+    static constexpr bool bad = false;
+    struct R {
+        double d;
+    };
+    __device__ __forceinline__ R of(double d) { return R{d}; }
+    __device__ __forceinline__ double operator()(double x, const R &r) { return x / r.d; }
+    __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q) { return x / r.d + y / q.d; }
+    __device__ __forceinline__ double fraction(double x, const R &r) { return x / r.d; }
+    __device__ __forceinline__ void finite(double) {}
+};
+struct FastDiv {
+    static constexpr bool kFast = true;
+    bool bad = false;
+    using R = Rcp;
+    __device__ __forceinline__ R of(double d)
+    {
+        bad = bad || !plain_divisor(d);
+        return rcp_of(d);
     }
-}
+    __device__ __forceinline__ double operator()(double x, const R &r) { return quot_check(x, r, bad); }
+    __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q)
+    {
+        const double s = quot(x, r) + quot(y, q);
+        const bool zero = ((high_word(x) << 1) | low_word(x) | (high_word(y) << 1) | low_word(y)) == 0;
+        bad = bad || (!quot_in_range(s) && !zero);
+        return s;
+    }
+    __device__ __forceinline__ double fraction(double x, const R &r) { return quot(x, r); }
+    // (an infinity or NaN out of fraction() is left to the IEEE run)
+    __device__ __forceinline__ void finite(double q) { bad = bad || (high_word(q) & 0x7fffffffu) >= 0x7ff00000u; }
+};
+
+// A denominator made of spacings: on power-of-two grids (P2) the product with
+// its exact reciprocal r (Recip), elsewhere the division.
+template <bool P2, class DV>
+struct By {
+    typename DV::R R;
+    double r;
+    __device__ __forceinline__ By(DV &dv, double d, double r_)
+    {
+        if constexpr (!P2) R = dv.of(d);
+        r = r_;
+    }
+    __device__ __forceinline__ double operator()(DV &dv, double x) const
+    {
+        if constexpr (P2) return x * r;
+        else return dv(x, R);
+    }
+};
 
 // portableWrapper min/max semantics (include/pp/utils.h:277-335).
 __device__ __forceinline__ double pmin(double a, double b) { return a < b ? a : b; }
@@ -229,147 +281,102 @@ __device__ __forceinline__ double pmin_list4(double a, double b, double c, doubl
     return m;
 }
 
-// Da, ss and Di of the van Leer limiter written in every remap flux function
-// (e.g. xremap.cpp:309-314).
-__device__ __forceinline__ double limiter_Di(double sign_v, double phi, double dfi, double dfu,
-                                             double dxci, double dxcu, double dxbu)
+// The upwind one of two values as the reference picks it, a * vad_p + b * vad_m
+// with weights one and zero: the chosen value plus zero times the other, one
+// fused multiply-add whose product is exact, so signed zeros, infinities and
+// NaN come out as they do there.
+__device__ __forceinline__ double pick(bool up, double a, double b) { return fma_rn(up ? b : a, 0.0, up ? a : b); }
+
+// One face along a sweep as its upwind fluxes see it: up where the flow goes
+// up the sweep, phi the swept fraction, ci the cell length at the face and cu
+// the upwind one, bu the upwind volume.
+template <class DV>
+struct Face {
+    bool up;
+    double phi;
+    typename DV::R ci, cu;
+    double bu;
+};
+
+// The van Leer limited correction Di of every remap flux function (e.g.
+// xremap.cpp:305-316) and the upwind value fu.
+template <class DV>
+__device__ __forceinline__ double limited(DV &dv, const Face<DV> &F, double fm, double fi, double fp, double fp2,
+                                          double &fu)
 {
-    double Da = (2.0 - phi) * fabs(dfi) / dxci + (1.0 + phi) * fabs(dfu) / dxcu;
-    Da = Da * SIXTH;
-    double ss = 0.5 * ((dfi >= 0.0 ? 1.0 : -1.0) + (dfu >= 0.0 ? 1.0 : -1.0));
-    return sign_v * ss * pmin_list3(fabs(Da) * dxbu, fabs(dfi), fabs(dfu));
+    const double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
+    fu = pick(F.up, fi, fp);
+    const double dfu = pick(F.up, dfm, dfp);
+    const double Da = dv.pair((2.0 - F.phi) * fabs(dfi), F.ci, (1.0 + F.phi) * fabs(dfu), F.cu) * SIXTH;
+    // sign_v * ss * min, with ss = 0.5 * (sign(dfi) + sign(dfu)): the minimum
+    // with the product's sign, or a zero with sign_v's where the slopes differ
+    const double m = pmin_list3(fabs(Da) * F.bu, fabs(dfi), fabs(dfu));
+    const bool pi = dfi >= 0.0, pu = dfu >= 0.0;
+    const double v = F.up ? 1.0 : -1.0;
+    return (pi == pu ? (pi ? v : -v) : 0.0 * v) * m;
 }
 
 // Evans-Hawley constrained-transport flux of a transverse face field
-// (vx_by_flux xremap.cpp:269-319 and the five analogues in x/y/zremap.cpp).
-// With the four quotients b/db along the sweep given (fm = bm / dbm, ...):
-// each is the same value at its point for every flux that reads it, so a
-// kernel can form it once per point.
-__device__ __forceinline__ double ct_flux_q(double v_advect, double dt, double fm, double fi, double fp, double fp2,
-                                            double dbi, double dbp, double dci, double dcm, double dcp,
-                                            double cv1i, double cv1p)
+// (vx_by_flux xremap.cpp:269-319 and the five analogues in x/y/zremap.cpp),
+// from the four quotients b/db along the sweep, and the mass flux through a
+// face (x_mass_flux xremap.cpp:373-422 and analogues): o_v is the swept
+// length or volume.
+template <class DV>
+__device__ __forceinline__ double swept_flux(DV &dv, const Face<DV> &F, double o_v, double fm, double fi, double fp,
+                                             double fp2)
 {
-    double o_v = v_advect * dt;
-    double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
-    double sign_v = (v_advect >= 0.0) ? 1.0 : -1.0;
-    double vad_p = (sign_v + 1.0) * 0.5;
-    double vad_m = 1.0 - vad_p;
-    double fu = fi * vad_p + fp * vad_m;
-    double dfu = dfm * vad_p + dfp * vad_m;
-    double dxcu = dcm * vad_p + dcp * vad_m;
-    double dxbu = cv1i * vad_p + cv1p * vad_m;
-    double dxu = dbi * vad_p + dbp * vad_m;
-    double phi = fabs(o_v) / dxu;
-    double Di = limiter_Di(sign_v, phi, dfi, dfu, dci, dxcu, dxbu);
-    return (fu + Di * (1.0 - phi)) * o_v;
+    double fu;
+    const double Di = limited(dv, F, fm, fi, fp, fp2, fu);
+    return (fu + Di * (1.0 - F.phi)) * o_v;
 }
 
-__device__ __forceinline__ double ct_flux(double v_advect, double dt, double bm, double bi, double bp,
-                                          double bp2, double dbm, double dbi, double dbp, double dbp2,
-                                          double dci, double dcm, double dcp, double cv1i, double cv1p)
+// Specific-energy flux (x_energy_flux xremap.cpp:429-483 and analogues) and
+// momentum flux (x_mom_flux xremap.cpp:485-566 and analogues) before their
+// product with dm; dmu is the swept mass fraction.
+template <class DV>
+__device__ __forceinline__ double carried(DV &dv, const Face<DV> &F, double fm, double fi, double fp, double fp2, double dmu)
 {
-    double o_v = v_advect * dt;
-    double fm = bm / dbm, fi = bi / dbi, fp = bp / dbp, fp2 = bp2 / dbp2;
-    double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
-    double sign_v = (v_advect >= 0.0) ? 1.0 : -1.0;
-    double vad_p = (sign_v + 1.0) * 0.5;
-    double vad_m = 1.0 - vad_p;
-    double fu = fi * vad_p + fp * vad_m;
-    double dfu = dfm * vad_p + dfp * vad_m;
-    double dxcu = dcm * vad_p + dcp * vad_m;
-    double dxbu = cv1i * vad_p + cv1p * vad_m;
-    double dxu = dbi * vad_p + dbp * vad_m;
-    double phi = fabs(o_v) / dxu;
-    double Di = limiter_Di(sign_v, phi, dfi, dfu, dci, dxcu, dxbu);
-    return (fu + Di * (1.0 - phi)) * o_v;
-}
-
-// Mass flux through a face (x_mass_flux xremap.cpp:373-422 and analogues).
-__device__ __forceinline__ double mass_flux(double v_advect, double dt, double area, double fm, double fi,
-                                            double fp, double fp2, double dci, double dcm, double dcp,
-                                            double cv1i, double cv1p)
-{
-    double o_v = v_advect * dt * area;
-    double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
-    double sign_v = (v_advect >= 0.0) ? 1.0 : -1.0;
-    double vad_p = (sign_v + 1.0) * 0.5;
-    double vad_m = 1.0 - vad_p;
-    double fu = fi * vad_p + fp * vad_m;
-    double dfu = dfm * vad_p + dfp * vad_m;
-    double dxcu = dcm * vad_p + dcp * vad_m;
-    double dxbu = cv1i * vad_p + cv1p * vad_m;
-    double phi = fabs(o_v) / dxbu;
-    double Di = limiter_Di(sign_v, phi, dfi, dfu, dci, dxcu, dxbu);
-    return (fu + Di * (1.0 - phi)) * o_v;
-}
-
-// Specific-energy flux (x_energy_flux xremap.cpp:429-483 and analogues).
-__device__ __forceinline__ double energy_flux(double v_advect, double dt, double area, double fm, double fi,
-                                              double fp, double fp2, double dci, double dcm, double dcp,
-                                              double cv1i, double cv1p, double rho1i, double rho1p, double dm)
-{
-    double o_v = v_advect * dt * area;
-    double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
-    double sign_v = (v_advect >= 0.0) ? 1.0 : -1.0;
-    double vad_p = (sign_v + 1.0) * 0.5;
-    double vad_m = 1.0 - vad_p;
-    double fu = fi * vad_p + fp * vad_m;
-    double dfu = dfm * vad_p + dfp * vad_m;
-    double dxcu = dcm * vad_p + dcp * vad_m;
-    double dxbu = cv1i * vad_p + cv1p * vad_m;
-    double phi = fabs(o_v) / dxbu;
-    double Di = limiter_Di(sign_v, phi, dfi, dfu, dci, dxcu, dxbu);
-    double rhou = rho1i * vad_p + rho1p * vad_m;
-    double dmu = fabs(dm) / dxbu / rhou;
-    return (fu + Di * (1.0 - dmu)) * dm;
-}
-
-// Momentum flux before its product with dm (x_mom_flux xremap.cpp:485-566
-// and analogues; the z sweep divides |dm| by (dzbu * rhou) in one step,
-// zremap.cpp:509).
-template <bool ZFORM>
-__device__ __forceinline__ double mom_flux(double v_advect, double dt, double area, double fm, double fi,
-                                           double fp, double fp2, double dci, double dcm, double dcp,
-                                           double cvci, double cvcp, double rvi, double rvp, double dm)
-{
-    double o_v = v_advect * dt * area;
-    double dfm = fi - fm, dfi = fp - fi, dfp = fp2 - fp;
-    double sign_v = (o_v >= 0.0) ? 1.0 : -1.0;
-    double vad_p = (sign_v + 1.0) * 0.5;
-    double vad_m = 1.0 - vad_p;
-    double fu = fi * vad_p + fp * vad_m;
-    double dfu = dfm * vad_p + dfp * vad_m;
-    double dxcu = dcm * vad_p + dcp * vad_m;
-    double dxbu = cvci * vad_p + cvcp * vad_m;
-    double phi = fabs(o_v) / dxbu;
-    double Di = limiter_Di(sign_v, phi, dfi, dfu, dci, dxcu, dxbu);
-    double rhou = rvi * vad_p + rvp * vad_m;
-    double dmu = ZFORM ? fabs(dm) / (dxbu * rhou) : fabs(dm) / dxbu / rhou;
+    double fu;
+    const double Di = limited(dv, F, fm, fi, fp, fp2, fu);
     return fu + Di * (1.0 - dmu);
+}
+
+// |dm| / dxbu / rhou (the z sweep's momentum flux divides by dxbu * rhou in
+// one step, zremap.cpp:509).
+template <bool ZFORM, class DV>
+__device__ __forceinline__ double mass_fraction(DV &dv, double dm, const typename DV::R &bu, double rhou)
+{
+    double dmu;
+    if constexpr (ZFORM) dmu = dv.fraction(fabs(dm), dv.of(bu.d * rhou));
+    else dmu = dv.fraction(dv.fraction(fabs(dm), bu), dv.of(rhou));
+    dv.finite(dmu);
+    return dmu;
 }
 
 // Caramana edge viscosity (lagran.cpp:56-93).  v[a] are the four points
 // along the edge direction, o1/o2 the edge ends.
-template <bool P2, class A>
-__device__ __forceinline__ double edge_viscosity(double dt, double visc1, double v2n, const A &vx,
+template <bool P2, class DV, class A>
+__device__ __forceinline__ double edge_viscosity(DV &div, double dt, double visc1, double v2n, const A &vx,
                                                  const A &vy, const A &vz, const A &rho_v,
                                                  double dvdots, double dx, double dxm, double dxp,
                                                  double cs_edge, int o0, int o1, int o2, int o3, double rdx = 0.0)
 {
     dvdots = pmin(0.0, dvdots);
     double rv1 = rho_v[o1], rv2 = rho_v[o2];
-    double rho_edge = 2.0 * rv1 * rv2 / (rv1 + rv2);
+    double rho_edge = div(2.0 * rv1 * rv2, div.of(rv1 + rv2));
     double vx1 = vx[o1], vx2 = vx[o2], vy1 = vy[o1], vy2 = vy[o2], vz1 = vz[o1], vz2 = vz[o2];
     double dvx = vx1 - vx2, dvy = vy1 - vy2, dvz = vz1 - vz2;
     double dv2 = dvx * dvx + dvy * dvy + dvz * dvz;
     double dv = sqrt(dv2);
-    bool small = div_by<P2>(dv * dt, dx, rdx) < 1.e-14;
-    dvdots = small ? 0.0 : dvdots / dv;
+    bool small = (P2 ? dv * dt * rdx : div(dv * dt, div.of(dx))) < 1.e-14;
+    // (where the jump is too small its quotients are not used: divide by one)
+    dvdots = small ? 0.0 : div(dvdots, div.of(small ? 1.0 : dv));
     double dvxm = vx[o0] - vx1, dvxp = vx2 - vx[o3];
     double dvym = vy[o0] - vy1, dvyp = vy2 - vy[o3];
     double dvzm = vz[o0] - vz1, dvzp = vz2 - vz[o3];
-    double rl = small ? 1.0 : (dvxp * dvx + dvyp * dvy + dvzp * dvz) * dx / (dxp * dv2);
-    double rr = small ? 1.0 : (dvxm * dvx + dvym * dvy + dvzm * dvz) * dx / (dxm * dv2);
+    double rl = div((dvxp * dvx + dvyp * dvy + dvzp * dvz) * dx, div.of(small ? 1.0 : dxp * dv2));
+    double rr = div((dvxm * dvx + dvym * dvy + dvzm * dvz) * dx, div.of(small ? 1.0 : dxm * dv2));
+    if (small) rl = rr = 1.0;
     double psi = pmin_list4(0.5 * (rr + rl), 2.0 * rl, 2.0 * rr, 1.0);
     psi = pmax(0.0, psi);
     double q_k_bar = rho_edge * (v2n * dv + sqrt(v2n * v2n * dv2 + (visc1 * cs_edge) * (visc1 * cs_edge)));

@@ -1,0 +1,130 @@
+// lare_div.cuh -- correctly rounded division without branches, for several
+// numerators over one denominator.
+//
+// The remap and the predictor divide several numerators by the same volume,
+// and every IEEE division costs about 14 fused multiply-adds of FP64 pipe
+// time, eight more instructions and a branch to its slow path, which also
+// keeps the compiler from moving loads up past it.  The forms here are
+// straight-line and give the same bits:
+//   rcp_fast   r = RN(1/d): the hardware's 20-bit seed, one third-order and
+//              one second-order Newton step.  A second-order step from an
+//              r within one ulp rounds correctly unless d's significand is all
+//              ones (Markstein).
+//   quot       q = RN(x/d) from r = RN(1/d) by Markstein's theorem (P.
+//              Markstein, "Computation of elementary functions on the IBM
+//              RISC System/6000 processor", 1990; Muller et al., "Handbook of
+//              Floating-Point Arithmetic"): if q is a faithful rounding of
+//              x/d and rem = x - d*q is formed exactly by an FMA, then
+//              RN(q + rem*r) = RN(x/d).  q = RN(x*r + RN(x*e)) with
+//              e = RN(r * (1 - d*r)), the part of 1/d that r misses, is within
+//              half an ulp and 2^-50 of one.
+// Conditions: d plain (plain_divisor: positive, exponent in -120..119, not
+// all ones), and |x/d| in 2^-600..2^600 (quot_in_range on the result: then x,
+// x*e and rem are normal, or exactly zero) or x zero.  The callers check them
+// and go back to the IEEE division otherwise, NaN and infinities included.
+#pragma once
+
+#include <cmath>
+#include <cstring>
+
+namespace sams {
+namespace dev {
+
+// (host forms for the checks that run without a GPU)
+__host__ __device__ __forceinline__ double fma_rn(double a, double b, double c)
+{
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return std::fma(a, b, c);
+#endif
+}
+__host__ __device__ __forceinline__ unsigned high_word(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2hiint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, sizeof u);
+    return (unsigned)(u >> 32);
+#endif
+}
+__host__ __device__ __forceinline__ unsigned low_word(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned)__double2loint(x);
+#else
+    unsigned long long u;
+    std::memcpy(&u, &x, sizeof u);
+    return (unsigned)u;
+#endif
+}
+// 1/d to 20 bits or more.
+__host__ __device__ __forceinline__ double rcp_seed(double d)
+{
+#ifdef __CUDA_ARCH__
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    return r;
+#else
+    const double r = 1.0 / d;
+    unsigned long long u;
+    std::memcpy(&u, &r, sizeof u);
+    u &= 0xffffffff00000000ull;  // the hardware's result has a zero low word
+    double s;
+    std::memcpy(&s, &u, sizeof s);
+    return s;
+#endif
+}
+
+__host__ __device__ __forceinline__ bool plain_divisor(double d)
+{
+    const unsigned h = high_word(d);
+    return h - ((unsigned)(1023 - 120) << 20) < (240u << 20) && !(low_word(d) == 0xffffffffu && (h & 0xfffffu) == 0xfffffu);
+}
+__host__ __device__ __forceinline__ bool quot_in_range(double q)
+{
+    return (high_word(q) & 0x7fffffffu) - ((unsigned)(1023 - 600) << 20) < (1200u << 20);
+}
+// ((h << 1) | l drops the sign)
+__host__ __device__ __forceinline__ bool is_zero(double x) { return ((high_word(x) << 1) | low_word(x)) == 0; }
+
+struct Rcp {
+    double d, r, e;
+};
+
+__host__ __device__ __forceinline__ double rcp_fast(double d)
+{
+    const double s = rcp_seed(d);
+    const double h = fma_rn(-d, s, 1.0);
+    const double r = fma_rn(s, fma_rn(h, h, h), s);
+    return fma_rn(r, fma_rn(-d, r, 1.0), r);
+}
+__host__ __device__ __forceinline__ Rcp rcp_with(double d, double r)
+{
+    Rcp R;
+    R.d = d;
+    R.r = r;
+    R.e = r * fma_rn(-d, r, 1.0);
+    return R;
+}
+__host__ __device__ __forceinline__ Rcp rcp_of(double d) { return rcp_with(d, rcp_fast(d)); }
+
+__host__ __device__ __forceinline__ double quot(double x, const Rcp &R)
+{
+    const double q = fma_rn(x, R.r, x * R.e);
+    return fma_rn(fma_rn(-R.d, q, x), R.r, q);
+}
+
+// x / R.d with a zero numerator's sign kept (R.d positive); bad is set where
+// the result may not be the IEEE quotient.
+__host__ __device__ __forceinline__ double quot_check(double x, const Rcp &R, bool &bad)
+{
+    const double q = quot(x, R);
+    const bool zero = is_zero(x);
+    bad = bad || (!quot_in_range(q) && !zero);
+    return zero ? x : q;
+}
+
+}  // namespace dev
+}  // namespace sams

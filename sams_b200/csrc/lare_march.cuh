@@ -155,8 +155,7 @@ __device__ __forceinline__ void pred(const Ctx &c, const MarchTile &m, int b, in
         if (!cell) return;
         const int slot = i % 3;
         double out[P1::NOUT];
-        bool half_p;
-        P1::compute<GEO, P2>(c, resistive, i, j, k, out, half_p);
+        P1::compute<GEO, P2>(c, resistive, i, j, k, out);
 #pragma unroll
         for (int q = 0; q < P1::PE; ++q) ring[(q * 3 + slot) * kRP + t] = out[q];
         ring[(P1::PE * 3 + slot) * kRP + t] = out[P1::PE] + out[P1::PI];
@@ -258,7 +257,7 @@ struct PrepMarch {
         prefetch(c.f[SAMS_F_BY], o);
         prefetch(c.f[SAMS_F_BZ], o);
     }
-    static constexpr int NR = 2, kMinBlocks = 5;  // register cap tuned on B200
+    static constexpr int NR = 2, kMinBlocks = 4;  // register cap tuned on B200
     template <bool GEO, bool P2>
     __device__ static void produce(const Ctx &c, int resistive, int i, int j, int k, bool own, double *out)
     {

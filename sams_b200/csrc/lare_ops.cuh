@@ -32,6 +32,8 @@
 // same multiplication order.
 #pragma once
 
+#include <type_traits>
+
 #include "lare_device.cuh"
 #include "sams_lare_layout.h"
 
@@ -172,6 +174,22 @@ struct NodePrep {
     template <bool GEO, bool P2, class S>
     __device__ static void run_src(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY, int QZ)
     {
+        using DV = typename std::conditional<P2, IeeeDiv, FastDiv>::type;  // (P2 divides by nothing)
+        DV dv;
+        average<GEO, P2>(dv, c, i, j, k, src, q0, QX, QY, QZ);
+        if (dv.bad) average_ieee<GEO, P2>(c, i, j, k, src, q0, QX, QY, QZ);
+    }
+    template <bool GEO, bool P2, class S>
+    __device__ static __noinline__ void average_ieee(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY,
+                                                     int QZ)
+    {
+        IeeeDiv dv;
+        average<GEO, P2>(dv, c, i, j, k, src, q0, QX, QY, QZ);
+    }
+    template <bool GEO, bool P2, class DV, class S>
+    __device__ __forceinline__ static void average(DV &dv, const Ctx &c, int i, int j, int k, const S &src, int q0, int QX,
+                                                   int QY, int QZ)
+    {
         const Geom &g = c.g;
         struct Arr {
             const S &s;
@@ -188,11 +206,13 @@ struct NodePrep {
         double sum_rho_cv = rho[o0] * cv0 + rho[o1] * cv1 + rho[o2] * cv2 + rho[o3] * cv3 +
                             rho[o4] * cv4 + rho[o5] * cv5 + rho[o6] * cv6 + rho[o7] * cv7;
         double sum_cv = cv0 + cv1 + cv2 + cv3 + cv4 + cv5 + cv6 + cv7;
-        c.s[S_RHOV][on] = div_by<P2>(sum_rho_cv, sum_cv, 0.125 * c.rc.cv);
-        double cv_v = 0.125 * sum_cv;
+        // cv_v = 0.125 * sum_cv (lagran.cpp:142-151); the sound speed divides
+        // 0.125 * sum by it, the same quotient as of the two sums
+        const By<P2, DV> by_cv(dv, sum_cv, 0.125 * c.rc.cv);
+        c.s[S_RHOV][on] = by_cv(dv, sum_rho_cv);
         double sum = cs[o0] * cv0 + cs[o1] * cv1 + cs[o2] * cv2 + cs[o3] * cv3 +
                      cs[o4] * cv4 + cs[o5] * cv5 + cs[o6] * cv6 + cs[o7] * cv7;
-        c.s[S_CSV][on] = div_by<P2>(0.125 * sum, cv_v, c.rc.cv);
+        c.s[S_CSV][on] = by_cv(dv, sum);
     }
 };
 
@@ -207,7 +227,20 @@ struct Alpha {
     // the edge viscosity of direction E (0 x, 1 y, 2 z) at (i, j, k), where
     // that direction's range holds the point
     template <int E, bool GEO, bool P2>
-    __device__ static void edge(const Ctx &c, int i, int j, int k)
+    __device__ __forceinline__ static void edge(const Ctx &c, int i, int j, int k)
+    {
+        FastDiv dv;
+        edge_by<E, GEO, P2>(dv, c, i, j, k);
+        if (dv.bad) edge_ieee<E, GEO, P2>(c, i, j, k);
+    }
+    template <int E, bool GEO, bool P2>
+    __device__ static __noinline__ void edge_ieee(const Ctx &c, int i, int j, int k)
+    {
+        IeeeDiv dv;
+        edge_by<E, GEO, P2>(dv, c, i, j, k);
+    }
+    template <int E, bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static void edge_by(DV &dv, const Ctx &c, int i, int j, int k)
     {
         const Geom &g = c.g;
         const RO vx{c.f[SAMS_F_VX]}, vy{c.f[SAMS_F_VY]}, vz{c.f[SAMS_F_VZ]};
@@ -220,7 +253,7 @@ struct Alpha {
             double dx = c.ax.dxb[i + 2], dxp = c.ax.dxb[i + 3], dxm = c.ax.dxb[i + 1];
             double dvdots = -(vx[o1] - vx[o2]);
             double cs_edge = pmin(cs_v[o1], cs_v[o2]);
-            c.s[S_A1][o] = edge_viscosity<P2>(dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.xb);
+            c.s[S_A1][o] = edge_viscosity<P2>(dv, dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.xb);
         }
         if (E == 1 && j >= 0 && j <= g.ny + 1) {  // alpha2: (-1..nx+1, 0..ny+1, 0..nz+2)
             int o1 = LOFF(i, j - 1, k - 1), o2 = LOFF(i, j, k - 1);
@@ -232,7 +265,7 @@ struct Alpha {
             }
             double dvdots = -(vy[o1] - vy[o2]);
             double cs_edge = pmin(cs_v[o1], cs_v[o2]);
-            c.s[S_A2][o] = edge_viscosity<P2>(dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.yb);
+            c.s[S_A2][o] = edge_viscosity<P2>(dv, dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.yb);
         }
         if (E == 2 && j <= g.ny + 1 && k <= g.nz + 1) {  // alpha3: (-1..nx+1, -1..ny+1, 0..nz+1)
             int o1 = o - 1, o2 = o;
@@ -244,7 +277,7 @@ struct Alpha {
             }
             double dvdots = -(vz[o1] - vz[o2]);
             double cs_edge = pmin(cs_v[o1], cs_v[o2]);
-            c.s[S_A3][o] = edge_viscosity<P2>(dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.zb);
+            c.s[S_A3][o] = edge_viscosity<P2>(dv, dt, visc1, v2n, vx, vy, vz, rho_v, dvdots, dx, dxm, dxp, cs_edge, o0, o1, o2, o3, c.rc.zb);
         }
     }
     template <bool GEO, bool P2>
@@ -272,7 +305,22 @@ struct Visc {
     // (:303-305, with the three edge jumps it needs formed again, the same
     // expressions) and its CFL candidate (set_dt, :380-443).
     template <bool GEO, bool P2>
-    __device__ static void heat_forces(const Ctx &c, int i, int j, int k, bool &nonfinite)
+    __device__ __forceinline__ static void heat_forces(const Ctx &c, int i, int j, int k, bool &nonfinite)
+    {
+        using DV = typename std::conditional<P2, IeeeDiv, FastDiv>::type;  // (P2 divides by nothing)
+        DV dv;
+        heat_forces_by<GEO, P2>(dv, c, i, j, k, nonfinite);
+        if (dv.bad) heat_forces_ieee<GEO, P2>(c, i, j, k);
+    }
+    template <bool GEO, bool P2>
+    __device__ static __noinline__ void heat_forces_ieee(const Ctx &c, int i, int j, int k)
+    {
+        IeeeDiv dv;
+        bool seen = false;  // (the first run has set the caller's flag)
+        heat_forces_by<GEO, P2>(dv, c, i, j, k, seen);
+    }
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static void heat_forces_by(DV &dv, const Ctx &c, int i, int j, int k, bool &nonfinite)
     {
         const Geom &g = c.g;
         const RO vx{c.f[SAMS_F_VX]}, vy{c.f[SAMS_F_VY]}, vz{c.f[SAMS_F_VZ]};
@@ -313,7 +361,7 @@ struct Visc {
                     - 0.25 * dx * dy * a3a[o - SX - SY] * a11
                     - 0.25 * dx * dy * a3a[o - SY] * a12;
         const double cv = (GEO && c.p.geometry) ? cv_at<GEO>(c, i, j, k) : dx * (dyp * dzp);
-        c.s[S_VH][o] = div_by<P2>(vh, cv, c.rc.cv);
+        c.s[S_VH][o] = By<P2, DV>(dv, cv, c.rc.cv)(dv, vh);
         if (i > g.nx || j > g.ny || k > g.nz) return;
         // checked where run checks it: the cells of the CFL range
         if (!(GEO && c.p.geometry && i < 1) && !(fabs(vh) <= DBL_MAX)) nonfinite = true;
@@ -328,8 +376,9 @@ struct Visc {
         double sum_cv = cv_at<GEO>(c, i, j, k) + cv_at<GEO>(c, ip, j, k) + cv_at<GEO>(c, i, jp, k) + cv_at<GEO>(c, ip, jp, k) +
                         cv_at<GEO>(c, i, j, kp) + cv_at<GEO>(c, ip, j, kp) + cv_at<GEO>(c, i, jp, kp) + cv_at<GEO>(c, ip, jp, kp);
         double cv_v = 0.125 * sum_cv;
-#define FV(v) div_by<P2>(e1 * (v[o] - v[o - SX]) + e2 * (v[o] - v[o + SX]) + e3 * (v[o] - v[o - SY]) + \
-                e4 * (v[o] - v[o + SY]) + e5 * (v[o] - v[o - 1]) + e6 * (v[o] - v[o + 1]), cv_v, c.rc.cv)
+        const By<P2, DV> by_cv(dv, cv_v, c.rc.cv);
+#define FV(v) by_cv(dv, e1 * (v[o] - v[o - SX]) + e2 * (v[o] - v[o + SX]) + e3 * (v[o] - v[o - SY]) + \
+                e4 * (v[o] - v[o + SY]) + e5 * (v[o] - v[o - 1]) + e6 * (v[o] - v[o + 1]))
         c.s[S_FXV][o] = FV(vx);
         c.s[S_FYV][o] = FV(vy);
         c.s[S_FZV][o] = FV(vz);
@@ -337,7 +386,26 @@ struct Visc {
     }
     // (cells 0..n; DBL_MAX outside the CFL range)
     template <bool GEO, bool P2>
-    __device__ static double cfl(const Ctx &c, int i, int j, int k, bool &nonfinite)
+    __device__ __forceinline__ static double cfl(const Ctx &c, int i, int j, int k, bool &nonfinite)
+    {
+        FastDiv dv;
+        bool seen = false;
+        const double best = cfl_by<GEO, P2>(dv, c, i, j, k, seen);
+        if (dv.bad) return cfl_ieee<GEO, P2>(c, i, j, k, &nonfinite);
+        nonfinite = nonfinite || seen;
+        return best;
+    }
+    template <bool GEO, bool P2>
+    __device__ static __noinline__ double cfl_ieee(const Ctx &c, int i, int j, int k, bool *nonfinite)
+    {
+        IeeeDiv dv;
+        bool seen = false;
+        const double best = cfl_by<GEO, P2>(dv, c, i, j, k, seen);
+        if (seen) *nonfinite = true;
+        return best;
+    }
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static double cfl_by(DV &dv, const Ctx &c, int i, int j, int k, bool &nonfinite)
     {
         const Geom &g = c.g;
         const RO vx{c.f[SAMS_F_VX]}, vy{c.f[SAMS_F_VY]}, vz{c.f[SAMS_F_VZ]};
@@ -361,16 +429,18 @@ struct Visc {
         double pressure = (gm - 1.0) * rho * __ldg(c.f[SAMS_F_ENERGY_ELECTRON] + o) +
                           (gm - 1.0) * rho * __ldg(c.f[SAMS_F_ENERGY_ION] + o);
         double rho0 = pmax(rho, NONE_ZERO);
-        double cs2 = gm * pressure / rho0;
-        double w1 = div_by<P2>(bx[o] * bx[o] + by[o] * by[o] + bz[o] * bz[o], c.p.mu0, c.rc.mu0) / rho0;
-        double c_visc2 = p_visc / rho0;
+        const typename DV::R by_rho = dv.of(rho0);
+        double cs2 = dv(gm * pressure, by_rho);
+        const double b2 = bx[o] * bx[o] + by[o] * by[o] + bz[o] * bz[o];
+        double w1 = dv(P2 ? b2 * c.rc.mu0 : b2 / c.p.mu0, by_rho);
+        double c_visc2 = dv(p_visc, by_rho);
         // outside Cartesian geometry the CFL range starts at x index 1 (lagran.cpp:384)
         if (GEO && c.p.geometry && i < 1) return DBL_MAX;
         // lagran.cpp:396-398
         const double dhy = (GEO && c.p.geometry) ? dyp * c.gf.hyc[i + 2] : dyp;
         const double dhz = (GEO && c.p.geometry) ? dzp * c.gf.hzc[h2_index(c, i, j)] : dzp;
         double length = pmin(pmin(dx, dhy), dhz);
-        double dt1 = length / (sqrt(c_visc2) + sqrt(cs2 + w1 + c_visc2));
+        double dt1 = dv(length, dv.of(sqrt(c_visc2) + sqrt(cs2 + w1 + c_visc2)));
         double ax = 0.25 * (dyp * dzp), ay = 0.25 * (dx * dzp), az = 0.25 * (dx * dyp);
         if (GEO && c.p.geometry) {  // lagran.cpp:404-406 reads the metric arrays
             ax = 0.25 * dxab_at<GEO>(c, i, j, k);
@@ -387,9 +457,9 @@ struct Visc {
         double avxm = fabs(vxbm), avxp = fabs(vxbp), avym = fabs(vybm);
         double avyp = fabs(vybp), avzm = fabs(vzbm), avzp = fabs(vzbp);
         double volume = cv;
-        double dt2 = volume / pmax(pmax(pmax(avxm, avxp), dvx), 1.0e-10 * volume);
-        double dt3 = volume / pmax(pmax(pmax(avym, avyp), dvy), 1.0e-10 * volume);
-        double dt4 = volume / pmax(pmax(pmax(avzm, avzp), dvz), 1.0e-10 * volume);
+        double dt2 = dv(volume, dv.of(pmax(pmax(pmax(avxm, avxp), dvx), 1.0e-10 * volume)));
+        double dt3 = dv(volume, dv.of(pmax(pmax(pmax(avym, avyp), dvy), 1.0e-10 * volume)));
+        double dt4 = dv(volume, dv.of(pmax(pmax(pmax(avzm, avzp), dvz), 1.0e-10 * volume)));
         const double chk = dt1 + dt2 + dt3 + dt4 + p_visc;
         if (!(fabs(chk) <= DBL_MAX)) nonfinite = true;
         return pmin(pmin(pmin(dt1, dt2), dt3), dt4);
@@ -418,31 +488,37 @@ struct ResistRK {
     // outputs: the three edge fluxes and the Ohmic heating rate
     enum { FX, FY, FZ, CURLB, NOUT };
     template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
+    __device__ __forceinline__ static void compute(const Ctx &c, int i, int j, int k, double *out)
     {
-        double out[NOUT];
-        compute<GEO, P2>(c, i, j, k, out);
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        c.s[S_FLUXX][o] = out[FX];
-        c.s[S_FLUXY][o] = out[FY];
-        c.s[S_FLUXZ][o] = out[FZ];
-        c.s[S_CURLB][o] = out[CURLB];
+        using DV = typename std::conditional<P2, IeeeDiv, FastDiv>::type;  // (P2 divides by nothing)
+        DV dv;
+        compute_by<GEO, P2>(dv, c, i, j, k, out);
+        if (dv.bad) {
+            double slow[NOUT];
+            compute_ieee<GEO, P2>(c, i, j, k, slow);
+            for (int q = 0; q < NOUT; ++q) out[q] = slow[q];
+        }
     }
     template <bool GEO, bool P2>
-    __device__ static void compute(const Ctx &c, int i, int j, int k, double *out)
+    __device__ static __noinline__ void compute_ieee(const Ctx &c, int i, int j, int k, double *out)
+    {
+        IeeeDiv dv;
+        compute_by<GEO, P2>(dv, c, i, j, k, out);
+    }
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static void compute_by(DV &dv, const Ctx &c, int i, int j, int k, double *out)
     {
         const Geom &g = c.g;
         const RO bx{c.f[SAMS_F_BX]}, by{c.f[SAMS_F_BY]}, bz{c.f[SAMS_F_BZ]};
         const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
         const double dxc = c.ax.dxc[i + 2], dyc = c.ax.dyc[j + 2], dzc = c.ax.dzc[k + 2];
-        const double rx = c.rc.xc, ry = c.rc.yc, rz = c.rc.zc;
-        double jx1 = div_by<P2>(bz[o + SY] - bz[o], dyc, ry) - div_by<P2>(by[o + 1] - by[o], dzc, rz);
-        double jx2 = div_by<P2>(bz[o + SX + SY] - bz[o + SX], dyc, ry) - div_by<P2>(by[o + SX + 1] - by[o + SX], dzc, rz);
-        double jy1 = div_by<P2>(bx[o + 1] - bx[o], dzc, rz) - div_by<P2>(bz[o + SX] - bz[o], dxc, rx);
-        double jy2 = div_by<P2>(bx[o + SY + 1] - bx[o + SY], dzc, rz) - div_by<P2>(bz[o + SX + SY] - bz[o + SY], dxc, rx);
-        double jz1 = div_by<P2>(by[o + SX] - by[o], dxc, rx) - div_by<P2>(bx[o + SY] - bx[o], dyc, ry);
-        double jz2 = div_by<P2>(by[o + SX + 1] - by[o + 1], dxc, rx) - div_by<P2>(bx[o + SY + 1] - bx[o + 1], dyc, ry);
+        const By<P2, DV> by_x(dv, dxc, c.rc.xc), by_y(dv, dyc, c.rc.yc), by_z(dv, dzc, c.rc.zc);
+        double jx1 = by_y(dv, bz[o + SY] - bz[o]) - by_z(dv, by[o + 1] - by[o]);
+        double jx2 = by_y(dv, bz[o + SX + SY] - bz[o + SX]) - by_z(dv, by[o + SX + 1] - by[o + SX]);
+        double jy1 = by_z(dv, bx[o + 1] - bx[o]) - by_x(dv, bz[o + SX] - bz[o]);
+        double jy2 = by_z(dv, bx[o + SY + 1] - bx[o + SY]) - by_x(dv, bz[o + SX + SY] - bz[o + SY]);
+        double jz1 = by_x(dv, by[o + SX] - by[o]) - by_y(dv, bx[o + SY] - bx[o]);
+        double jz2 = by_x(dv, by[o + SX + 1] - by[o + 1]) - by_y(dv, bx[o + SY + 1] - bx[o + 1]);
         double jx = 0.5 * (jx1 + jx2), jy = 0.5 * (jy1 + jy2), jz = 0.5 * (jz1 + jz2);
         // eta_bg + eta0 where |J| > j_max, else eta_bg.  When the two have the
         // same bits (eta0 = 0: the configurations' uniform eta) the choice
@@ -466,27 +542,40 @@ struct ResistB {
     {
         set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
     }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int last, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        double *bx = c.f[SAMS_F_BX], *by = c.f[SAMS_F_BY], *bz = c.f[SAMS_F_BZ];
-        if (last) {
-            c.s[S_B1X][o] = bx[o];
-            c.s[S_B1Y][o] = by[o];
-            c.s[S_B1Z][o] = bz[o];
-        }
-        const ArraySrc src{{c.s[S_FLUXX], c.s[S_FLUXY], c.s[S_FLUXZ], c.s[S_CURLB]}};
-        run_src<P2>(c, i, j, k, src, o, g.sx, g.sy, 1, bx, by, bz);
-    }
     // The update at (i, j, k) with the fluxes of ResistRK read through
     // src(array, q) for the cell q = q0 - dx*QX - dy*QY - dz*QZ (dx, dy, dz in
     // {0, 1}); the new B goes to nbx/nby/nbz[o] (unchanged values included),
     // the electron energy is updated in place.
     template <bool P2, class S>
-    __device__ static void run_src(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY, int QZ,
-                                   double *nbx, double *nby, double *nbz)
+    __device__ __forceinline__ static void run_src(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY,
+                                                   int QZ, double *nbx, double *nby, double *nbz)
+    {
+        FastDiv dv;
+        double out[4];
+        update<P2>(dv, c, i, j, k, src, q0, QX, QY, QZ, out);
+        if (dv.bad) {
+            double slow[4];
+            update_ieee<P2>(c, i, j, k, src, q0, QX, QY, QZ, slow);
+            for (int q = 0; q < 4; ++q) out[q] = slow[q];
+        }
+        const int o = box_off(c.g, i, j, k);
+        nbx[o] = out[0];
+        nby[o] = out[1];
+        nbz[o] = out[2];
+        if (i >= 1 && i <= c.g.nx && j >= 1 && j <= c.g.ny && k >= 1 && k <= c.g.nz)
+            c.f[SAMS_F_ENERGY_ELECTRON][o] += out[3];
+    }
+    template <bool P2, class S>
+    __device__ static __noinline__ void update_ieee(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY,
+                                                    int QZ, double *out)
+    {
+        IeeeDiv dv;
+        update<P2>(dv, c, i, j, k, src, q0, QX, QY, QZ, out);
+    }
+    // new B and the electron energy's increment
+    template <bool P2, class DV, class S>
+    __device__ __forceinline__ static void update(DV &dv, const Ctx &c, int i, int j, int k, const S &src, int q0, int QX,
+                                                  int QY, int QZ, double *out)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
@@ -498,31 +587,30 @@ struct ResistB {
         const Arr fx{src, ResistRK::FX}, fy{src, ResistRK::FY}, fz{src, ResistRK::FZ};
         const double dt = c.sc->dt_sub;
         const int q = q0, SX = QX, SY = QY;
-        double bxo = __ldg(c.f[SAMS_F_BX] + o), byo = __ldg(c.f[SAMS_F_BY] + o), bzo = __ldg(c.f[SAMS_F_BZ] + o);
+        double bxn = __ldg(c.f[SAMS_F_BX] + o), byn = __ldg(c.f[SAMS_F_BY] + o), bzn = __ldg(c.f[SAMS_F_BZ] + o);
         const bool inx = i >= 0 && i <= g.nx, iny = j >= 0 && j <= g.ny, inz = k >= 0 && k <= g.nz;
         const bool inx1 = i >= 1 && i <= g.nx, iny1 = j >= 1 && j <= g.ny, inz1 = k >= 1 && k <= g.nz;
-        double bxn = bxo, byn = byo, bzn = bzo;
         if (inx && iny1 && inz1) {
-            double area = c.ax.dyb[j + 2] * c.ax.dzb[k + 2];
-            bxn = bxo + div_by<P2>((fz[q] - fz[q - SY] + fz[q - QZ] - fz[q - SY - QZ] - fy[q] + fy[q - QZ] - fy[q - SY] + fy[q - SY - QZ]) * dt, area, c.rc.yb * c.rc.zb);
+            const By<P2, DV> by_area(dv, c.ax.dyb[j + 2] * c.ax.dzb[k + 2], c.rc.yb * c.rc.zb);
+            bxn = bxn + by_area(dv, (fz[q] - fz[q - SY] + fz[q - QZ] - fz[q - SY - QZ] - fy[q] + fy[q - QZ] - fy[q - SY] + fy[q - SY - QZ]) * dt);
         }
         if (inx1 && iny && inz1) {
-            double area = c.ax.dxb[i + 2] * c.ax.dzb[k + 2];
-            byn = byo + div_by<P2>((fx[q] - fx[q - QZ] + fx[q - SX] - fx[q - SX - QZ] - fz[q] + fz[q - SX] - fz[q - QZ] + fz[q - SX - QZ]) * dt, area, c.rc.xb * c.rc.zb);
+            const By<P2, DV> by_area(dv, c.ax.dxb[i + 2] * c.ax.dzb[k + 2], c.rc.xb * c.rc.zb);
+            byn = byn + by_area(dv, (fx[q] - fx[q - QZ] + fx[q - SX] - fx[q - SX - QZ] - fz[q] + fz[q - SX] - fz[q - QZ] + fz[q - SX - QZ]) * dt);
         }
         if (inx1 && iny1 && inz) {
-            double area = c.ax.dxb[i + 2] * c.ax.dyb[j + 2];
-            bzn = bzo + div_by<P2>((fy[q] - fy[q - SX] + fy[q - SY] - fy[q - SX - SY] - fx[q] + fx[q - SY] - fx[q - SX] + fx[q - SX - SY]) * dt, area, c.rc.xb * c.rc.yb);
+            const By<P2, DV> by_area(dv, c.ax.dxb[i + 2] * c.ax.dyb[j + 2], c.rc.xb * c.rc.yb);
+            bzn = bzn + by_area(dv, (fy[q] - fy[q - SX] + fy[q - SY] - fy[q - SX - SY] - fx[q] + fx[q - SY] - fx[q - SX] + fx[q - SX - SY]) * dt);
         }
-        nbx[o] = bxn;
-        nby[o] = byn;
-        nbz[o] = bzn;
+        out[0] = bxn;
+        out[1] = byn;
+        out[2] = bzn;
+        out[3] = 0.0;
         if (inx1 && iny1 && inz1) {
             const Arr curlb{src, ResistRK::CURLB};
             double sum_curlb = curlb[q] + curlb[q - SX] + curlb[q - SY] + curlb[q - SX - SY] +
                                curlb[q - QZ] + curlb[q - SX - QZ] + curlb[q - SY - QZ] + curlb[q - SX - SY - QZ];
-            double *ee = c.f[SAMS_F_ENERGY_ELECTRON];
-            ee[o] += sum_curlb * dt / (8.0 * __ldg(c.f[SAMS_F_RHO] + o));
+            out[3] = dv(sum_curlb * dt, dv.of(8.0 * __ldg(c.f[SAMS_F_RHO] + o)));
         }
     }
 };
@@ -535,29 +623,29 @@ struct Pred1 {
     {
         set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
     }
-    // Outputs of one cell, in this order: cv1, b1x*cv1, b1y*cv1, b1z*cv1 and
-    // (where the cell is in 0..n+1 in every dimension, `half_p` set) the
-    // half-step p_e, p_i.  Reads the step-start p_e/p_i of resistive runs
+    // Outputs of one cell (0..n+1 in every dimension), in this order: cv1,
+    // b1x*cv1, b1y*cv1, b1z*cv1 and the half-step p_e, p_i.  Reads the step-start p_e/p_i of resistive runs
     // from S_PE/S_PI.
     enum { CV1, B1X, B1Y, B1Z, PE, PI, NOUT };
     template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int resistive, int i, int j, int k)
+    __device__ __forceinline__ static void compute(const Ctx &c, int resistive, int i, int j, int k, double *out)
     {
-        double out[NOUT];
-        bool half_p;
-        compute<GEO, P2>(c, resistive, i, j, k, out, half_p);
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        c.s[S_B1X][o] = out[B1X];
-        c.s[S_B1Y][o] = out[B1Y];
-        c.s[S_B1Z][o] = out[B1Z];
-        c.s[S_CV1][o] = out[CV1];
-        if (!half_p) return;
-        c.s[S_PE][o] = out[PE];
-        c.s[S_PI][o] = out[PI];
+        FastDiv dv;
+        compute_by<GEO, P2>(dv, c, resistive, i, j, k, out);
+        if (dv.bad) {
+            double slow[NOUT];
+            compute_ieee<GEO, P2>(c, resistive, i, j, k, slow);
+            for (int q = 0; q < NOUT; ++q) out[q] = slow[q];
+        }
     }
     template <bool GEO, bool P2>
-    __device__ static void compute(const Ctx &c, int resistive, int i, int j, int k, double *out, bool &half_p)
+    __device__ static __noinline__ void compute_ieee(const Ctx &c, int resistive, int i, int j, int k, double *out)
+    {
+        IeeeDiv dv;
+        compute_by<GEO, P2>(dv, c, resistive, i, j, k, out);
+    }
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static void compute_by(DV &dv, const Ctx &c, int resistive, int i, int j, int k, double *out)
     {
         const Geom &g = c.g;
         const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
@@ -574,32 +662,33 @@ struct Pred1 {
         double vzb = 0.25 * (vz[a] + vz[am] + vz[bm] + vz[am - SY]);
         double vzbm = 0.25 * (vz[cm] + vz[am - 1] + vz[bm - 1] + vz[am - SY - 1]);
         double vol = cv_at<GEO>(c, i, j, k);
-        double dvxdx = div_by<P2>(vxb * dxab0 - vxbm * dxabm, vol, c.rc.cv);
-        double dvydy = div_by<P2>(vyb * dyab0 - vybm * dyabm, vol, c.rc.cv);
-        double dvzdz = div_by<P2>(vzb * dzab0 - vzbm * dzabm, vol, c.rc.cv);
-        double dv = (dvxdx + dvydy + dvzdz) * dt / 2.0;
-        double cv1 = vol * (1.0 + dv);
+        const By<P2, DV> by_vol(dv, vol, c.rc.cv);
+        double dvxdx = by_vol(dv, vxb * dxab0 - vxbm * dxabm);
+        double dvydy = by_vol(dv, vyb * dyab0 - vybm * dyabm);
+        double dvzdz = by_vol(dv, vzb * dzab0 - vzbm * dzabm);
+        const double dvol = (dvxdx + dvydy + dvzdz) * dt / 2.0;
+        double cv1 = vol * (1.0 + dvol);
 
         vxb = 0.25 * (vx[a] + vx[am] + vx[cm] + vx[am - 1]);
         vxbm = 0.25 * (vx[bm] + vx[bm - SX] + vx[bm - 1] + vx[bm - SX - 1]);
         vyb = 0.25 * (vy[a] + vy[bm] + vy[cm] + vy[bm - 1]);
         vybm = 0.25 * (vy[am] + vy[am - SY] + vy[am - 1] + vy[am - SY - 1]);
-        double dvxdy = div_by<P2>(vxb * dyab0 - vxbm * dyabm, vol, c.rc.cv);
-        double dvydx = div_by<P2>(vyb * dxab0 - vybm * dxabm, vol, c.rc.cv);
+        double dvxdy = by_vol(dv, vxb * dyab0 - vxbm * dyabm);
+        double dvydx = by_vol(dv, vyb * dxab0 - vybm * dxabm);
 
         vxb = 0.25 * (vx[a] + vx[am] + vx[bm] + vx[am - SY]);
         vxbm = 0.25 * (vx[cm] + vx[am - 1] + vx[bm - 1] + vx[am - SY - 1]);
         double vzb2 = 0.25 * (vz[a] + vz[bm] + vz[cm] + vz[bm - 1]);
         double vzbm2 = 0.25 * (vz[am] + vz[am - SY] + vz[am - 1] + vz[am - SY - 1]);
-        double dvxdz = div_by<P2>(vxb * dzab0 - vxbm * dzabm, vol, c.rc.cv);
-        double dvzdx = div_by<P2>(vzb2 * dxab0 - vzbm2 * dxabm, vol, c.rc.cv);
+        double dvxdz = by_vol(dv, vxb * dzab0 - vxbm * dzabm);
+        double dvzdx = by_vol(dv, vzb2 * dxab0 - vzbm2 * dxabm);
 
         vyb = 0.25 * (vy[a] + vy[am] + vy[bm] + vy[am - SY]);
         vybm = 0.25 * (vy[cm] + vy[am - 1] + vy[bm - 1] + vy[am - SY - 1]);
         vzb2 = 0.25 * (vz[a] + vz[am] + vz[cm] + vz[am - 1]);
         vzbm2 = 0.25 * (vz[bm] + vz[bm - SX] + vz[bm - 1] + vz[bm - SX - 1]);
-        double dvydz = div_by<P2>(vyb * dzab0 - vybm * dzabm, vol, c.rc.cv);
-        double dvzdy = div_by<P2>(vzb2 * dyab0 - vzbm2 * dyabm, vol, c.rc.cv);
+        double dvydz = by_vol(dv, vyb * dzab0 - vybm * dzabm);
+        double dvzdy = by_vol(dv, vzb2 * dyab0 - vzbm2 * dyabm);
 
         double b1x, b1y, b1z;
         if (resistive) {
@@ -615,27 +704,27 @@ struct Pred1 {
         double w3 = b1x * dvxdx + b1y * dvxdy + b1z * dvxdz;
         double w4 = b1x * dvydx + b1y * dvydy + b1z * dvydz;
         double w5 = b1x * dvzdx + b1y * dvzdy + b1z * dvzdz;
-        b1x = (b1x + w3 * dt / 2.0) / (1.0 + dv);
-        b1y = (b1y + w4 * dt / 2.0) / (1.0 + dv);
-        b1z = (b1z + w5 * dt / 2.0) / (1.0 + dv);
+        const typename DV::R by_dvol = dv.of(1.0 + dvol);
+        b1x = dv(b1x + w3 * dt / 2.0, by_dvol);
+        b1y = dv(b1y + w4 * dt / 2.0, by_dvol);
+        b1z = dv(b1z + w5 * dt / 2.0, by_dvol);
         out[B1X] = b1x * cv1;
         out[B1Y] = b1y * cv1;
         out[B1Z] = b1z * cv1;
         out[CV1] = cv1;
 
-        half_p = !(i < 0 || i > g.nx + 1 || j < 0 || j > g.ny + 1 || k < 0 || k > g.nz + 1);
-        if (!half_p) return;
         const double gm = c.p.gamma;
         double rho = __ldg(c.f[SAMS_F_RHO] + o), ee = __ldg(c.f[SAMS_F_ENERGY_ELECTRON] + o);
         double ei = __ldg(c.f[SAMS_F_ENERGY_ION] + o);
         double pe = resistive ? __ldg(c.s[S_PE] + o) : (gm - 1.0) * rho * ee;
         double pi = resistive ? __ldg(c.s[S_PI] + o) : (gm - 1.0) * rho * ei;
-        double dvv = div_by<P2>(cv1, vol, c.rc.cv) - 1.0;
-        double e1_e = ee - pe * dvv / rho;
-        double e1_i = ei - pi * dvv / rho;
-        e1_i += __ldg(c.s[S_VH] + o) * dt / 2.0 / rho;
-        out[PE] = e1_e * (gm - 1.0) * rho * vol / cv1;
-        out[PI] = e1_i * (gm - 1.0) * rho * vol / cv1;
+        double dvv = by_vol(dv, cv1) - 1.0;
+        const typename DV::R by_rho = dv.of(rho), by_cv1 = dv.of(cv1);
+        double e1_e = ee - dv(pe * dvv, by_rho);
+        double e1_i = ei - dv(pi * dvv, by_rho);
+        e1_i += dv(__ldg(c.s[S_VH] + o) * dt / 2.0, by_rho);
+        out[PE] = dv(e1_e * (gm - 1.0) * rho * vol, by_cv1);
+        out[PI] = dv(e1_i * (gm - 1.0) * rho * vol, by_cv1);
     }
 };
 
@@ -647,17 +736,26 @@ struct Pred2 {
     {
         set_bounds(lo, hi, 0, g.nx, 0, g.ny, 0, g.nz);
     }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const ArraySrc src{{c.s[S_CV1], c.s[S_B1X], c.s[S_B1Y], c.s[S_B1Z], c.s[S_PE], c.s[S_PI]}};
-        run_src<GEO, P2>(c, i, j, k, src, LOFF(i, j, k), g.sx, g.sy, 1);
-    }
     // The node's update with Pred1's outputs read through src(array, q) for
     // the cell q = q0 + dx*QX + dy*QY + dz*QZ (dx, dy, dz in {0, 1}).
     template <bool GEO, bool P2, class S>
-    __device__ static void run_src(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY, int QZ)
+    __device__ __forceinline__ static void run_src(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY,
+                                                   int QZ)
+    {
+        FastDiv dv;
+        node<GEO, P2>(dv, c, i, j, k, src, q0, QX, QY, QZ);
+        if (dv.bad) node_ieee<GEO, P2>(c, i, j, k, src, q0, QX, QY, QZ);
+    }
+    template <bool GEO, bool P2, class S>
+    __device__ static __noinline__ void node_ieee(const Ctx &c, int i, int j, int k, const S &src, int q0, int QX, int QY,
+                                                  int QZ)
+    {
+        IeeeDiv dv;
+        node<GEO, P2>(dv, c, i, j, k, src, q0, QX, QY, QZ);
+    }
+    template <bool GEO, bool P2, class DV, class S>
+    __device__ __forceinline__ static void node(DV &dv, const Ctx &c, int i, int j, int k, const S &src, int q0, int QX,
+                                                int QY, int QZ)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
@@ -691,13 +789,14 @@ struct Pred2 {
         double ppxy = ptot(qxy), ppxz = ptot(qxz), ppyz = ptot(qyz), ppxyz = ptot(qxyz);
         double w1 = pp + ppy + ppz + ppyz;
         double w2 = ppx + ppxy + ppxz + ppxyz;
-        double fx = div_by<P2>((w1 - w2) * 0.25, dx, c.rc.xc);
+        const By<P2, DV> by_x(dv, dx, c.rc.xc), by_y(dv, dhy, c.rc.yc), by_z(dv, dhz, c.rc.zc);
+        double fx = by_x(dv, (w1 - w2) * 0.25);
         w1 = pp + ppx + ppz + ppxz;
         w2 = ppy + ppxy + ppyz + ppxyz;
-        double fy = div_by<P2>((w1 - w2) * 0.25, dhy, c.rc.yc);
+        double fy = by_y(dv, (w1 - w2) * 0.25);
         w1 = pp + ppx + ppy + ppxy;
         w2 = ppz + ppxz + ppyz + ppxyz;
-        double fz = div_by<P2>((w1 - w2) * 0.25, dhz, c.rc.zc);
+        double fz = by_z(dv, (w1 - w2) * 0.25);
 
         double cvx = cv1[q0] + cv1[qy] + cv1[qz] + cv1[qyz];
         double cvxp = cv1[qx] + cv1[qxy] + cv1[qxz] + cv1[qxyz];
@@ -706,57 +805,60 @@ struct Pred2 {
         double cvz = cv1[q0] + cv1[qx] + cv1[qy] + cv1[qxy];
         double cvzp = cv1[qz] + cv1[qxz] + cv1[qyz] + cv1[qxyz];
 
+        const typename DV::R by_cvx = dv.of(cvx), by_cvxp = dv.of(cvxp), by_cvy = dv.of(cvy), by_cvyp = dv.of(cvyp),
+                             by_cvz = dv.of(cvz), by_cvzp = dv.of(cvzp);
         double jx;
         if (geo) {
-            w1 = (bz1[q0] + bz1[qx] + bz1[qz] + bz1[qxz]) * h3 / cvy;
-            w2 = (bz1[qy] + bz1[qxy] + bz1[qyz] + bz1[qxyz]) * h3y / cvyp;
-            jx = (w2 - w1) / dhy / h3c;
+            w1 = dv((bz1[q0] + bz1[qx] + bz1[qz] + bz1[qxz]) * h3, by_cvy);
+            w2 = dv((bz1[qy] + bz1[qxy] + bz1[qyz] + bz1[qxyz]) * h3y, by_cvyp);
+            jx = by_y(dv, w2 - w1) / h3c;
         } else {
-            w1 = (bz1[q0] + bz1[qx] + bz1[qz] + bz1[qxz]) / cvy;
-            w2 = (bz1[qy] + bz1[qxy] + bz1[qyz] + bz1[qxyz]) / cvyp;
-            jx = div_by<P2>(w2 - w1, dhy, c.rc.yc);
+            w1 = dv((bz1[q0] + bz1[qx] + bz1[qz] + bz1[qxz]), by_cvy);
+            w2 = dv((bz1[qy] + bz1[qxy] + bz1[qyz] + bz1[qxyz]), by_cvyp);
+            jx = by_y(dv, w2 - w1);
         }
-        w1 = (by1[q0] + by1[qx] + by1[qy] + by1[qxy]) / cvz;
-        w2 = (by1[qz] + by1[qxz] + by1[qyz] + by1[qxyz]) / cvzp;
-        jx -= div_by<P2>(w2 - w1, dhz, c.rc.zc);
+        w1 = dv((by1[q0] + by1[qx] + by1[qy] + by1[qxy]), by_cvz);
+        w2 = dv((by1[qz] + by1[qxz] + by1[qyz] + by1[qxyz]), by_cvzp);
+        jx -= by_z(dv, w2 - w1);
 
         double jy;
         if (geo) {
-            w1 = (bz1[q0] + bz1[qy] + bz1[qz] + bz1[qyz]) * h3 / cvx;
-            w2 = (bz1[qx] + bz1[qxy] + bz1[qxz] + bz1[qxyz]) * h3x / cvxp;
-            jy = -(w2 - w1) / dx / h3c;
+            w1 = dv((bz1[q0] + bz1[qy] + bz1[qz] + bz1[qyz]) * h3, by_cvx);
+            w2 = dv((bz1[qx] + bz1[qxy] + bz1[qxz] + bz1[qxyz]) * h3x, by_cvxp);
+            jy = by_x(dv, -(w2 - w1)) / h3c;
         } else {
-            w1 = (bz1[q0] + bz1[qy] + bz1[qz] + bz1[qyz]) / cvx;
-            w2 = (bz1[qx] + bz1[qxy] + bz1[qxz] + bz1[qxyz]) / cvxp;
-            jy = div_by<P2>(-(w2 - w1), dx, c.rc.xc);
+            w1 = dv((bz1[q0] + bz1[qy] + bz1[qz] + bz1[qyz]), by_cvx);
+            w2 = dv((bz1[qx] + bz1[qxy] + bz1[qxz] + bz1[qxyz]), by_cvxp);
+            jy = by_x(dv, -(w2 - w1));
         }
-        w1 = (bx1[q0] + bx1[qx] + bx1[qy] + bx1[qxy]) / cvz;
-        w2 = (bx1[qz] + bx1[qxz] + bx1[qyz] + bx1[qxyz]) / cvzp;
-        jy += div_by<P2>(w2 - w1, dhz, c.rc.zc);
+        w1 = dv((bx1[q0] + bx1[qx] + bx1[qy] + bx1[qxy]), by_cvz);
+        w2 = dv((bx1[qz] + bx1[qxz] + bx1[qyz] + bx1[qxyz]), by_cvzp);
+        jy += by_z(dv, w2 - w1);
 
         double jz;
         if (geo) {
-            w1 = (by1[q0] + by1[qy] + by1[qz] + by1[qyz]) * h2 / cvx;
-            w2 = (by1[qx] + by1[qxy] + by1[qxz] + by1[qxyz]) * h2x / cvxp;
-            jz = (w2 - w1) / dx / h2c;
+            w1 = dv((by1[q0] + by1[qy] + by1[qz] + by1[qyz]) * h2, by_cvx);
+            w2 = dv((by1[qx] + by1[qxy] + by1[qxz] + by1[qxyz]) * h2x, by_cvxp);
+            jz = by_x(dv, w2 - w1) / h2c;
         } else {
-            w1 = (by1[q0] + by1[qy] + by1[qz] + by1[qyz]) / cvx;
-            w2 = (by1[qx] + by1[qxy] + by1[qxz] + by1[qxyz]) / cvxp;
-            jz = div_by<P2>(w2 - w1, dx, c.rc.xc);
+            w1 = dv((by1[q0] + by1[qy] + by1[qz] + by1[qyz]), by_cvx);
+            w2 = dv((by1[qx] + by1[qxy] + by1[qxz] + by1[qxyz]), by_cvxp);
+            jz = by_x(dv, w2 - w1);
         }
-        w1 = (bx1[q0] + bx1[qx] + bx1[qz] + bx1[qxz]) / cvy;
-        w2 = (bx1[qy] + bx1[qxy] + bx1[qyz] + bx1[qxyz]) / cvyp;
-        jz -= div_by<P2>(w2 - w1, dhy, c.rc.yc);
+        w1 = dv((bx1[q0] + bx1[qx] + bx1[qz] + bx1[qxz]), by_cvy);
+        w2 = dv((bx1[qy] + bx1[qxy] + bx1[qyz] + bx1[qxyz]), by_cvyp);
+        jz -= by_y(dv, w2 - w1);
 
 #define SUM8(a) (a[q0] + a[qx] + a[qy] + a[qxy] + a[qz] + a[qxz] + a[qyz] + a[qxyz])
-        double bxv = SUM8(bx1) / (cvx + cvxp);
-        double byv = SUM8(by1) / (cvx + cvxp);
-        double bzv = SUM8(bz1) / (cvx + cvxp);
+        const typename DV::R by_cv = dv.of(cvx + cvxp);
+        double bxv = dv(SUM8(bx1), by_cv);
+        double byv = dv(SUM8(by1), by_cv);
+        double bzv = dv(SUM8(bz1), by_cv);
 #undef SUM8
-        const double mu0 = c.p.mu0;
-        fx += div_by<P2>(jy * bzv - jz * byv, mu0, c.rc.mu0);
-        fy += div_by<P2>(jz * bxv - jx * bzv, mu0, c.rc.mu0);
-        fz += div_by<P2>(jx * byv - jy * bxv, mu0, c.rc.mu0);
+        const By<P2, DV> by_mu0(dv, c.p.mu0, c.rc.mu0);
+        fx += by_mu0(dv, jy * bzv - jz * byv);
+        fy += by_mu0(dv, jz * bxv - jx * bzv);
+        fz += by_mu0(dv, jx * byv - jy * bxv);
         if (geo) {  // geometric source terms (lagran.cpp:711-721)
             const double rv = __ldg(c.s[S_RHOV] + o), r = c.gf.xb[i + 2];
             const double ux = __ldg(c.f[SAMS_F_VX] + o), uy = __ldg(c.f[SAMS_F_VY] + o), uz = __ldg(c.f[SAMS_F_VZ] + o);
@@ -778,10 +880,10 @@ struct Pred2 {
         c.s[S_FY][o] = sy;
         c.s[S_FZ][o] = sz;
         const double dt = c.sc->dt;
-        const double rho_v = __ldg(c.s[S_RHOV] + o);
-        c.f[SAMS_F_VX1][o] = __ldg(c.f[SAMS_F_VX] + o) + dt / 2.0 * sx / rho_v;
-        c.f[SAMS_F_VY1][o] = __ldg(c.f[SAMS_F_VY] + o) + dt / 2.0 * sy / rho_v;
-        c.f[SAMS_F_VZ1][o] = __ldg(c.f[SAMS_F_VZ] + o) + dt / 2.0 * sz / rho_v;
+        const typename DV::R by_rho = dv.of(__ldg(c.s[S_RHOV] + o));
+        c.f[SAMS_F_VX1][o] = __ldg(c.f[SAMS_F_VX] + o) + dv(dt / 2.0 * sx, by_rho);
+        c.f[SAMS_F_VY1][o] = __ldg(c.f[SAMS_F_VY] + o) + dv(dt / 2.0 * sy, by_rho);
+        c.f[SAMS_F_VZ1][o] = __ldg(c.f[SAMS_F_VZ] + o) + dv(dt / 2.0 * sz, by_rho);
     }
 };
 
@@ -792,12 +894,6 @@ struct Corr1 {
     __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
     {
         set_bounds(lo, hi, 0, g.nx + 1, 0, g.ny + 1, 0, g.nz + 1);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        c.s[S_VH][LOFF(i, j, k)] = heating<GEO, P2>(c, i, j, k);
     }
     // Product of the velocity jumps at the start of the step and of the
     // half step along an edge.  Swapping a and b negates both factors, which
@@ -839,27 +935,6 @@ struct Corr1 {
     }
     // visc_heat of cell (i, j, k) (the corrector's shock_heating)
     template <bool GEO, bool P2>
-    __device__ static double heating(const Ctx &c, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
-        const int mm0 = o - SX - SY, m00 = o - SX, om0 = o - SY;
-        double a[12];
-        a[0] = dd(c, mm0, om0);
-        a[1] = dd(c, om0, o);
-        a[2] = dd(c, o, m00);
-        a[3] = dd(c, m00, mm0);
-        a[4] = dd(c, mm0 + 1, om0 + 1);
-        a[5] = dd(c, om0 + 1, o + 1);
-        a[6] = dd(c, o + 1, m00 + 1);
-        a[7] = dd(c, m00 + 1, mm0 + 1);
-        a[8] = dd(c, o - 1, o);
-        a[9] = dd(c, m00 - 1, m00);
-        a[10] = dd(c, mm0 - 1, mm0);
-        a[11] = dd(c, om0 - 1, om0);
-        return heating_finish<GEO, P2>(c, i, j, k, a);
-    }
-    template <bool GEO, bool P2>
     __device__ __forceinline__ static double heating_finish(const Ctx &c, int i, int j, int k, const double *a)
     {
         const Geom &g = c.g;
@@ -877,7 +952,11 @@ struct Corr1 {
                      0.25 * dx * dz * a2a[o - SX] * a4 - 0.25 * dy * dz * a1a[o + 1] * a5 - 0.25 * dx * dz * a2a[o + 1] * a6 -
                      0.25 * dy * dz * a1a[o + SY + 1] * a7 - 0.25 * dx * dz * a2a[o - SX + 1] * a8 - 0.25 * dy * dy * a3a[o] * a9 -
                      0.25 * dx * dy * a3a[o - SX] * a10 - 0.25 * dy * dy * a3a[o - SX - SY] * a11 - 0.25 * dx * dy * a3a[o - SY] * a12);
-        return pmax(div_by<P2>(vh, cv_at<GEO>(c, i, j, k), c.rc.cv), 0.0);
+        const double cv = cv_at<GEO>(c, i, j, k);
+        if constexpr (P2) return pmax(vh * c.rc.cv, 0.0);
+        FastDiv dv;
+        const double q = dv(vh, dv.of(cv));
+        return pmax(dv.bad ? vh / cv : q, 0.0);
     }
 };
 
@@ -885,39 +964,55 @@ struct Corr1 {
 // (lagran.cpp:754-798).  The corrector's cv1 is not kept: the x sweep
 // recomputes it over the whole range before any read.
 struct Corr2 {
-    static constexpr int kMinBlocks = 6;  // blocks of 256 per SM (register cap), tuned on B200
+    static constexpr int kMinBlocks = 5;  // blocks of 256 per SM (register cap), tuned on B200
     __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
     {
         set_bounds(lo, hi, 0, g.nx, 0, g.ny, 0, g.nz);
     }
+    enum { VX, VY, VZ, EE, EI, RHO, NOUT };
     template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
+    __device__ __forceinline__ static void run(const Ctx &c, int, int i, int j, int k)
     {
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        velocity(c, o, c.f[SAMS_F_VX], c.f[SAMS_F_VY], c.f[SAMS_F_VZ]);
-        if (i < 1 || j < 1 || k < 1) return;
-        energy<GEO, P2>(c, i, j, k, __ldg(c.s[S_VH] + o));
+        const int o = box_off(c.g, i, j, k);
+        const bool cell = i >= 1 && j >= 1 && k >= 1;
+        double out[NOUT];
+        FastDiv dv;
+        compute<GEO, P2>(dv, c, i, j, k, cell, out);
+        if (dv.bad) {
+            double slow[NOUT];
+            compute_ieee<GEO, P2>(c, i, j, k, cell, slow);
+            for (int q = 0; q < NOUT; ++q) out[q] = slow[q];
+        }
+        c.f[SAMS_F_VX][o] = out[VX];
+        c.f[SAMS_F_VY][o] = out[VY];
+        c.f[SAMS_F_VZ][o] = out[VZ];
+        if (!cell) return;
+        c.f[SAMS_F_ENERGY_ELECTRON][o] = out[EE];
+        c.f[SAMS_F_ENERGY_ION][o] = out[EI];
+        c.f[SAMS_F_RHO][o] = out[RHO];
     }
-    // the node's final velocity into nvx/nvy/nvz[o] (the solve's own
-    // arrays in place, or the fused corrector's out-of-place arrays)
-    __device__ static void velocity(const Ctx &c, int o, double *nvx, double *nvy, double *nvz)
-    {
-        const double dt = c.sc->dt;
-        const double rho_v = __ldg(c.s[S_RHOV] + o);
-        const double vxo = c.f[SAMS_F_VX][o], vyo = c.f[SAMS_F_VY][o], vzo = c.f[SAMS_F_VZ][o];
-        // S_FX..S_FZ hold the total force f_visc + f (Pred2)
-        nvx[o] = vxo + dt * __ldg(c.s[S_FX] + o) / rho_v;
-        nvy[o] = vyo + dt * __ldg(c.s[S_FY] + o) / rho_v;
-        nvz[o] = vzo + dt * __ldg(c.s[S_FZ] + o) / rho_v;
-    }
-    // the cell's energies and density with its visc_heat vh (cells 1..n)
     template <bool GEO, bool P2>
-    __device__ static void energy(const Ctx &c, int i, int j, int k, double vh)
+    __device__ static __noinline__ void compute_ieee(const Ctx &c, int i, int j, int k, bool cell, double *out)
+    {
+        IeeeDiv dv;
+        compute<GEO, P2>(dv, c, i, j, k, cell, out);
+    }
+    // the node's final velocity and, on cells 1..n, the energies and density
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static void compute(DV &dv, const Ctx &c, int i, int j, int k, bool cell, double *out)
     {
         const Geom &g = c.g;
         const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
         const double dt = c.sc->dt;
+        {
+            const typename DV::R by_rho = dv.of(__ldg(c.s[S_RHOV] + o));
+            // S_FX..S_FZ hold the total force f_visc + f (Pred2)
+            out[VX] = c.f[SAMS_F_VX][o] + dv(dt * __ldg(c.s[S_FX] + o), by_rho);
+            out[VY] = c.f[SAMS_F_VY][o] + dv(dt * __ldg(c.s[S_FY] + o), by_rho);
+            out[VZ] = c.f[SAMS_F_VZ][o] + dv(dt * __ldg(c.s[S_FZ] + o), by_rho);
+        }
+        out[EE] = out[EI] = out[RHO] = 0.0;
+        if (!cell) return;
         const RO vx1{c.f[SAMS_F_VX1]}, vy1{c.f[SAMS_F_VY1]}, vz1{c.f[SAMS_F_VZ1]};
         const int a = o, am = o - SX, bm = o - SY, cm = o - 1;
         double vxb = 0.25 * (vx1[a] + vx1[bm] + vx1[cm] + vx1[bm - 1]);
@@ -926,16 +1021,16 @@ struct Corr2 {
         double vybm = 0.25 * (vy1[bm] + vy1[bm - SX] + vy1[bm - 1] + vy1[bm - SX - 1]);
         double vzb = 0.25 * (vz1[a] + vz1[am] + vz1[bm] + vz1[am - SY]);
         double vzbm = 0.25 * (vz1[cm] + vz1[am - 1] + vz1[bm - 1] + vz1[am - SY - 1]);
-        double vol = cv_at<GEO>(c, i, j, k);
-        double dvxdx = div_by<P2>(vxb * dxab_at<GEO>(c, i, j, k) - vxbm * dxab_at<GEO>(c, i - 1, j, k), vol, c.rc.cv);
-        double dvydy = div_by<P2>(vyb * dyab_at<GEO>(c, i, j, k) - vybm * dyab_at<GEO>(c, i, j - 1, k), vol, c.rc.cv);
-        double dvzdz = div_by<P2>(vzb * dzab_at<GEO>(c, i, j, k) - vzbm * dzab_at<GEO>(c, i, j, k - 1), vol, c.rc.cv);
-        double dv = (dvxdx + dvydy + dvzdz) * dt;
-        double *rho = c.f[SAMS_F_RHO], *ee = c.f[SAMS_F_ENERGY_ELECTRON], *ei = c.f[SAMS_F_ENERGY_ION];
-        double r = rho[o];
-        ee[o] -= dv * __ldg(c.s[S_PE] + o) / r;
-        ei[o] += (dt * vh - dv * __ldg(c.s[S_PI] + o)) / r;
-        rho[o] = r / (1.0 + dv);
+        const By<P2, DV> by_vol(dv, cv_at<GEO>(c, i, j, k), c.rc.cv);
+        double dvxdx = by_vol(dv, vxb * dxab_at<GEO>(c, i, j, k) - vxbm * dxab_at<GEO>(c, i - 1, j, k));
+        double dvydy = by_vol(dv, vyb * dyab_at<GEO>(c, i, j, k) - vybm * dyab_at<GEO>(c, i, j - 1, k));
+        double dvzdz = by_vol(dv, vzb * dzab_at<GEO>(c, i, j, k) - vzbm * dzab_at<GEO>(c, i, j, k - 1));
+        const double dvol = (dvxdx + dvydy + dvzdz) * dt;
+        const double r = c.f[SAMS_F_RHO][o], vh = __ldg(c.s[S_VH] + o);
+        const typename DV::R by_r = dv.of(r);
+        out[EE] = c.f[SAMS_F_ENERGY_ELECTRON][o] - dv(dvol * __ldg(c.s[S_PE] + o), by_r);
+        out[EI] = c.f[SAMS_F_ENERGY_ION][o] + dv(dt * vh - dvol * __ldg(c.s[S_PI] + o), by_r);
+        out[RHO] = dv(r, dv.of(1.0 + dvol));
     }
 };
 
@@ -991,14 +1086,23 @@ struct SweepVol {
     {
         set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
     }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int arg, int i, int j, int k)
-    {
-        compute<GEO, P2>(c, arg, i, j, k, true);
-    }
     // cv1 of the cell (i, j, k); its outputs are stored where `store`
     template <bool GEO, bool P2>
-    __device__ static double compute(const Ctx &c, int arg, int i, int j, int k, bool store)
+    __device__ __forceinline__ static double compute(const Ctx &c, int arg, int i, int j, int k, bool store)
+    {
+        using DV = typename std::conditional<P2, IeeeDiv, FastDiv>::type;  // (P2 divides by nothing)
+        DV dv;
+        const double cv1 = compute_by<GEO, P2>(dv, c, arg, i, j, k, store);
+        return dv.bad ? compute_ieee<GEO, P2>(c, arg, i, j, k, store) : cv1;
+    }
+    template <bool GEO, bool P2>
+    __device__ static __noinline__ double compute_ieee(const Ctx &c, int arg, int i, int j, int k, bool store)
+    {
+        IeeeDiv dv;
+        return compute_by<GEO, P2>(dv, c, arg, i, j, k, store);
+    }
+    template <bool GEO, bool P2, class DV>
+    __device__ __forceinline__ static double compute_by(DV &dq, const Ctx &c, int arg, int i, int j, int k, bool store)
     {
         const Geom &g = c.g;
         const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
@@ -1025,22 +1129,23 @@ struct SweepVol {
             vzbm = (vz1[cm] + vz1[am - 1] + vz1[bm - 1] + vz1[am - SY - 1]) * 0.25;
             tz = vzb * dzab_at<GEO>(c, i, j, k) - vzbm * dzab_at<GEO>(c, i, j, k - 1);
         }
+        const By<P2, DV> by_vol(dq, vol, c.rc.cv);
         double dv, cv2, db1;
         if (DIR == 0) {
-            double dvxdx = div_by<P2>(tx, vol, c.rc.cv), dvydy = div_by<P2>(1.0 * ty, vol, c.rc.cv), dvzdz = div_by<P2>(1.0 * tz, vol, c.rc.cv);
+            double dvxdx = by_vol(dq, tx), dvydy = by_vol(dq, 1.0 * ty), dvzdz = by_vol(dq, 1.0 * tz);
             dv = (dvydy + dvzdz) * dt;
             cv2 = vol * (1.0 + dv);
             dv = dv + dvxdx * dt;
             db1 = dxb0 + (vxb - vxbm) * dt;
         } else if (DIR == 1) {
-            double dvydy = div_by<P2>(ty, vol, c.rc.cv), dvzdz = div_by<P2>(1.0 * tz, vol, c.rc.cv);
+            double dvydy = by_vol(dq, ty), dvzdz = by_vol(dq, 1.0 * tz);
             dv = dvzdz * dt;
             cv2 = vol * (1.0 + dv);
             dv = dv + dvydy * dt;
             // hyc * dyb (yremap.cpp:78); hyc = 1 in Cartesian geometry
             db1 = ((GEO && c.p.geometry) ? c.gf.hyc[i + 2] * dyb0 : dyb0) + (vyb - vybm) * dt;
         } else {
-            double dvzdz = div_by<P2>(tz, vol, c.rc.cv);
+            double dvzdz = by_vol(dq, tz);
             dv = 0.0 * dt;
             cv2 = vol * (1.0 + dv);
             dv = dv + dvzdz * dt;
@@ -1062,19 +1167,6 @@ struct SweepVol {
 };
 
 struct SweepCvc {
-    static constexpr int kMinBlocks = 4;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 1, -1, g.ny + 1, -1, g.nz + 1);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const ArraySrc src{{c.s[S_R_CV1]}};
-        const int o = LOFF(i, j, k);
-        node(c, o, src, o, g.sx, g.sy, 1);
-    }
     // cvc1 at the node at offset o from cv1 of its eight cells read through
     // src(0, q), q = q0 + dx*QX + dy*QY + dz*QZ (dx, dy, dz in {0, 1})
     template <class S>
@@ -1083,55 +1175,6 @@ struct SweepCvc {
         c.s[S_R_CVC1][o] = 0.125 * (src(0, q0) + src(0, q0 + QX) + src(0, q0 + QY) + src(0, q0 + QX + QY) +
                                     src(0, q0 + QZ) + src(0, q0 + QX + QZ) + src(0, q0 + QY + QZ) +
                                     src(0, q0 + QX + QY + QZ));
-    }
-};
-
-// Both constrained-transport fluxes of a sweep.
-template <int DIR>
-struct SweepCT {
-    static constexpr int kMinBlocks = 4;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, 0, g.nx, 0, g.ny, 0, g.nz);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
-        const int d = dir_stride(g, DIR);
-        const double dt = c.sc->dt;
-        const RO db1{c.s[S_R_DB1]}, cvc1{c.s[S_R_CVC1]}, cv1{c.s[S_R_CV1]};
-        const RO v1{c.f[SAMS_F_VX1 + DIR]};
-        // transverse offsets of the two db1 samples averaged for each flux
-        int t1, t2, va1, va2;
-        RO b1, b2;
-        if (DIR == 0) {        // vx_by (avg +y, v avg -z), vx_bz (avg +z, v avg -y)
-            t1 = SY; va1 = -1; b1.p = c.f[SAMS_F_BY];
-            t2 = 1;  va2 = -SY; b2.p = c.f[SAMS_F_BZ];
-        } else if (DIR == 1) { // vy_bx (avg +x, v avg -z), vy_bz (avg +z, v avg -x)
-            t1 = SX; va1 = -1; b1.p = c.f[SAMS_F_BX];
-            t2 = 1;  va2 = -SX; b2.p = c.f[SAMS_F_BZ];
-        } else {               // vz_bx (avg +x, v avg -y), vz_by (avg +y, v avg -x)
-            t1 = SX; va1 = -SY; b1.p = c.f[SAMS_F_BX];
-            t2 = SY; va2 = -SX; b2.p = c.f[SAMS_F_BY];
-        }
-        const double dci = cvc1[o], dcm = cvc1[o - d], dcp = cvc1[o + d], cvi = cv1[o], cvp = cv1[o + d];
-        {
-            double v = (v1[o] + v1[o + va1]) * 0.5;
-            double dbm = (db1[o - d] + db1[o - d + t1]) * 0.5, dbi = (db1[o] + db1[o + t1]) * 0.5;
-            double dbp = (db1[o + d] + db1[o + d + t1]) * 0.5, dbp2 = (db1[o + 2 * d] + db1[o + 2 * d + t1]) * 0.5;
-            c.s[S_R_CT1][o] = ct_flux(v, dt, b1[o - d], b1[o], b1[o + d], b1[o + 2 * d], dbm, dbi, dbp, dbp2,
-                                      dci, dcm, dcp, cvi, cvp);
-        }
-        {
-            double v = (v1[o] + v1[o + va2]) * 0.5;
-            double dbm = (db1[o - d] + db1[o - d + t2]) * 0.5, dbi = (db1[o] + db1[o + t2]) * 0.5;
-            double dbp = (db1[o + d] + db1[o + d + t2]) * 0.5, dbp2 = (db1[o + 2 * d] + db1[o + 2 * d + t2]) * 0.5;
-            c.s[S_R_CT2][o] = ct_flux(v, dt, b2[o - d], b2[o], b2[o + d], b2[o + 2 * d], dbm, dbi, dbp, dbp2,
-                                      dci, dcm, dcp, cvi, cvp);
-        }
-        (void)SX;
     }
 };
 
@@ -1231,35 +1274,15 @@ __device__ __forceinline__ double face_area(const Ctx &c, int i, int j, int k)
     return DIR == 0 ? dxab_at<GEO>(c, i, j, k) : (DIR == 1 ? dyab_at<GEO>(c, i, j, k) : dzab_at<GEO>(c, i, j, k));
 }
 
-template <int DIR>
-struct SweepMass {
-    static constexpr int kMinBlocks = 5;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, 0, DIR == 0 ? g.nx : g.nx + 1, 0, DIR == 1 ? g.ny : g.ny + 1, 0,
-                   DIR == 2 ? g.nz : g.nz + 1);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        const int d = dir_stride(g, DIR);
-        const RO rho{c.f[SAMS_F_RHO]}, cvc1{c.s[S_R_CVC1]}, cv1{c.s[S_R_CV1]};
-        double v = face_velocity<DIR>(c, o);
-        c.f[SAMS_F_DM][o] = mass_flux(v, c.sc->dt, face_area<DIR, GEO>(c, i, j, k), rho[o - d], rho[o], rho[o + d],
-                                      rho[o + 2 * d], cvc1[o], cvc1[o - d], cvc1[o + d], cv1[o], cv1[o + d]);
-    }
-};
-
 // What SweepCTMass writes into dm's ghosts along the sweep.
 enum { kNoImages = 0, kPeriodicImages, kCopyImages };
 
-// SweepCT and SweepMass of one sweep in one kernel (k_ctmass): every
-// quotient b/db of the CT fluxes is formed once per point into a window store
-// and read by the four fluxes along the sweep that use it (the separate
-// kernel forms each four times).  quot() at one point along the sweep, then
-// fluxes() at the window's own points.
+// The two CT fluxes and the mass flux of one sweep in one kernel (k_ctmass):
+// every quotient b/db of the CT fluxes is formed once per point into a window
+// store and read by the four fluxes along the sweep that use it.  quot() at
+// one point along the sweep, then fluxes() at the window's own points.  (The
+// reciprocal of cvc1, which all three fluxes divide by, is formed again where
+// it is used: kept in the store too it cost 4 to 11% of the kernel.)
 template <int DIR>
 struct SweepCTMass {
     enum { F1, F2, DB1, DB2, NARR };  // the two quotients and their db averages
@@ -1274,7 +1297,20 @@ struct SweepCTMass {
     // scale: B is not yet in flux form (the x sweep with the scaling folded
     // into SweepCTUpd<0>): form BScale's b * area here, the same product
     template <bool GEO, class A>
-    __device__ static void quot(const Ctx &c, int i, int j, int k, A st, bool scale)
+    __device__ __forceinline__ static void quot(const Ctx &c, int i, int j, int k, A st, bool scale)
+    {
+        FastDiv dv;
+        quotients<GEO>(dv, c, i, j, k, st, scale);
+        if (dv.bad) quotients_ieee<GEO>(c, i, j, k, st, scale);
+    }
+    template <bool GEO, class A>
+    __device__ static __noinline__ void quotients_ieee(const Ctx &c, int i, int j, int k, A st, bool scale)
+    {
+        IeeeDiv dv;
+        quotients<GEO>(dv, c, i, j, k, st, scale);
+    }
+    template <bool GEO, class DV, class A>
+    __device__ __forceinline__ static void quotients(DV &dv, const Ctx &c, int i, int j, int k, A st, bool scale)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
@@ -1288,8 +1324,8 @@ struct SweepCTMass {
             v1 = v1 * dyab_at<GEO>(c, i, j, k);
             v2 = v2 * dzab_at<GEO>(c, i, j, k);
         }
-        st.put(F1, v1 / dba1);
-        st.put(F2, v2 / dba2);
+        st.put(F1, dv(v1, dv.of(dba1)));
+        st.put(F2, dv(v2, dv.of(dba2)));
         st.put(DB1, dba1);
         st.put(DB2, dba2);
     }
@@ -1302,27 +1338,14 @@ struct SweepCTMass {
     // index 0, which that fill overwrites, is left alone, so the fill is not
     // needed.
     template <bool GEO, class A>
-    __device__ static void fluxes(const Ctx &c, int i, int j, int k, A st, bool ct, int images)
+    __device__ __forceinline__ static void fluxes(const Ctx &c, int i, int j, int k, A st, bool ct, int images)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
         const int d = dir_stride(g, DIR);
-        const double dt = c.sc->dt;
-        const RO cvc1{c.s[S_R_CVC1]}, cv1{c.s[S_R_CV1]};
-        const double dci = cvc1[o], dcm = cvc1[o - d], dcp = cvc1[o + d], cvi = cv1[o], cvp = cv1[o + d];
-        if (ct) {
-            int t1, t2, va1, va2;
-            offsets(g, t1, t2, va1, va2);
-            const RO v1{c.f[SAMS_F_VX1 + DIR]};
-            const double v1o = v1[o];
-            c.s[S_R_CT1][o] = ct_flux_q((v1o + v1[o + va1]) * 0.5, dt, st.get(F1, -1), st.get(F1, 0), st.get(F1, 1),
-                                        st.get(F1, 2), st.get(DB1, 0), st.get(DB1, 1), dci, dcm, dcp, cvi, cvp);
-            c.s[S_R_CT2][o] = ct_flux_q((v1o + v1[o + va2]) * 0.5, dt, st.get(F2, -1), st.get(F2, 0), st.get(F2, 1),
-                                        st.get(F2, 2), st.get(DB2, 0), st.get(DB2, 1), dci, dcm, dcp, cvi, cvp);
-        }
-        const RO rho{c.f[SAMS_F_RHO]};
-        const double m = mass_flux(face_velocity<DIR>(c, o), dt, face_area<DIR, GEO>(c, i, j, k), rho[o - d],
-                                   rho[o], rho[o + d], rho[o + 2 * d], dci, dcm, dcp, cvi, cvp);
+        FastDiv dv;
+        double m = three<GEO>(dv, c, i, j, k, st, ct);
+        if (dv.bad) m = three_ieee<GEO>(c, i, j, k, st, ct);
         double *dm = c.f[SAMS_F_DM];
         if (images == kNoImages) {
             dm[o] = m;
@@ -1339,6 +1362,46 @@ struct SweepCTMass {
         if (s >= nd - 1) dm[o - nd * d] = m;
         if (s >= 1 && s <= 2) dm[o + nd * d] = m;
     }
+    template <bool GEO, class A>
+    __device__ static __noinline__ double three_ieee(const Ctx &c, int i, int j, int k, A st, bool ct)
+    {
+        IeeeDiv dv;
+        return three<GEO>(dv, c, i, j, k, st, ct);
+    }
+    // stores the CT fluxes where `ct` and returns the mass flux
+    template <bool GEO, class DV, class A>
+    __device__ __forceinline__ static double three(DV &dv, const Ctx &c, int i, int j, int k, A st, bool ct)
+    {
+        const Geom &g = c.g;
+        const int o = LOFF(i, j, k);
+        const int d = dir_stride(g, DIR);
+        const double dt = c.sc->dt;
+        const RO cvc1{c.s[S_R_CVC1]}, cv1{c.s[S_R_CV1]};
+        const double dcm = cvc1[o - d], dcp = cvc1[o + d], cvi = cv1[o], cvp = cv1[o + d];
+        const typename DV::R ci = dv.of(cvc1[o]);
+        auto face = [&](bool up, double phi, double bu) {
+            return Face<DV>{up, phi, ci, dv.of(pick(up, dcm, dcp)), bu};
+        };
+        if (ct) {
+            int t1, t2, va1, va2;
+            offsets(g, t1, t2, va1, va2);
+            const RO v1{c.f[SAMS_F_VX1 + DIR]};
+            const double v1o = v1[o];
+            auto flux = [&](int f, int db, int va) {
+                const double v = (v1o + v1[o + va]) * 0.5, o_v = v * dt;
+                const bool up = v >= 0.0;
+                const Face<DV> F = face(up, dv.fraction(fabs(o_v), dv.of(pick(up, st.get(db, 0), st.get(db, 1)))), pick(up, cvi, cvp));
+                return swept_flux(dv, F, o_v, st.get(f, -1), st.get(f, 0), st.get(f, 1), st.get(f, 2));
+            };
+            c.s[S_R_CT1][o] = flux(F1, DB1, va1);
+            c.s[S_R_CT2][o] = flux(F2, DB2, va2);
+        }
+        const RO rho{c.f[SAMS_F_RHO]};
+        const double v = face_velocity<DIR>(c, o), o_v = v * dt * face_area<DIR, GEO>(c, i, j, k);
+        const bool up = v >= 0.0;
+        const double bu = pick(up, cvi, cvp);
+        return swept_flux(dv, face(up, dv.fraction(fabs(o_v), dv.of(bu)), bu), o_v, rho[o - d], rho[o], rho[o + d], rho[o + 2 * d]);
+    }
 };
 
 // Range lo/hi of index q in dimension DIM for a sweep-direction-dependent
@@ -1348,6 +1411,36 @@ __device__ __forceinline__ bool in_sweep_range(int q, int n, int alo, int ahi_of
 {
     return DIM == DIR ? (q >= alo && q <= n + ahi_off) : (q >= blo && q <= n + bhi_off);
 }
+
+// The face through which a sweep carries both specific energies, and the one
+// of the three momenta, where cv1 and cvc1 change roles.
+template <class DV>
+struct CarryFace {
+    Face<DV> F;
+    double dmu;
+    // o_v the swept volume, lengths dci (at the face), dcm / dcp (below /
+    // above), volumes and densities on its two sides
+    template <bool ZFORM>
+    __device__ __forceinline__ void set(DV &dv, bool up, double o_v, double dci, double dcm, double dcp, double vi, double vp,
+                                        double ri, double rp, double dm)
+    {
+        const typename DV::R bu = dv.of(pick(up, vi, vp));
+        F.up = up;
+        F.phi = dv.fraction(fabs(o_v), bu);
+        F.ci = dv.of(dci);
+        F.cu = dv.of(pick(up, dcm, dcp));
+        F.bu = bu.d;
+        dmu = mass_fraction<ZFORM>(dv, dm, bu, pick(up, ri, rp));
+    }
+    __device__ __forceinline__ double carry(DV &dv, const double *f, int o, int d) const
+    {
+        return carried(dv, F, __ldg(f + o - d), __ldg(f + o), __ldg(f + o + d), __ldg(f + o + 2 * d), dmu);
+    }
+    __device__ __forceinline__ double carry_coherent(DV &dv, const double *f, int o, int d) const
+    {
+        return carried(dv, F, f[o - d], f[o], f[o + d], f[o + 2 * d], dmu);
+    }
+};
 
 // rho update, energy fluxes, vertex density, node cv2, node dm and the v1
 // shift (xremap.cpp:121-221 and the y/z analogues).
@@ -1378,11 +1471,12 @@ struct SweepS6 {
         if (all0n) {
             double v = face_velocity<DIR>(c, o);
             double area = face_area<DIR, GEO>(c, i, j, k);
-            const RO ee{c.f[SAMS_F_ENERGY_ELECTRON]}, ei{c.f[SAMS_F_ENERGY_ION]};
-            c.s[S_R_FE1][o] = energy_flux(v, dt, area, ee[o - d], ee[o], ee[o + d], ee[o + 2 * d], cvc1[o], cvc1[o - d],
-                                          cvc1[o + d], cv1[o], cv1[o + d], rho1[o], rho1[o + d], dm[o]);
-            c.s[S_R_FE2][o] = energy_flux(v, dt, area, ei[o - d], ei[o], ei[o + d], ei[o + 2 * d], cvc1[o], cvc1[o - d],
-                                          cvc1[o + d], cv1[o], cv1[o + d], rho1[o], rho1[o + d], dm[o]);
+            IeeeDiv dv;
+            CarryFace<IeeeDiv> F;
+            F.set<false>(dv, v >= 0.0, v * dt * area, cvc1[o], cvc1[o - d], cvc1[o + d], cv1[o], cv1[o + d], rho1[o],
+                         rho1[o + d], dm[o]);
+            c.s[S_R_FE1][o] = F.carry(dv, c.f[SAMS_F_ENERGY_ELECTRON], o, d) * dm[o];
+            c.s[S_R_FE2][o] = F.carry(dv, c.f[SAMS_F_ENERGY_ION], o, d) * dm[o];
             // node cv2 (0..n)^3
             c.s[S_R_CV2N][o] = (cv2[o] + cv2[o + SX] + cv2[o + SY] + cv2[o + SX + SY] +
                                 cv2[o + 1] + cv2[o + SX + 1] + cv2[o + SY + 1] + cv2[o + SX + SY + 1]) * 0.125;
@@ -1435,15 +1529,12 @@ struct SweepS7 {
         // x sweep uses dxac; the y and z sweeps both use dyac (zremap.cpp:475)
         double area = DIR == 0 ? dxac_at<GEO>(c, i, j, k) : dyac_at<GEO>(c, i, j, k);
         const double v = v1s[o], dmv = dmn[o];
-        const double dci = cv1[o + d], dcm = cv1[o], dcp = cv1[o + 2 * d], cvi = cvc1[o], cvp = cvc1[o + d];
-        const double rvi = rv[o], rvp = rv[o + d];
-        const RO ux{c.f[SAMS_F_VX]}, uy{c.f[SAMS_F_VY]}, uz{c.f[SAMS_F_VZ]};
-        const double f1 = mom_flux<DIR == 2>(v, dt, area, ux[o - d], ux[o], ux[o + d], ux[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
-        const double f2 = mom_flux<DIR == 2>(v, dt, area, uy[o - d], uy[o], uy[o + d], uy[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
-        const double f3 = mom_flux<DIR == 2>(v, dt, area, uz[o - d], uz[o], uz[o + d], uz[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
+        IeeeDiv dv;
+        CarryFace<IeeeDiv> F;
+        const double o_v = v * dt * area;
+        F.set<DIR == 2>(dv, o_v >= 0.0, o_v, cv1[o + d], cv1[o], cv1[o + 2 * d], cvc1[o], cvc1[o + d], rv[o], rv[o + d], dmv);
+        const double f1 = F.carry(dv, c.f[SAMS_F_VX], o, d), f2 = F.carry(dv, c.f[SAMS_F_VY], o, d),
+                     f3 = F.carry(dv, c.f[SAMS_F_VZ], o, d);
         // with the rke correction the flux is kept as is (its kinetic-energy
         // error needs it) and SweepS8 takes the product with dm
         const bool raw = c.p.rke != 0;
@@ -1559,7 +1650,21 @@ struct SweepFused {
 
     // SweepS6 at (i, j, k), sweep index -2..n+1.
     template <bool GEO, class A>
-    __device__ static void stage_a(const Ctx &c, int i, int j, int k, A b, const SweepOut &w, bool own)
+    __device__ __forceinline__ static void stage_a(const Ctx &c, int i, int j, int k, A b, const SweepOut &w, bool own)
+    {
+        FastDiv dv;
+        stage_a_by<GEO>(dv, c, i, j, k, b, w, own);
+        if (dv.bad) stage_a_ieee<GEO>(c, i, j, k, b, w, own);
+    }
+    template <bool GEO, class A>
+    __device__ static __noinline__ void stage_a_ieee(const Ctx &c, int i, int j, int k, A b, const SweepOut w, bool own)
+    {
+        IeeeDiv dv;
+        stage_a_by<GEO>(dv, c, i, j, k, b, w, own);
+    }
+    template <bool GEO, class DV, class A>
+    __device__ __forceinline__ static void stage_a_by(DV &dv, const Ctx &c, int i, int j, int k, A b, const SweepOut &w,
+                                                      bool own)
     {
         const Geom &g = c.g;
         const int SX = g.sx, SY = g.sy, o = LOFF(i, j, k);
@@ -1570,22 +1675,23 @@ struct SweepFused {
         const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
         const int qd = DIR == 0 ? i : (DIR == 1 ? j : k);
         if (own && i >= 1 && j >= 1 && k >= 1 && i <= g.nx && j <= g.ny && k <= g.nz)
-            w.rho[o] = (rho1[o] * cv1[o] + dm[o - d] - dm[o]) / cv2[o];
+            w.rho[o] = dv(rho1[o] * cv1[o] + dm[o - d] - dm[o], dv.of(cv2[o]));
         if (qd >= 0 && qd <= nd) {  // the lines are 0..n across the sweep
             double v = face_velocity<DIR>(c, o);
             double area = face_area<DIR, GEO>(c, i, j, k);
-            const RO ee{c.f[SAMS_F_ENERGY_ELECTRON]}, ei{c.f[SAMS_F_ENERGY_ION]};
-            b.put(FE1, energy_flux(v, dt, area, ee[o - d], ee[o], ee[o + d], ee[o + 2 * d], cvc1[o], cvc1[o - d],
-                                   cvc1[o + d], cv1[o], cv1[o + d], rho1[o], rho1[o + d], dm[o]));
-            b.put(FE2, energy_flux(v, dt, area, ei[o - d], ei[o], ei[o + d], ei[o + 2 * d], cvc1[o], cvc1[o - d],
-                                   cvc1[o + d], cv1[o], cv1[o + d], rho1[o], rho1[o + d], dm[o]));
+            CarryFace<DV> F;
+            F.template set<false>(dv, v >= 0.0, v * dt * area, cvc1[o], cvc1[o - d], cvc1[o + d], cv1[o], cv1[o + d], rho1[o],
+                                  rho1[o + d], dm[o]);
+            b.put(FE1, F.carry(dv, c.f[SAMS_F_ENERGY_ELECTRON], o, d) * dm[o]);
+            b.put(FE2, F.carry(dv, c.f[SAMS_F_ENERGY_ION], o, d) * dm[o]);
         }
         if (qd >= -1) {
             double sum = rho1[o] * cv1[o] + rho1[o + SX] * cv1[o + SX] + rho1[o + SY] * cv1[o + SY] +
                          rho1[o + SX + SY] * cv1[o + SX + SY] + rho1[o + 1] * cv1[o + 1] +
                          rho1[o + SX + 1] * cv1[o + SX + 1] + rho1[o + SY + 1] * cv1[o + SY + 1] +
                          rho1[o + SX + SY + 1] * cv1[o + SX + SY + 1];
-            b.put(RVN, DIR == 0 ? sum * 0.125 / cvc1[o] : sum * (0.125 / cvc1[o]));
+            const typename DV::R by_cvc = dv.of(cvc1[o]);
+            b.put(RVN, DIR == 0 ? dv(sum * 0.125, by_cvc) : sum * dv(0.125, by_cvc));
         }
         if (qd >= -1 && qd <= nd)
             b.put(DMN, (dm[o] + dm[o + SX] + dm[o + SY] + dm[o + SX + SY] + dm[o + 1] + dm[o + SX + 1] +
@@ -1601,9 +1707,16 @@ struct SweepFused {
         const int o = box_off(c.g, i, j, k);
         const RO rho1{c.s[S_R_RHO1]}, cv1{c.s[S_R_CV1]}, cv2{c.s[S_R_CV2]};
         const double *ee = c.f[SAMS_F_ENERGY_ELECTRON], *ei = c.f[SAMS_F_ENERGY_ION];
-        double den = cv2[o] * w.rho[o];  // stage A's rho (a coherent load)
-        const double e_new = (ee[o] * cv1[o] * rho1[o] + b.get(FE1, -1) - b.get(FE1, 0)) / den;
-        const double i_new = (ei[o] * cv1[o] * rho1[o] + b.get(FE2, -1) - b.get(FE2, 0)) / den;
+        const double den = cv2[o] * w.rho[o];  // stage A's rho (a coherent load)
+        const double xe = ee[o] * cv1[o] * rho1[o] + b.get(FE1, -1) - b.get(FE1, 0);
+        const double xi = ei[o] * cv1[o] * rho1[o] + b.get(FE2, -1) - b.get(FE2, 0);
+        FastDiv dv;
+        const Rcp by_den = dv.of(den);
+        double e_new = dv(xe, by_den), i_new = dv(xi, by_den);
+        if (dv.bad) {
+            e_new = xe / den;
+            i_new = xi / den;
+        }
         w.ee[o] = e_new;
         w.ei[o] = i_new;
     }
@@ -1612,7 +1725,20 @@ struct SweepFused {
     // -1..n (after stage_b_energy everywhere: they overwrite the energy
     // fluxes).
     template <bool GEO, class A>
-    __device__ static void stage_b_mom(const Ctx &c, int i, int j, int k, A b)
+    __device__ __forceinline__ static void stage_b_mom(const Ctx &c, int i, int j, int k, A b)
+    {
+        FastDiv dv;
+        stage_b_mom_by<GEO>(dv, c, i, j, k, b);
+        if (dv.bad) stage_b_mom_ieee<GEO>(c, i, j, k, b);
+    }
+    template <bool GEO, class A>
+    __device__ static __noinline__ void stage_b_mom_ieee(const Ctx &c, int i, int j, int k, A b)
+    {
+        IeeeDiv dv;
+        stage_b_mom_by<GEO>(dv, c, i, j, k, b);
+    }
+    template <bool GEO, class DV, class A>
+    __device__ __forceinline__ static void stage_b_mom_by(DV &dv, const Ctx &c, int i, int j, int k, A b)
     {
         const Geom &g = c.g;
         const int o = LOFF(i, j, k);
@@ -1623,15 +1749,12 @@ struct SweepFused {
         double area = DIR == 0 ? dxac_at<GEO>(c, i, j, k) : dyac_at<GEO>(c, i, j, k);
         const RO v1{c.f[SAMS_F_VX1 + DIR]};
         const double v = (v1[o] + v1[o + d]) * 0.5, dmv = b.get(DMN, 0);
-        const double dci = cv1[o + d], dcm = cv1[o], dcp = cv1[o + 2 * d], cvi = cvc1[o], cvp = cvc1[o + d];
-        const double rvi = b.get(RVN, 0), rvp = b.get(RVN, 1);
-        const double *ux = c.f[SAMS_F_VX], *uy = c.f[SAMS_F_VY], *uz = c.f[SAMS_F_VZ];
-        const double f1 = mom_flux<DIR == 2>(v, dt, area, ux[o - d], ux[o], ux[o + d], ux[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
-        const double f2 = mom_flux<DIR == 2>(v, dt, area, uy[o - d], uy[o], uy[o + d], uy[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
-        const double f3 = mom_flux<DIR == 2>(v, dt, area, uz[o - d], uz[o], uz[o + d], uz[o + 2 * d], dci, dcm, dcp,
-                                             cvi, cvp, rvi, rvp, dmv);
+        CarryFace<DV> F;
+        const double o_v = v * dt * area;
+        F.template set<DIR == 2>(dv, o_v >= 0.0, o_v, cv1[o + d], cv1[o], cv1[o + 2 * d], cvc1[o], cvc1[o + d], b.get(RVN, 0),
+                                 b.get(RVN, 1), dmv);
+        const double f1 = F.carry_coherent(dv, c.f[SAMS_F_VX], o, d), f2 = F.carry_coherent(dv, c.f[SAMS_F_VY], o, d),
+                     f3 = F.carry_coherent(dv, c.f[SAMS_F_VZ], o, d);
         b.put(FM1, f1 * dmv);
         b.put(FM2, f2 * dmv);
         b.put(FM3, f3 * dmv);
@@ -1647,12 +1770,20 @@ struct SweepFused {
         const double cv2o = (cv2[o] + cv2[o + SX] + cv2[o + SY] + cv2[o + SX + SY] + cv2[o + 1] + cv2[o + SX + 1] +
                              cv2[o + SY + 1] + cv2[o + SX + SY + 1]) * 0.125;
         const double rvo = b.get(RVN, 0), cvco = __ldg(c.s[S_R_CVC1] + o);
-        const double rho_v1 = (rvo * cvco + b.get(DMN, -1) - b.get(DMN, 0)) / cv2o;
-        const double den = cv2o * rho_v1;
+        const double xr = rvo * cvco + b.get(DMN, -1) - b.get(DMN, 0);
         const double *ux = c.f[SAMS_F_VX], *uy = c.f[SAMS_F_VY], *uz = c.f[SAMS_F_VZ];
-        const double nx = (rvo * ux[o] * cvco + b.get(FM1, -1) - b.get(FM1, 0)) / den;
-        const double ny = (rvo * uy[o] * cvco + b.get(FM2, -1) - b.get(FM2, 0)) / den;
-        const double nz = (rvo * uz[o] * cvco + b.get(FM3, -1) - b.get(FM3, 0)) / den;
+        const double xx = rvo * ux[o] * cvco + b.get(FM1, -1) - b.get(FM1, 0);
+        const double xy = rvo * uy[o] * cvco + b.get(FM2, -1) - b.get(FM2, 0);
+        const double xz = rvo * uz[o] * cvco + b.get(FM3, -1) - b.get(FM3, 0);
+        FastDiv dv;
+        const Rcp by_den = dv.of(cv2o * dv(xr, dv.of(cv2o)));
+        double nx = dv(xx, by_den), ny = dv(xy, by_den), nz = dv(xz, by_den);
+        if (dv.bad) {
+            const double den = cv2o * (xr / cv2o);
+            nx = xx / den;
+            ny = xy / den;
+            nz = xz / den;
+        }
         w.ux[o] = nx;
         w.uy[o] = ny;
         w.uz[o] = nz;
@@ -1818,18 +1949,6 @@ template <class Op>
 struct CapP2 {
     static constexpr int value = Op::kMinBlocks;
 };
-template <>
-struct CapP2<NodePrep> {
-    static constexpr int value = 5;
-};
-template <>
-struct CapP2<ResistRK> {
-    static constexpr int value = 5;
-};
-template <>
-struct CapP2<Pred1> {
-    static constexpr int value = 6;
-};
 
 // Register cap of an op in the batched engine (lare_batch.cu), whose solves
 // are typically thin (n x n x 4): rows of nine doubles, tiles of eight
@@ -1840,11 +1959,8 @@ struct CapBatch {
     static constexpr int value = Op::kMinBlocks;
 };
 template <> struct CapBatch<BScale> { static constexpr int value = 8; };
-template <> struct CapBatch<SweepCvc> { static constexpr int value = 8; };
 template <> struct CapBatch<Corr2> { static constexpr int value = 5; };
-template <int D> struct CapBatch<SweepVol<D>> { static constexpr int value = 4; };
 template <int D> struct CapBatch<SweepCTUpd<D>> { static constexpr int value = 8; };
-template <int D> struct CapBatch<SweepMass<D>> { static constexpr int value = 4; };
 template <int D> struct CapBatch<SweepS7<D>> { static constexpr int value = 4; };
 template <int D> struct CapBatch<SweepS8<D>> { static constexpr int value = 8; };
 

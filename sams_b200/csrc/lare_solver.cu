@@ -44,7 +44,7 @@ constexpr int kThreads = 256;
 // geometry is curvilinear (its metric factors are applied); the Cartesian
 // instantiation has no trace of them.
 template <class Op, bool GEO, bool P2>
-__global__ void __launch_bounds__(kThreads, (MinBlocks<Op, P2>::value)) k_op(Ctx c, int arg)
+__global__ void __launch_bounds__(kThreads, (MinBlocks<Op, P2>::value)) k_op(const __grid_constant__ Ctx c, int arg)
 {
     int lo[3], hi[3];
     Op::bounds(c.g, arg, lo, hi);
@@ -69,56 +69,56 @@ using march::WinTile;
 using march::ZTile;
 
 template <bool GEO, bool P2, int CW>
-__global__ void __launch_bounds__(kMThreads, 3) k_pred_march(Ctx c, MarchTile m, int resistive, double *pe_out, double *pi_out)
+__global__ void __launch_bounds__(kMThreads, 3) k_pred_march(const __grid_constant__ Ctx c, MarchTile m, int resistive, double *pe_out, double *pi_out)
 {
     extern __shared__ double ring[];
     march::pred<GEO, P2, CW>(c, m, (int)blockIdx.x, resistive, pe_out, pi_out, ring);
 }
 
 template <class P, bool GEO, bool P2, int CW>
-__global__ void __launch_bounds__(kMThreads, P::kMinBlocks) k_cellnode_march(Ctx c, MarchTile m, int arg)
+__global__ void __launch_bounds__(kMThreads, P::kMinBlocks) k_cellnode_march(const __grid_constant__ Ctx c, MarchTile m, int arg)
 {
     extern __shared__ double ring[];
     march::cellnode<P, GEO, P2, CW>(c, m, (int)blockIdx.x, arg, ring);
 }
 
 template <bool GEO, bool P2, int CW>
-__global__ void __launch_bounds__(kMThreads, march::kHeatMinBlocks) k_heat_march(Ctx c, MarchTile m)
+__global__ void __launch_bounds__(kMThreads, march::kHeatMinBlocks) k_heat_march(const __grid_constant__ Ctx c, MarchTile m)
 {
     extern __shared__ double ring[];
     march::heat_edges<GEO, P2, CW>(c, m, (int)blockIdx.x, ring);
 }
 
 template <bool GEO, bool P2, int CW>
-__global__ void __launch_bounds__(kMThreads, 5) k_resist_march(Ctx c, MarchTile m, double *nbx, double *nby, double *nbz)
+__global__ void __launch_bounds__(kMThreads, P2 ? 5 : 4) k_resist_march(const __grid_constant__ Ctx c, MarchTile m, double *nbx, double *nby, double *nbz)
 {
     extern __shared__ double ring[];
     march::resist<GEO, P2, CW>(c, m, (int)blockIdx.x, nbx, nby, nbz, ring);
 }
 
 template <int DIR, bool GEO>
-__global__ void __launch_bounds__(ops::kWinThreads, 5) k_ctmass(Ctx c, WinTile w, int scale, int images)  // cap tuned on B200
+__global__ void __launch_bounds__(ops::kWinThreads, 5) k_ctmass(const __grid_constant__ Ctx c, WinTile w, int scale, int images)  // cap tuned on B200
 {
     extern __shared__ double csm[];
     march::ctmass<DIR, GEO>(c, w, (int)blockIdx.x, scale, images, csm);
 }
 
 template <bool GEO>
-__global__ void __launch_bounds__(march::kZCtThreads, 4) k_ctmass_z(Ctx c, ZTile z, int images)
+__global__ void __launch_bounds__(march::kZCtThreads, 4) k_ctmass_z(const __grid_constant__ Ctx c, ZTile z, int images)
 {
     __shared__ double zsm[ops::SweepCTMass<2>::NARR * march::kZCtThreads];
     march::ctmass_z<GEO>(c, z, (int)blockIdx.x, images, zsm);
 }
 
 template <int DIR, bool GEO>
-__global__ void __launch_bounds__(ops::kWinThreads, 4) k_psweep(Ctx c, WinTile wt, ops::SweepOut w, int ct_arg)  // window shape and cap tuned on B200
+__global__ void __launch_bounds__(ops::kWinThreads, 4) k_psweep(const __grid_constant__ Ctx c, WinTile wt, ops::SweepOut w, int ct_arg)  // window shape and cap tuned on B200
 {
     extern __shared__ double psm[];
     march::psweep<DIR, GEO>(c, wt, (int)blockIdx.x, w, ct_arg, psm);
 }
 
 template <bool GEO>
-__global__ void __launch_bounds__(kZThreads, 4) k_zsweep(Ctx c, int ct_arg)  // 4 blocks per SM: 96^3 133 -> 116 us, 256^3 1.45 -> 1.36 ms against 5; 3 was 10% slower
+__global__ void __launch_bounds__(kZThreads, 4) k_zsweep(const __grid_constant__ Ctx c, int ct_arg)  // 4 blocks per SM: 96^3 133 -> 116 us, 256^3 1.45 -> 1.36 ms against 5; 3 was 10% slower
 {
     extern __shared__ double zsm[];
     march::zsweep<GEO>(c, (int)blockIdx.x, ct_arg, zsm);
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kZThreads, 4) k_zsweep(Ctx c, int ct_arg)  // 
 // energies outside 1..n, velocities outside 0..n in some dimension): copied
 // from the solve's arrays, so the new arrays are complete boxes.  One
 // thread per shell point: the rho / energy shell, then the velocity shell.
-__global__ void __launch_bounds__(kThreads) k_copy_shell(Ctx c, ops::SweepOut w)
+__global__ void __launch_bounds__(kThreads) k_copy_shell(const __grid_constant__ Ctx c, ops::SweepOut w)
 {
     ops::copy_shell(c, c.g, w, (long long)blockIdx.x * blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
 }
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kThreads) k_copy_shell(Ctx c, ops::SweepOut w)
 // doubles order like their bit patterns, so an integer atomicMin is an
 // exact, order-free minimum.
 template <bool GEO, bool P2>
-__global__ void __launch_bounds__(kThreads, 4) k_visc_split(Ctx c)  // 4 blocks per SM, tuned on B200
+__global__ void __launch_bounds__(kThreads, 3) k_visc_split(const __grid_constant__ Ctx c)
 {
     int lo[3], hi[3];
     ops::Visc::bounds(c.g, 0, lo, hi);
@@ -247,7 +247,7 @@ __device__ __forceinline__ int field_lb(int f, int d) { return field_half(f, d) 
 // and z in turn leaves every ghost point equal to the interior point it
 // wraps to, w(q) = q + n for q <= 0 and q - n for q >= n + 1 (a half-cell
 // index n keeps its value), so all ghosts are filled by one gather.
-__global__ void __launch_bounds__(kThreads) k_bc_periodic(Ctx c, FieldList fl)
+__global__ void __launch_bounds__(kThreads) k_bc_periodic(const __grid_constant__ Ctx c, FieldList fl)
 {
     const int f = fl.id[blockIdx.y];
     const Geom &g = c.g;
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(kThreads) k_bc_periodic(Ctx c, FieldList fl)
 
 // One (dimension, edge) of the given fields, exactly as the reference's
 // boundary-condition objects apply it (lare_bc.cuh).
-__global__ void __launch_bounds__(kThreads) k_bc_edge(Ctx c, FieldList fl, BcTable bt, int d, int e)
+__global__ void __launch_bounds__(kThreads) k_bc_edge(const __grid_constant__ Ctx c, FieldList fl, BcTable bt, int d, int e)
 {
     const int f = fl.id[blockIdx.y];
     const int kind = bt.kind[f][d][e];
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kThreads) k_bc_edge(Ctx c, FieldList fl, BcTab
 // All conditions of the given fields in one pass over each field's ghost
 // shell, where they compose (bc_composable): the six edge launches of a fill
 // with walls become one.
-__global__ void __launch_bounds__(kThreads) k_bc_compose(Ctx c, FieldList fl, BcTable bt)
+__global__ void __launch_bounds__(kThreads) k_bc_compose(const __grid_constant__ Ctx c, FieldList fl, BcTable bt)
 {
     const int f = fl.id[blockIdx.y];
     const BcShell sh(c.g, f);
@@ -901,8 +901,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     launch_cellnode<PrepMarch>(resistive);
     launch<ops::Alpha>(0);
     {
-        // Visc with two threads per cell (k_visc_split): 1.21 -> 1.12 ms at
-        // 256^3 against one thread per cell at 128 registers
+        // Visc with two threads per cell (k_visc_split)
         int lo[3], hi[3];
         ops::Visc::bounds(ctx_.g, 0, lo, hi);
         const long long plane = (long long)(hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
