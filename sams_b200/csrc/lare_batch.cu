@@ -968,16 +968,15 @@ void Batch::enqueue_step()
     if (!fold_) launch<ops::BScale>(C_REMAP, 0);
     launch_cellnode<march::VolMarch<0>>(C_X, fused_xy_ ? 1 : 0);
     launch_ctmass<0>(C_X, fold_ ? 1 : 0);
-    launch<ops::SweepCTUpd<0>>(C_X, fold_ ? 1 : 0);
-    stages<0>(C_X, 0, false);
+    stages<0>(C_X, fold_ ? 1 : 0);
     bc_fill(C_Y, FM_ALL9, false);
     launch_cellnode<march::VolMarch<1>>(C_Y, fused_xy_ ? 1 : 0);
     launch_ctmass<1>(C_Y, 0);
-    stages<1>(C_Y, 0, true);
+    stages<1>(C_Y, 0);
     bc_fill(C_REMAP, FM_ALL9, false);
     launch_cellnode<march::VolMarch<2>>(C_REMAP, 0);
     launch_ctmass<2>(C_REMAP, 0);
-    stages<2>(C_REMAP, fold_ ? 2 : 0, true);
+    stages<2>(C_REMAP, fold_ ? 2 : 0);
     bc_fill(C_REMAP, FM_ALL9, false);
     if (!fold_) {
         launch<ops::BScale>(C_REMAP, 1);
@@ -986,17 +985,16 @@ void Batch::enqueue_step()
     if (has_rke_) launch<ops::RkeEnergy>(C_REMAP, 0);
 }
 
-// S6-S8 of one sweep: fused, with the sweep's CT update (where `update` asks
-// for it) at the same points, or the separate kernels.
+// The CT update and S6-S8 of one sweep: one kernel, or the separate ones.
 template <int DIR>
-void Batch::stages(int ctx, int ct_arg, bool update)
+void Batch::stages(int ctx, int ct_arg)
 {
     if constexpr (DIR == 2) {
         if (zfuse_) return launch_zsweep(ctx, ct_arg);
     } else {
-        if (fused_xy_) return launch_psweep<DIR>(ctx, update ? ct_arg : -1);
+        if (fused_xy_) return launch_psweep<DIR>(ctx, ct_arg);
     }
-    if (update) launch<ops::SweepCTUpd<DIR>>(ctx, ct_arg);
+    launch<ops::SweepCTUpd<DIR>>(ctx, ct_arg);
     launch<ops::SweepS6<DIR>>(ctx, 0);
     launch<ops::SweepS7<DIR>>(ctx, 0);
     if (has_rke_) {  // solves without rke return at once (Phys::rke)

@@ -101,7 +101,7 @@ private:
     template <int DIR> void launch_ctmass(int ctx, int scale);
     template <int DIR> void launch_psweep(int ctx, int ct_arg);
     void launch_zsweep(int ctx, int ct_arg);
-    template <int DIR> void stages(int ctx, int ct_arg, bool update);
+    template <int DIR> void stages(int ctx, int ct_arg);
     void bc_fill(int ctx, unsigned mask, bool resistive_only);
     void bc_edges(int ctx, unsigned mask, int d, bool dm_only, bool resistive_only);
     void drop_graphs();

@@ -589,9 +589,8 @@ __device__ __forceinline__ void ctmass_z(const Ctx &c, const ZTile &z, int b, in
 // the transverse plane is (a, k) in 0..na x 0..nz.  The solve's state arrays
 // are only read; the new rho, energies and velocities go to w.  Halo points
 // recompute stage A (two before, one after) and stage B (one before) without
-// writing the state.  ct_arg >= 0: each own point (0..n in every dimension)
-// also takes the sweep's CT update of B (SweepCTUpd<DIR> with that
-// argument); no stage reads B.
+// writing the state.  Each own point (0..n in every dimension) also takes the
+// sweep's CT update of B (SweepCTUpd<DIR> with ct_arg); no stage reads B.
 template <int DIR, bool GEO>
 __device__ __forceinline__ void psweep(const Ctx &c, const WinTile &wt, int b, const ops::SweepOut &w, int ct_arg,
                                        double *psm)
@@ -633,16 +632,15 @@ __device__ __forceinline__ void psweep(const Ctx &c, const WinTile &wt, int b, c
     __syncthreads();
     for (int s = s0 + sl; s <= s1; s += TS)
         if (on) F::stage_c(c, DIR == 0 ? s : a, DIR == 0 ? a : s, k, at(s), w);
-    if (ct_arg >= 0)
-        for (int s = s0 + sl; s <= s1; s += TS)
-            if (on) ops::SweepCTUpd<DIR>::template run<GEO, false>(c, ct_arg, DIR == 0 ? s : a, DIR == 0 ? a : s, k);
+    for (int s = s0 + sl; s <= s1; s += TS)
+        if (on) ops::SweepCTUpd<DIR>::template run<GEO, false>(c, ct_arg, DIR == 0 ? s : a, DIR == 0 ? a : s, k);
 }
 
 // The z sweep's stages S6, S7 and S8 (ops::SweepFused<2>) over whole z
 // lines, in place: a block holds kZThreads / (nz + 4) lines of (i, j) in
-// 0..nx x 0..ny, one thread per k = -2..nz+1 of each.  ct_arg >= 0: each
-// point of 0..n also takes the z sweep's CT update of B (SweepCTUpd<2> with
-// that argument), which nothing else in the kernel reads or writes.
+// 0..nx x 0..ny, one thread per k = -2..nz+1 of each.  Each point of 0..n also
+// takes the z sweep's CT update of B (SweepCTUpd<2> with ct_arg), which
+// nothing else in the kernel reads or writes.
 constexpr int kZThreads = ops::kZLineThreads;
 template <bool GEO>
 __device__ __forceinline__ void zsweep(const Ctx &c, int b, int ct_arg, double *zsm)
@@ -666,13 +664,11 @@ __device__ __forceinline__ void zsweep(const Ctx &c, int b, int ct_arg, double *
         prefetch(c.f[SAMS_F_DM], o);
         prefetch(c.f[SAMS_F_ENERGY_ELECTRON], o);
         prefetch(c.f[SAMS_F_ENERGY_ION], o);
-        if (ct_arg >= 0) {
-            prefetch(c.f[SAMS_F_BX], o);
-            prefetch(c.f[SAMS_F_BY], o);
-            prefetch(c.f[SAMS_F_BZ], o);
-            prefetch(c.s[S_R_CT1], o);
-            prefetch(c.s[S_R_CT2], o);
-        }
+        prefetch(c.f[SAMS_F_BX], o);
+        prefetch(c.f[SAMS_F_BY], o);
+        prefetch(c.f[SAMS_F_BZ], o);
+        prefetch(c.s[S_R_CT1], o);
+        prefetch(c.s[S_R_CT2], o);
     }
     if (on) F::stage_a<GEO>(c, i, j, k, st, w, true);
     __syncthreads();
@@ -680,7 +676,7 @@ __device__ __forceinline__ void zsweep(const Ctx &c, int b, int ct_arg, double *
     if (on && k >= -1 && k <= g.nz) F::stage_b_mom<GEO>(c, i, j, k, st);  // its own slots: no barrier between
     __syncthreads();
     if (on && k >= 0 && k <= g.nz) F::stage_c(c, i, j, k, st, w);
-    if (ct_arg >= 0 && on && k >= 0 && k <= g.nz) ops::SweepCTUpd<2>::run<GEO, false>(c, ct_arg, i, j, k);
+    if (on && k >= 0 && k <= g.nz) ops::SweepCTUpd<2>::run<GEO, false>(c, ct_arg, i, j, k);
 }
 
 }  // namespace march

@@ -948,15 +948,13 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     launch_cellnode<VolMarch<0>>(fused_xy ? 1 : 0);
     const bool dm_x = launch_ctmass<0>(b_fill_all ? 1 : 0);
     // The CT update changes only B, which the dm fill and the stages S6-S8
-    // do not read, so the y and z sweeps' fused stages take it at their
-    // points 0..n (its whole range).  In the x sweep, with the B scaling
-    // folded in, it stays a kernel of its own: inside k_psweep it measured
-    // slower on B200 (14 us per step), in the y and z sweeps faster (13 and
-    // 40 us).
-    launch<ops::SweepCTUpd<0>>(b_fill_all ? 1 : 0);
+    // do not read, so the fused stages take it at their points 0..n (its
+    // whole range; with the B scaling folded in, the fill after the sweep
+    // writes B's ghosts from those points).
+    if (!fused_xy) launch<ops::SweepCTUpd<0>>(b_fill_all ? 1 : 0);
     if (!dm_x) bc_fill_dim(FM_DM, 0);
     if (fused_xy) {
-        launch_psweep<0>(-1);
+        launch_psweep<0>(b_fill_all ? 1 : 0);
     } else {
         launch<ops::SweepS6<0>>(0);
         launch<ops::SweepS7<0>>(0);
