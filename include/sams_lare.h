@@ -250,8 +250,9 @@ int sams_lare_serve_destroy(sams_lare_server *s);
  * sends each submitted solve to the least-loaded one: among the devices
  * whose budget can hold the solve, those where it fits next to what is
  * already admitted or queued come first, then the least outstanding work
- * (pending_cell_updates), then the fewest committed bytes, then the lowest
- * index.  A device may be listed more than once (two servers share it).
+ * (pending_cell_updates), then the fewest committed bytes, then the least
+ * work placed on it so far, then the lowest index.  A device may be listed
+ * more than once (two servers share it).
  * Tickets are the router's own; every call mirrors its sams_lare_serve_*
  * counterpart. */
 typedef struct sams_lare_router sams_lare_router;

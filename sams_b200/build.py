@@ -19,7 +19,7 @@ CU_SOURCES = ["lare_solver.cu", "lare_batch.cu", "lare_serve.cu", "lare_capi.cu"
               "lare_router.cu", "lare_dist.cu", "lare_fp64_roof.cu"]
 C_SOURCES = ["lare_ic.c"]
 HEADERS = ["lare_device.cuh", "lare_ops.cuh", "lare_march.cuh", "lare_bc.cuh", "lare_solver.cuh",
-           "lare_batch.cuh", "lare_dump.cuh", "lare_geom_host.h"]
+           "lare_batch.cuh", "lare_dump.cuh", "lare_geom_host.h", "lare_repack.cuh", "lare_div.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

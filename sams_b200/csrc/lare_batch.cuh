@@ -106,6 +106,7 @@ private:
     void bc_edges(int ctx, unsigned mask, int d, bool dm_only, bool resistive_only);
     void drop_graphs();
     void free_slot(BatchSlot &s);
+    unsigned repack_grid(const Geom &g) const;
 
     int device_ = 0;
     cudaStream_t own_stream_ = nullptr;

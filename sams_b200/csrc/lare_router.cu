@@ -35,6 +35,7 @@ double now_s()
 struct sams_lare_router {
     std::vector<sams_lare_server *> servers;
     std::vector<int64_t> budget;
+    std::vector<double> taken;  // cell-updates placed on each server since creation
     std::mutex mu;
     int64_t next_id = 1;
     std::map<int64_t, Placement> placed;
@@ -93,6 +94,7 @@ int sams_lare_router_create(const int *devices, int ndevices, int64_t budget_byt
         }
         r->servers.push_back(s);
         r->budget.push_back(budget_bytes_per_device);
+        r->taken.push_back(0.0);
     }
     *out = r;
     return SAMS_OK;
@@ -120,13 +122,28 @@ int sams_lare_router_submit(sams_lare_router *r, const sams_lare_params *p, cons
     int64_t bytes = 0;
     int rc = sams_lare_serve_solve_bytes(p, &bytes);
     if (rc != SAMS_OK) return rc;
+    // Servers alike in load and bytes (idle ones, when solves finish faster
+    // than they come) tie, and the rule takes the first: list them by the work
+    // placed on them so far, so that such a stream spreads too.
+    std::vector<int> order(n);
+    for (int q = 0; q < n; ++q) order[q] = q;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return r->taken[a] < r->taken[b]; });
+    std::vector<double> pend(n);
+    std::vector<int64_t> comm(n), bud(n);
+    for (int q = 0; q < n; ++q) {
+        pend[q] = pending[order[q]];
+        comm[q] = committed[order[q]];
+        bud[q] = r->budget[order[q]];
+    }
     int pick = -1;
-    rc = sams_lare_route_pick(n, pending.data(), committed.data(), r->budget.data(), bytes, &pick);
+    rc = sams_lare_route_pick(n, pend.data(), comm.data(), bud.data(), bytes, &pick);
     if (rc != SAMS_OK) return rc;
+    pick = order[pick];
     Placement pl;
     pl.server = pick;
     rc = sams_lare_serve_submit(r->servers[pick], p, bcs, ic, nsteps, out, &pl.ticket);
     if (rc != SAMS_OK) return rc;
+    r->taken[pick] += (double)p->nx * (double)p->ny * (double)p->nz * (double)nsteps;
     *ticket = r->next_id++;
     r->placed.emplace(*ticket, pl);
     return SAMS_OK;

@@ -29,6 +29,7 @@
 #include "lare_march.cuh"
 #include "lare_bc.cuh"
 #include "lare_geom_host.h"
+#include "lare_repack.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -189,22 +190,6 @@ __global__ void __launch_bounds__(kThreads, 3) k_visc_split(const __grid_constan
         double m = wmin[0];
         for (int w = 1; w < kThreads / 32; ++w) m = dev::pmin(m, wmin[w]);
         if (m < DBL_MAX) atomicMin(&c.sc->dtmin_bits, (unsigned long long)__double_as_longlong(m));
-    }
-}
-
-// Dense box buffer <-> padded device rows (to_padded = 1: dense -> padded).
-__global__ void k_repack(const double *__restrict__ src, double *__restrict__ dst, Geom g, int to_padded)
-{
-    const long long n = (long long)(g.nx + 5) * (g.ny + 5) * (g.nz + 5);
-    const int ez = g.nz + 5;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (long long)gridDim.x * blockDim.x) {
-        const long long row = t / ez;
-        const long long p = row * g.sy + (g.zoff - 2) + (t - row * ez);
-        if (to_padded)
-            dst[p] = src[t];
-        else
-            dst[t] = src[p];
     }
 }
 
