@@ -29,39 +29,6 @@ constexpr int kFillPoints = kT;  // shell points per entry of the fill's block l
 // single solve), and those fields.
 __constant__ const int kSweepOut[6] = {S_FX, S_FY, S_FZ, S_VH, S_FXV, S_FYV};
 
-// Points of the shell that kb_bc_fill walks, and point t of it.
-__host__ __device__ inline int fill_points(const Geom &g)
-{
-    return 6 * (g.ny + 5) * (g.nz + 5) + (g.nx - 1) * 6 * (g.nz + 5) + (g.nx - 1) * (g.ny - 1) * 6;
-}
-__device__ __forceinline__ int shell_index(int n, int t) { return t < 3 ? t - 2 : n + t - 3; }  // -2, -1, 0, n .. n+2
-__device__ __forceinline__ bool fill_point(const Geom &g, int t, int &q0, int &q1, int &q2)
-{
-    const int E1 = g.ny + 5, E2 = g.nz + 5;
-    const int A = 6 * E1 * E2, B = (g.nx - 1) * 6 * E2, C = (g.nx - 1) * (g.ny - 1) * 6;
-    if (t < A) {
-        const int x = t / (E1 * E2), r = t - x * (E1 * E2), y = r / E2;
-        q0 = shell_index(g.nx, x);
-        q1 = y - 2;
-        q2 = r - y * E2 - 2;
-        return true;
-    }
-    if ((t -= A) < B) {
-        const int i = t / (6 * E2), r = t - i * (6 * E2), y = r / E2;
-        q0 = 1 + i;
-        q1 = shell_index(g.ny, y);
-        q2 = r - y * E2 - 2;
-        return true;
-    }
-    if ((t -= B) < C) {
-        const int i = t / ((g.ny - 1) * 6), r = t - i * ((g.ny - 1) * 6), j = r / 6;
-        q0 = 1 + i;
-        q1 = 1 + j;
-        q2 = shell_index(g.nz, r - j * 6);
-        return true;
-    }
-    return false;
-}
 // Whether field f's own range holds the point and has it as a ghost.
 __device__ __forceinline__ bool field_ghost(const Geom &g, int f, int q0, int q1, int q2)
 {
@@ -310,7 +277,8 @@ __device__ __forceinline__ int locate(const long long *off, int n, long long g)
 // ghost shell: its whole box -2..n+2 outside 1..n (1..n-1: the half-cell
 // fields' index n is a ghost too), x slabs, then y slabs inside x, then z
 // slabs inside x and y.  A point is decomposed once and then written for every
-// field in whose own range it is a ghost.
+// field in whose own range it is a ghost, one field after another (all loads
+// first, as periodic_copy has them, was 3% slower here).
 __global__ void __launch_bounds__(kT) kb_bc_fill(const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st,
                                                  const BcTable *__restrict__ bcs, const BlockRef *__restrict__ blocks, int n,
                                                  unsigned mask, int resistive_only)

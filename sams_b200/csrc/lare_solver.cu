@@ -226,57 +226,12 @@ struct FieldList {
     int id[SAMS_NFIELDS];
 };
 
-__device__ __forceinline__ int field_lb(int f, int d) { return field_half(f, d) ? -2 : -1; }
-
-// All-periodic fields: applying the lower then upper periodic copy in x, y
-// and z in turn leaves every ghost point equal to the interior point it
-// wraps to, w(q) = q + n for q <= 0 and q - n for q >= n + 1 (a half-cell
-// index n keeps its value), so all ghosts are filled by one gather.
-__global__ void __launch_bounds__(kThreads) k_bc_periodic(const __grid_constant__ Ctx c, FieldList fl)
+// All-periodic fields, one thread per point of the shell (periodic_copy).
+template <unsigned MASK>
+__global__ void __launch_bounds__(kThreads) k_bc_periodic(const __grid_constant__ Ctx c)
 {
-    const int f = fl.id[blockIdx.y];
-    const Geom &g = c.g;
-    const int n[3] = {g.nx, g.ny, g.nz};
-    int lb[3], ext[3], gh[3];
-    for (int d = 0; d < 3; ++d) {
-        lb[d] = field_lb(f, d);
-        ext[d] = n[d] + 3 - lb[d];
-        gh[d] = ext[d] - n[d];
-    }
-    // 32-bit index arithmetic: a field's shell has fewer points than the
-    // field, and a field has fewer than 2^31 (checked at set-up)
-    const int A = gh[0] * ext[1] * ext[2];
-    const int B = n[0] * gh[1] * ext[2];
-    const int C = n[0] * n[1] * gh[2];
-    int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    int q[3];
-    if (t < A) {
-        const int pl = ext[1] * ext[2];
-        const int gi = t / pl, r = t - gi * pl;
-        q[0] = gi < 1 - lb[0] ? lb[0] + gi : n[0] + 1 + (gi - (1 - lb[0]));
-        q[1] = lb[1] + r / ext[2];
-        q[2] = lb[2] + r % ext[2];
-    } else if ((t -= A) < B) {
-        const int pl = gh[1] * ext[2];
-        const int i = t / pl, r = t - i * pl;
-        const int gj = r / ext[2];
-        q[0] = 1 + i;
-        q[1] = gj < 1 - lb[1] ? lb[1] + gj : n[1] + 1 + (gj - (1 - lb[1]));
-        q[2] = lb[2] + (r - gj * ext[2]);
-    } else if ((t -= B) < C) {
-        const int pl = n[1] * gh[2];
-        const int i = t / pl, r = t - i * pl;
-        const int gk = r % gh[2];
-        q[0] = 1 + i;
-        q[1] = 1 + r / gh[2];
-        q[2] = gk < 1 - lb[2] ? lb[2] + gk : n[2] + 1 + (gk - (1 - lb[2]));
-    } else {
-        return;
-    }
-    int s[3];
-    for (int d = 0; d < 3; ++d) s[d] = q[d] <= 0 ? q[d] + n[d] : (q[d] >= n[d] + 1 ? q[d] - n[d] : q[d]);
-    double *a = c.f[f];
-    a[box_off(g, q[0], q[1], q[2])] = a[box_off(g, s[0], s[1], s[2])];
+    int q0, q1, q2;
+    if (fill_point(c.g, (int)(blockIdx.x * blockDim.x + threadIdx.x), q0, q1, q2)) periodic_copy<MASK>(c, q0, q1, q2);
 }
 
 // One (dimension, edge) of the given fields, exactly as the reference's
@@ -816,8 +771,10 @@ bool Solver::all_periodic(unsigned mask) const
     return true;
 }
 
-void Solver::bc_fill(unsigned mask)
+template <unsigned MASK>
+void Solver::bc_fill()
 {
+    constexpr unsigned mask = MASK;
     FieldList fl = make_list(mask);
     if (fl.n == 0) return;
     if (halo_) {  // a slab: x by exchange, then y and z in the same order as below
@@ -829,13 +786,9 @@ void Solver::bc_fill(unsigned mask)
     const Geom &g = ctx_.g;
     // the one-pass gather needs every source inside the domain (n >= 3)
     if (all_periodic(mask) && std::min(g.nx, std::min(g.ny, g.nz)) >= kBcSequentialBelow) {
-        // the largest ghost shell is the all-half-cell one
-        const long long e0 = g.nx + 5, e1 = g.ny + 5, e2 = g.nz + 5;
-        const long long cnt = 5 * e1 * e2 + (long long)g.nx * 5 * e2 + (long long)g.nx * g.ny * 5;
-        dim3 grid((unsigned)ceil_div(cnt, kThreads), (unsigned)fl.n);
-        k_bc_periodic<<<grid, kThreads, 0, stream_>>>(ctx_, fl);
+        const unsigned blocks = (unsigned)ceil_div(fill_points(g), kThreads);
+        k_bc_periodic<MASK><<<blocks, kThreads, 0, stream_>>>(ctx_);
         ++launches_;
-        (void)e0;
         return;
     }
     const int n[3] = {g.nx, g.ny, g.nz};
@@ -906,11 +859,11 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     if (resistive) {
         for (int sub = 0; sub < 2; ++sub) {
             launch_resist(sub == 1);
-            bc_fill(FM_BFIELD | FM_ENERGY);
+            bc_fill<FM_BFIELD | FM_ENERGY>();
         }
     }
     launch_pred(resistive);
-    bc_fill(FM_REMAPV);
+    bc_fill<FM_REMAPV>();
     mark(1);
     // ---- corrector ----
     // (Corr1 and Corr2 as one pass, with the velocities written out of place,
@@ -918,7 +871,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     // Corr1's 2 when fused.)
     launch_heat();
     launch<ops::Corr2>(0);
-    bc_fill(FM_VELOCITY | FM_ENERGY | FM_DENSITY);
+    bc_fill<FM_VELOCITY | FM_ENERGY | FM_DENSITY>();
     mark(2);
     // ---- remap ----
     // B to and from flux form (BScale) folded into the x and z sweeps' CT
@@ -949,7 +902,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
         }
         launch<ops::SweepS8<0>>(0);
     }
-    bc_fill(FM_ALL9);
+    bc_fill<FM_ALL9>();
     mark(3);
     launch_cellnode<VolMarch<1>>(fused_xy ? 1 : 0);
     const bool dm_y = launch_ctmass<1>(0);
@@ -966,7 +919,7 @@ void Solver::enqueue_step(cudaEvent_t *marks)
         }
         launch<ops::SweepS8<1>>(0);
     }
-    bc_fill(FM_ALL9);
+    bc_fill<FM_ALL9>();
     mark(4);
     launch_cellnode<VolMarch<2>>(0);
     const bool dm_z = launch_ctmass<2>(0);
@@ -997,10 +950,10 @@ void Solver::enqueue_step(cudaEvent_t *marks)
     // with the B scaling folded into the z sweep's CT update, B needs no pass
     // of its own before the fill, so all nine fields take one fill (the fill
     // of each field is independent of the others')
-    bc_fill(FM_ALL9);
+    bc_fill<FM_ALL9>();
     if (!b_fill_all) {
         launch<ops::BScale>(1);
-        bc_fill(FM_BFIELD);
+        bc_fill<FM_BFIELD>();
     }
     if (p_.rke) launch<ops::RkeEnergy>(0);  // after the remap (shared_data.h:414-417)
     mark(5);

@@ -105,7 +105,7 @@ public:
 
 private:
     int check(cudaError_t e, const char *what);
-    void bc_fill(unsigned mask);
+    template <unsigned MASK> void bc_fill();
     void bc_fill_dim(unsigned mask, int dim);
     bool all_periodic(unsigned mask) const;
     bool ghosts_refilled(unsigned mask) const;
