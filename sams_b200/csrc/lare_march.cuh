@@ -122,7 +122,6 @@ struct RingSrc {
 // The predictor's ring: Pred1's outputs with p_e + p_i in the PE slot (Pred2
 // reads only that sum), five arrays.
 struct PredRingSrc {
-    static constexpr bool kPressureSum = true;
     static constexpr int NR = ops::Pred1::PI;  // CV1, B1X, B1Y, B1Z, PE (= p_e + p_i)
     const double *ring;
     __device__ double operator()(int arr, int q) const { return ring[arr * 3 * kRP + q]; }

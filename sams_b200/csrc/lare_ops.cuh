@@ -1,10 +1,10 @@
-// lare_ops.cuh -- the fused phases of one LARE3D timestep as per-point
-// device operations.  Each Op has
+// lare_ops.cuh -- the phases of one LARE3D timestep as device operations on one
+// point.  Those that a launcher runs by themselves have
 //   bounds(g, arg, lo, hi)   the index box the phase covers, and
 //   run(c, arg, i, j, k)     the work of one (i, j, k) of that box,
-// so the same code runs under the single-solve launcher (one grid per
-// phase) and the batched launcher (one grid over a worklist of tiles from
-// many solves).
+// so the same code runs under the single-solve launcher (one grid per phase)
+// and the batched launcher (one grid over a worklist of tiles from many
+// solves); the others are parts of the fused kernels (lare_march.cuh).
 //
 // Fusion plan (reference kernels each op replaces in brackets):
 //   CellPrep   cs                                  [lagran.cpp:113-125, 192-198]
@@ -12,17 +12,17 @@
 //   Alpha      alpha1..3                           [lagran.cpp:218-279]
 //   Visc       visc_heat, f*_visc, CFL candidate   [lagran.cpp:284-376, 388-439]
 //   ResistRK   eta (on the fly), edge E, curlb     [lagran.cpp:449-474, 511-533]
-//   ResistB    B update, Ohmic heating, b1 copy    [lagran.cpp:482-499, 541-587]
+//   ResistB    B update, Ohmic heating             [lagran.cpp:482-499, 541-587]
 //   Pred1      cv1, half-step B*cv1, p_e/p_i       [lagran.cpp:598-614, 810-880]
 //   Pred2      forces, v1                          [lagran.cpp:619-733]
 //   Corr1      shock heating                       [lagran.cpp:888-992]
 //   Corr2      velocity, energies, density         [lagran.cpp:754-798]
-//   BScale / BUnscale  B <-> flux form             [remap.cpp:46-50, 91-95]
+//   BScale     B <-> flux form                     [remap.cpp:46-50, 91-95]
 //   SweepVol   cv1, cv2, db1, rho1, dm = 0         [xremap.cpp:24-70 + y/z]
 //   SweepCvc   cvc1                                [xremap.cpp:74-81]
-//   SweepCT    both CT fluxes                      [xremap.cpp:269-371]
+//   SweepCTMass both CT fluxes, dm                 [xremap.cpp:269-422]
 //   SweepCTUpd both CT updates                     [xremap.cpp:87-115]
-//   SweepMass  dm                                  [xremap.cpp:373-422]
+//   SweepFused S6-S8 as stages of one kernel; separately (rke):
 //   SweepS6    rho, energy fluxes, vertex rho_v,   [xremap.cpp:121-221]
 //              cv2 (node), dm (node), v1 shift
 //   SweepS7    energy updates, momentum fluxes*dm  [xremap.cpp:130-152, 485-566]
@@ -104,38 +104,12 @@ __host__ __device__ inline void set_bounds(int *lo, int *hi, int a0, int b0, int
 // Lagrangian phase
 // ---------------------------------------------------------------------------
 
-// Per-point outputs of one op as another op reads them from global memory:
-// src(arr, q) is array arr at offset q.  (The fused kernels read the same
-// values from a shared-memory ring instead.)
-struct ArraySrc {
-    static constexpr bool kPressureSum = false;  // p_e and p_i are separate arrays (see Pred2)
-    const double *a[6];
-    __device__ double operator()(int arr, int q) const { return __ldg(a[arr] + q); }
-};
-
 // Sound speed on cells; with resistive MHD also keeps p_e and p_i, which the
 // predictor reads as they were at the start of the step (lagran.cpp:121-123,
 // 606-607): between the two, the resistive sub-steps heat the electrons and
 // refill the energies' ghost cells (energy_bcs), so recomputing them there
 // would differ wherever a ghost was not already its boundary value.
 struct CellPrep {
-    static constexpr int kMinBlocks = 6;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int resistive, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const int o = LOFF(i, j, k);
-        double rho, pe, pi;
-        c.s[S_CS][o] = sound_speed(c, o, rho, pe, pi);
-        if (resistive) {
-            c.s[S_PE][o] = pe;
-            c.s[S_PI][o] = pi;
-        }
-    }
     // cs of the cell at offset o, with its rho, p_e and p_i
     __device__ static double sound_speed(const Ctx &c, int o, double &rho, double &pe, double &pi)
     {
@@ -157,18 +131,6 @@ struct CellPrep {
 
 // Node density and sound speed (8-cell volume-weighted averages).
 struct NodePrep {
-    static constexpr int kMinBlocks = 4;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 1, -1, g.ny + 1, -1, g.nz + 1);
-    }
-    template <bool GEO, bool P2>
-    __device__ static void run(const Ctx &c, int, int i, int j, int k)
-    {
-        const Geom &g = c.g;
-        const ArraySrc src{{c.f[SAMS_F_RHO], c.s[S_CS]}};
-        run_src<GEO, P2>(c, i, j, k, src, LOFF(i, j, k), g.sx, g.sy, 1);
-    }
     // rho (array 0) and cs (array 1) of the node's eight cells read through
     // src(array, q), q = q0 + dx*QX + dy*QY + dz*QZ (dx, dy, dz in {0, 1})
     template <bool GEO, bool P2, class S>
@@ -480,11 +442,7 @@ struct Visc {
 // evaluated at the same point from the same B, so computed once), edge
 // electric fields and Ohmic heating rate.
 struct ResistRK {
-    static constexpr int kMinBlocks = 6;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, 0, g.nx, 0, g.ny, 0, g.nz);
-    }
+    // (on 0..n in every dimension)
     // outputs: the three edge fluxes and the Ohmic heating rate
     enum { FX, FY, FZ, CURLB, NOUT };
     template <bool GEO, bool P2>
@@ -537,11 +495,6 @@ struct ResistRK {
 // heating; on the last sub-step also keeps the pre-update face B as b1,
 // which the predictor reads (resistive_effects' copy, lagran.cpp:482-484).
 struct ResistB {
-    static constexpr int kMinBlocks = 6;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
-    }
     // The update at (i, j, k) with the fluxes of ResistRK read through
     // src(array, q) for the cell q = q0 - dx*QX - dy*QY - dz*QZ (dx, dy, dz in
     // {0, 1}); the new B goes to nbx/nby/nbz[o] (unchanged values included),
@@ -618,11 +571,6 @@ struct ResistB {
 // Predictor, part 1: half-step cell volume and B (then scaled by cv1), and
 // the half-step pressures (lagran.cpp:598-614, 806-882).
 struct Pred1 {
-    static constexpr int kMinBlocks = 4;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
-    }
     // Outputs of one cell (0..n+1 in every dimension), in this order: cv1,
     // b1x*cv1, b1y*cv1, b1z*cv1 and the half-step p_e, p_i.  Reads the step-start p_e/p_i of resistive runs
     // from S_PE/S_PI.
@@ -731,11 +679,7 @@ struct Pred1 {
 // Predictor, part 2: pressure and J x B forces on nodes and the half-step
 // velocity (lagran.cpp:619-733, Cartesian).
 struct Pred2 {
-    static constexpr int kMinBlocks = 4;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, 0, g.nx, 0, g.ny, 0, g.nz);
-    }
+    // (nodes 0..n)
     // The node's update with Pred1's outputs read through src(array, q) for
     // the cell q = q0 + dx*QX + dy*QY + dz*QZ (dx, dy, dz in {0, 1}).
     template <bool GEO, bool P2, class S>
@@ -764,10 +708,10 @@ struct Pred2 {
             int a;
             __device__ double operator[](int q) const { return s(a, q); }
         };
-        const Arr pe{src, Pred1::PE}, pi{src, Pred1::PI}, cv1{src, Pred1::CV1};
-        // p_e + p_i of cell q: a source with kPressureSum holds that sum (the
-        // same addition, made where the values were produced) under PE
-        auto ptot = [&](int q) { return S::kPressureSum ? pe[q] : pe[q] + pi[q]; };
+        const Arr pe{src, Pred1::PE}, cv1{src, Pred1::CV1};
+        // the source holds p_e + p_i under PE (the same addition, made where the
+        // values were produced)
+        auto ptot = [&](int q) { return pe[q]; };
         const Arr bx1{src, Pred1::B1X}, by1{src, Pred1::B1Y}, bz1{src, Pred1::B1Z};
         const double dx = c.ax.dxc[i + 2], dy = c.ax.dyc[j + 2], dz = c.ax.dzc[k + 2];
         // metric factors (lagran.cpp:627-630; all 1.0 in Cartesian geometry)
@@ -890,11 +834,6 @@ struct Pred2 {
 // Corrector, part 1: shock heating with the half-step velocities
 // (lagran.cpp:884-993, including its dy*dy factors at :987).
 struct Corr1 {
-    static constexpr int kMinBlocks = 2;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, 0, g.nx + 1, 0, g.ny + 1, 0, g.nz + 1);
-    }
     // Product of the velocity jumps at the start of the step and of the
     // half step along an edge.  Swapping a and b negates both factors, which
     // gives the same product up to the sign of a zero; a cell's heating is
@@ -1081,11 +1020,7 @@ __device__ __forceinline__ int dir_stride(const Geom &g, int dir)
 // adding zero does not change the sum.
 template <int DIR>
 struct SweepVol {
-    static constexpr int kMinBlocks = 6;  // blocks of 256 per SM (register cap), tuned on B200
-    __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
-    {
-        set_bounds(lo, hi, -1, g.nx + 2, -1, g.ny + 2, -1, g.nz + 2);
-    }
+    // (cells -1..n+2)
     // cv1 of the cell (i, j, k); its outputs are stored where `store`
     template <bool GEO, bool P2>
     __device__ __forceinline__ static double compute(const Ctx &c, int arg, int i, int j, int k, bool store)
@@ -1403,14 +1338,6 @@ struct SweepCTMass {
         return swept_flux(dv, face(up, dv.fraction(fabs(o_v), dv.of(bu)), bu), o_v, rho[o - d], rho[o], rho[o + d], rho[o + 2 * d]);
     }
 };
-
-// Range lo/hi of index q in dimension DIM for a sweep-direction-dependent
-// interval: [alo, ahi] along the sweep, [blo, bhi] across it.
-template <int DIR, int DIM>
-__device__ __forceinline__ bool in_sweep_range(int q, int n, int alo, int ahi_off, int blo, int bhi_off)
-{
-    return DIM == DIR ? (q >= alo && q <= n + ahi_off) : (q >= blo && q <= n + bhi_off);
-}
 
 // The face through which a sweep carries both specific energies, and the one
 // of the three momenta, where cv1 and cvc1 change roles.
@@ -1941,15 +1868,6 @@ struct RkeEnergy {
 
 #undef LOFF
 
-// Register cap (blocks of 256 per SM) of an op's power-of-two instantiation:
-// multiplying by reciprocals instead of calling the division routine lets
-// the compiler keep more values live, so these caps were tuned separately
-// on B200 (the same sweep as kMinBlocks, on the 256^3 step).
-template <class Op>
-struct CapP2 {
-    static constexpr int value = Op::kMinBlocks;
-};
-
 // Register cap of an op in the batched engine (lare_batch.cu), whose solves
 // are typically thin (n x n x 4): rows of nine doubles, tiles of eight
 // planes.  Swept on B200 like kMinBlocks, on the batched step of 64
@@ -1959,21 +1877,17 @@ struct CapBatch {
     static constexpr int value = Op::kMinBlocks;
 };
 template <> struct CapBatch<BScale> { static constexpr int value = 8; };
-template <> struct CapBatch<Corr2> { static constexpr int value = 5; };
 template <int D> struct CapBatch<SweepCTUpd<D>> { static constexpr int value = 8; };
 template <int D> struct CapBatch<SweepS7<D>> { static constexpr int value = 4; };
 template <int D> struct CapBatch<SweepS8<D>> { static constexpr int value = 8; };
 
 }  // namespace ops
 
-// Blocks-per-SM bound of a kernel running Op.
-template <class Op, bool P2>
-struct MinBlocks {
-    static constexpr int value = P2 ? ops::CapP2<Op>::value : Op::kMinBlocks;
-};
+// Blocks-per-SM bound of a batched kernel running Op (on power-of-two grids
+// the single solve's).
 template <class Op, bool P2>
 struct MinBlocksBatch {
-    static constexpr int value = P2 ? ops::CapP2<Op>::value : ops::CapBatch<Op>::value;
+    static constexpr int value = P2 ? Op::kMinBlocks : ops::CapBatch<Op>::value;
 };
 
 }  // namespace sams

@@ -6,10 +6,9 @@
 //   1. admit queued requests in arrival order while their device footprint
 //      fits the budget and, when a cap is set, the interior cells of the
 //      running solves stay under it (allocate, upload the initial state);
-//   2. advance every running solve by one step: solves whose step runs the
-//      single-solve path's fused kernels (Solver::fused_path: z lines long
-//      enough to fill their tiles) each launch their own step graph on their
-//      own stream, and all other solves advance together by one batched
+//   2. advance every running solve by one step: solves with long z lines
+//      (Solver::fused_path) each launch their own step graph on their own
+//      stream, and all other solves advance together by one batched
 //      step (one graph launch; re-recorded when that set changes), on one
 //      more stream, so the steps of all running solves overlap on the GPU;
 //   3. retire solves that reached their step count: copy the state to the
@@ -52,7 +51,7 @@ struct Request {
     int64_t done = 0;
     long long cells = 0;
     int slot = -1;                          // batch slot (batched solves)
-    std::unique_ptr<sams::Solver> solo;     // own solver (fused-path solves)
+    std::unique_ptr<sams::Solver> solo;     // own solver (Solver::fused_path)
     bool fused = false;
     int status = SAMS_SERVE_QUEUED;
     bool cancel = false;  // set by sams_lare_serve_cancel while running
@@ -224,7 +223,7 @@ void sams_lare_server::loop()
             admit_locked();
         }
         if (running.empty()) continue;
-        // one step for every running solve: each fused-path solve launches
+        // one step for every running solve: each with its own solver launches
         // its own step graph on its own stream, the others one batched step
         std::vector<Request *> lost;  // solves whose step could not run
         bool any_batched = false;

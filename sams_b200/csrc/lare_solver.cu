@@ -1,28 +1,29 @@
 // lare_solver.cu -- kernels and step orchestration of one LARE3D solve.
 //
 // One step on the device, in launch order (reference events in brackets;
-// the standard path: Cartesian or curvilinear, no rke, every dimension at
-// least three cells, every B edge with a condition):
+// bodies of the fused kernels in lare_march.cuh):
 //   [startOfTimestep -> lagrangian_step, lagran.cpp:95-173]
 //     k_cellnode_march (CellPrep + NodePrep), Alpha, k_visc_split (Visc +
-//     CFL block minima), DtFinalize, resistive only: 2 x {k_resist_march (ResistRK +
-//     ResistB), fill B + energies}, k_pred_march (Pred1 + Pred2), fill v1
+//     CFL block minima), k_dt_finalize, resistive only: 2 x {k_resist_march
+//     (ResistRK + ResistB), fill B + energies}, k_pred_march (Pred1 + Pred2),
+//     fill v1
 //   [halfTimestep -> corrector_step, lagran.cpp:739-804]
-//     k_edge_march (Corr1 from per-node edge terms), Corr2, fill v +
+//     k_heat_march (Corr1 from per-node edge terms), Corr2, fill v +
 //     energies + rho
 //   [endOfTimestep -> eulerian_remap, remap.cpp:23-111]
-//     x: k_cellnode_march (SweepVol + SweepCvc), k_ctmass (SweepCT +
-//        SweepMass), SweepCTUpd (with B to flux form, BScale), fill dm along
-//        x, k_psweep (S6-S8 out of place), fill the nine state fields
-//     y: k_cellnode_march, k_ctmass, fill dm along y, k_psweep (S6-S8 out
-//        of place, with SweepCTUpd), fill the nine state fields
-//     z: k_cellnode_march (SweepVol + SweepCvc), k_ctmass_z, fill dm along
-//        z, k_zsweep (S6-S8 in place, with SweepCTUpd bringing B back from
-//        flux form), fill the nine state fields
-// Other solves take the separate kernels (CellPrep, NodePrep, Corr1,
-// SweepVol, SweepCvc, BScale, SweepS6/S7/S8, the rke kernels, k_copy_shell) where a
-// condition above fails (thin grids, rke, a field edge without a condition).
-// The runner's step++/time += dt (runner.h:573-574) happens in DtFinalize.
+//     x: k_cellnode_march (SweepVol + SweepCvc), k_ctmass (CT and mass
+//        fluxes, dm's ghosts along x), k_psweep (S6-S8 out of place, with
+//        SweepCTUpd bringing B to flux form), fill the nine state fields
+//     y: the same along y
+//     z: k_cellnode_march, k_ctmass_z, k_zsweep (S6-S8 in place, with
+//        SweepCTUpd bringing B back from flux form), fill
+// A fill is one launch (k_bc_periodic, k_bc_compose) unless conditions do not
+// compose (k_bc_edge, one launch per dimension and edge).  With rke the
+// sweeps' stages are separate kernels (SweepS6/S7/S8, the rke kernels); with
+// a B edge that has no condition, or fewer than three cells somewhere, B is
+// scaled by passes of its own (BScale) and k_copy_shell completes the
+// out-of-place arrays.
+// The runner's step++/time += dt (runner.h:573-574) happens in k_dt_finalize.
 // Nothing is read back to the host inside a step.
 #include "lare_solver.cuh"
 #include "lare_ops.cuh"
@@ -45,7 +46,7 @@ constexpr int kThreads = 256;
 // geometry is curvilinear (its metric factors are applied); the Cartesian
 // instantiation has no trace of them.
 template <class Op, bool GEO, bool P2>
-__global__ void __launch_bounds__(kThreads, (MinBlocks<Op, P2>::value)) k_op(const __grid_constant__ Ctx c, int arg)
+__global__ void __launch_bounds__(kThreads, Op::kMinBlocks) k_op(const __grid_constant__ Ctx c, int arg)
 {
     int lo[3], hi[3];
     Op::bounds(c.g, arg, lo, hi);
@@ -279,7 +280,7 @@ FieldList make_list(unsigned mask)
 long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
 // Whether n values split into tiles of w lanes keep at least three quarters
-// of the lanes busy (thin grids, e.g. n x n x 4 solves, leave most idle).
+// of the lanes busy.
 bool lanes_full(long long n, long long w) { return 4 * n >= 3 * w * ceil_div(n, w); }
 
 }  // namespace

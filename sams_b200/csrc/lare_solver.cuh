@@ -59,8 +59,9 @@ public:
     // arrays, the host-transfer staging buffer, axes and metric tables (an
     // upper bound, for admission under a memory budget).
     static long long bytes_for(const sams_lare_params &p);
-    // Whether the step of a solve of these parameters runs the fused
-    // marching and windowed kernels (its z lines fill their tiles).
+    // Whether a server runs a solve of these parameters on a stream of its
+    // own (long z lines: large enough to fill much of the GPU) instead of in
+    // the batched step.
     static bool fused_path(const sams_lare_params &p);
     // One x slab of a larger grid: p.nx is the slab's own cell count, the
     // x axis and metric tables are those of the whole grid (slab.nx_global
