@@ -204,8 +204,7 @@ struct RO {
 // non-negative numerators and fraction() x / d, x not negative, where a result below 2^-600,
 // added to or taken from one or two, may be anything below that.
 //
-// With IEEE divisions throughout, each a branch to its slow path that loads
-// do not move past, against now (us, 256^3 power-of-two grid / 96^3):
+// With IEEE divisions throughout, against now (us, 256^3 power-of-two grid / 96^3):
 // predictor 1451 / 154 -> 1233 / 129, x stages 1239 / 85 -> 1051 / 71, y stages
 // 1367 / 93 -> 1198 / 81, z stages 1367 / 116 -> 1257 / 86, edge viscosity
 // 866 / 52 -> 767 / 48, corrector 597 / 38 -> 540 / 32; k_visc_split

@@ -1,21 +1,24 @@
 // lare_div.cuh -- correctly rounded division without branches, for several
 // numerators over one denominator.
 //
-// The remap and the predictor divide several numerators by the same volume,
-// and every IEEE division costs about 14 fused multiply-adds of FP64 pipe
-// time, eight more instructions and a branch to its slow path, which also
-// keeps the compiler from moving loads up past it.  The forms here are
-// straight-line and give the same bits:
-//   rcp_fast   r = RN(1/d): the hardware's 20-bit seed, one third-order and
-//              one second-order Newton step.  A second-order step from an
-//              r within one ulp rounds correctly unless d's significand is all
-//              ones (Markstein).
+// The remap and the predictor divide several numerators by the same volume or
+// density.  The forms here share the reciprocal, are straight-line and give
+// the same bits:
+//   rcp_fast   r = RN(1/d): three Newton-Raphson steps r + r*(1 - d*r), each
+//              with the two FMAs of the cited chapters, from a seed with
+//              relative error e.  A step squares the error and rounds, so two
+//              of them leave e^4 and half an ulp: within one ulp for e up to
+//              2^-14 (e^4 = 2^-56 is an eighth of an ulp at most).  The PTX
+//              manual gives the seed 20 bits.  The third step, from an r within
+//              one ulp, rounds correctly unless d's significand is all ones
+//              (Markstein).
 //   quot       q = RN(x/d) from r = RN(1/d) by Markstein's theorem (P.
 //              Markstein, "Computation of elementary functions on the IBM
 //              RISC System/6000 processor", 1990; Muller et al., "Handbook of
-//              Floating-Point Arithmetic"): if q is a faithful rounding of
-//              x/d and rem = x - d*q is formed exactly by an FMA, then
-//              RN(q + rem*r) = RN(x/d).  q = RN(x*r + RN(x*e)) with
+//              Floating-Point Arithmetic", the chapter on division by
+//              Newton-Raphson iteration with an FMA): if q is a faithful
+//              rounding of x/d and rem = x - d*q is formed exactly by an FMA,
+//              then RN(q + rem*r) = RN(x/d).  q = RN(x*r + RN(x*e)) with
 //              e = RN(r * (1 - d*r)), the part of 1/d that r misses, is within
 //              half an ulp and 2^-50 of one.
 // Conditions: d plain (plain_divisor: positive, exponent in -120..119, not
@@ -59,7 +62,8 @@ __host__ __device__ __forceinline__ unsigned low_word(double x)
     return (unsigned)u;
 #endif
 }
-// 1/d to 20 bits or more.
+// 1/d to about 20 bits (the PTX manual's figure for rcp.approx.ftz.f64, whose
+// result has a zero low word).
 __host__ __device__ __forceinline__ double rcp_seed(double d)
 {
 #ifdef __CUDA_ARCH__
@@ -70,7 +74,7 @@ __host__ __device__ __forceinline__ double rcp_seed(double d)
     const double r = 1.0 / d;
     unsigned long long u;
     std::memcpy(&u, &r, sizeof u);
-    u &= 0xffffffff00000000ull;  // the hardware's result has a zero low word
+    u &= 0xffffffff00000000ull;
     double s;
     std::memcpy(&s, &u, sizeof s);
     return s;
@@ -93,13 +97,11 @@ struct Rcp {
     double d, r, e;
 };
 
-__host__ __device__ __forceinline__ double rcp_fast(double d)
-{
-    const double s = rcp_seed(d);
-    const double h = fma_rn(-d, s, 1.0);
-    const double r = fma_rn(s, fma_rn(h, h, h), s);
-    return fma_rn(r, fma_rn(-d, r, 1.0), r);
-}
+// 1/d from the approximation r, its error squared.
+__host__ __device__ __forceinline__ double newton(double d, double r) { return fma_rn(r, fma_rn(-d, r, 1.0), r); }
+// RN(1/d) from a seed within 2^-14 of it.
+__host__ __device__ __forceinline__ double rcp_from(double d, double seed) { return newton(d, newton(d, newton(d, seed))); }
+__host__ __device__ __forceinline__ double rcp_fast(double d) { return rcp_from(d, rcp_seed(d)); }
 __host__ __device__ __forceinline__ Rcp rcp_with(double d, double r)
 {
     Rcp R;
