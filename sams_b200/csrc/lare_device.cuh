@@ -215,32 +215,32 @@ struct IeeeDiv {
     struct R {
         double d;
     };
-    __device__ __forceinline__ R of(double d) { return R{d}; }
-    __device__ __forceinline__ double operator()(double x, const R &r) { return x / r.d; }
-    __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q) { return x / r.d + y / q.d; }
-    __device__ __forceinline__ double fraction(double x, const R &r) { return x / r.d; }
-    __device__ __forceinline__ void finite(double) {}
+    __host__ __device__ __forceinline__ R of(double d) { return R{d}; }
+    __host__ __device__ __forceinline__ double operator()(double x, const R &r) { return x / r.d; }
+    __host__ __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q) { return x / r.d + y / q.d; }
+    __host__ __device__ __forceinline__ double fraction(double x, const R &r) { return x / r.d; }
+    __host__ __device__ __forceinline__ void finite(double) {}
 };
 struct FastDiv {
     static constexpr bool kFast = true;
     bool bad = false;
     using R = Rcp;
-    __device__ __forceinline__ R of(double d)
+    __host__ __device__ __forceinline__ R of(double d)
     {
-        bad = bad || !plain_divisor(d);
+        bad = bad || !usable_divisor(d);
         return rcp_of(d);
     }
-    __device__ __forceinline__ double operator()(double x, const R &r) { return quot_check(x, r, bad); }
-    __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q)
+    __host__ __device__ __forceinline__ double operator()(double x, const R &r) { return quot_check(x, r, bad); }
+    __host__ __device__ __forceinline__ double pair(double x, const R &r, double y, const R &q)
     {
         const double s = quot(x, r) + quot(y, q);
         const bool zero = ((high_word(x) << 1) | low_word(x) | (high_word(y) << 1) | low_word(y)) == 0;
         bad = bad || (!quot_in_range(s) && !zero);
         return s;
     }
-    __device__ __forceinline__ double fraction(double x, const R &r) { return quot(x, r); }
+    __host__ __device__ __forceinline__ double fraction(double x, const R &r) { return quot(x, r); }
     // (an infinity or NaN out of fraction() is left to the IEEE run)
-    __device__ __forceinline__ void finite(double q) { bad = bad || (high_word(q) & 0x7fffffffu) >= 0x7ff00000u; }
+    __host__ __device__ __forceinline__ void finite(double q) { bad = bad || (high_word(q) & 0x7fffffffu) >= 0x7ff00000u; }
 };
 
 // A denominator made of spacings: on power-of-two grids (P2) the product with
