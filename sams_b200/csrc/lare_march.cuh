@@ -646,6 +646,7 @@ __device__ __forceinline__ void zsweep(const Ctx &c, int b, int ct_arg, double *
 {
     using F = ops::SweepFused<2>;
     static_assert(!F::kSharedFluxSlots, "the z passes of stage B run without a barrier between them");
+    static_assert(std::is_same<typename F::EnergyIn, const double *>::value, "arrays written in place are not read as RO");
     const Geom &g = c.g;
     const int W = g.nz + 4, lines = kZThreads / W, S = lines * W;
     const int line = (int)threadIdx.x / W, k = (int)threadIdx.x % W - 2;

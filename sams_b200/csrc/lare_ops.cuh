@@ -1359,11 +1359,9 @@ struct CarryFace {
         F.bu = bu.d;
         dmu = mass_fraction<ZFORM>(dv, dm, bu, pick(up, ri, rp));
     }
-    __device__ __forceinline__ double carry(DV &dv, const double *f, int o, int d) const
-    {
-        return carried(dv, F, __ldg(f + o - d), __ldg(f + o), __ldg(f + o + d), __ldg(f + o + 2 * d), dmu);
-    }
-    __device__ __forceinline__ double carry_coherent(DV &dv, const double *f, int o, int d) const
+    // f: RO where no thread of the kernel writes the array, else a plain pointer
+    template <class A>
+    __device__ __forceinline__ double carry(DV &dv, const A &f, int o, int d) const
     {
         return carried(dv, F, f[o - d], f[o], f[o + d], f[o + 2 * d], dmu);
     }
@@ -1402,8 +1400,8 @@ struct SweepS6 {
             CarryFace<IeeeDiv> F;
             F.set<false>(dv, v >= 0.0, v * dt * area, cvc1[o], cvc1[o - d], cvc1[o + d], cv1[o], cv1[o + d], rho1[o],
                          rho1[o + d], dm[o]);
-            c.s[S_R_FE1][o] = F.carry(dv, c.f[SAMS_F_ENERGY_ELECTRON], o, d) * dm[o];
-            c.s[S_R_FE2][o] = F.carry(dv, c.f[SAMS_F_ENERGY_ION], o, d) * dm[o];
+            c.s[S_R_FE1][o] = F.carry(dv, RO{c.f[SAMS_F_ENERGY_ELECTRON]}, o, d) * dm[o];
+            c.s[S_R_FE2][o] = F.carry(dv, RO{c.f[SAMS_F_ENERGY_ION]}, o, d) * dm[o];
             // node cv2 (0..n)^3
             c.s[S_R_CV2N][o] = (cv2[o] + cv2[o + SX] + cv2[o + SY] + cv2[o + SX + SY] +
                                 cv2[o + 1] + cv2[o + SX + 1] + cv2[o + SY + 1] + cv2[o + SX + SY + 1]) * 0.125;
@@ -1460,8 +1458,8 @@ struct SweepS7 {
         CarryFace<IeeeDiv> F;
         const double o_v = v * dt * area;
         F.set<DIR == 2>(dv, o_v >= 0.0, o_v, cv1[o + d], cv1[o], cv1[o + 2 * d], cvc1[o], cvc1[o + d], rv[o], rv[o + d], dmv);
-        const double f1 = F.carry(dv, c.f[SAMS_F_VX], o, d), f2 = F.carry(dv, c.f[SAMS_F_VY], o, d),
-                     f3 = F.carry(dv, c.f[SAMS_F_VZ], o, d);
+        const double f1 = F.carry(dv, RO{c.f[SAMS_F_VX]}, o, d), f2 = F.carry(dv, RO{c.f[SAMS_F_VY]}, o, d),
+                     f3 = F.carry(dv, RO{c.f[SAMS_F_VZ]}, o, d);
         // with the rke correction the flux is kept as is (its kinetic-energy
         // error needs it) and SweepS8 takes the product with dm
         const bool raw = c.p.rke != 0;
@@ -1574,6 +1572,9 @@ struct SweepFused {
     // faster than five).
     enum { FE1, FE2, RVN, DMN, FM3, FM1 = DIR == 2 ? 5 : FE1, FM2 = DIR == 2 ? 6 : FE2, NARR = DIR == 2 ? 7 : 5 };
     static constexpr bool kSharedFluxSlots = DIR != 2;
+    // The energies that stage A reads: the z stages write them in the same
+    // kernel, so their loads are coherent ones; out of place they are only read.
+    using EnergyIn = typename std::conditional<DIR == 2, const double *, RO>::type;
 
     // SweepS6 at (i, j, k), sweep index -2..n+1.
     template <bool GEO, class A>
@@ -1601,16 +1602,14 @@ struct SweepFused {
         const RO dm{c.f[SAMS_F_DM]};
         const int nd = DIR == 0 ? g.nx : (DIR == 1 ? g.ny : g.nz);
         const int qd = DIR == 0 ? i : (DIR == 1 ? j : k);
-        if (own && i >= 1 && j >= 1 && k >= 1 && i <= g.nx && j <= g.ny && k <= g.nz)
-            w.rho[o] = dv(rho1[o] * cv1[o] + dm[o - d] - dm[o], dv.of(cv2[o]));
         if (qd >= 0 && qd <= nd) {  // the lines are 0..n across the sweep
             double v = face_velocity<DIR>(c, o);
             double area = face_area<DIR, GEO>(c, i, j, k);
             CarryFace<DV> F;
             F.template set<false>(dv, v >= 0.0, v * dt * area, cvc1[o], cvc1[o - d], cvc1[o + d], cv1[o], cv1[o + d], rho1[o],
                                   rho1[o + d], dm[o]);
-            b.put(FE1, F.carry(dv, c.f[SAMS_F_ENERGY_ELECTRON], o, d) * dm[o]);
-            b.put(FE2, F.carry(dv, c.f[SAMS_F_ENERGY_ION], o, d) * dm[o]);
+            b.put(FE1, F.carry(dv, EnergyIn{c.f[SAMS_F_ENERGY_ELECTRON]}, o, d) * dm[o]);
+            b.put(FE2, F.carry(dv, EnergyIn{c.f[SAMS_F_ENERGY_ION]}, o, d) * dm[o]);
         }
         if (qd >= -1) {
             double sum = rho1[o] * cv1[o] + rho1[o + SX] * cv1[o + SX] + rho1[o + SY] * cv1[o + SY] +
@@ -1623,6 +1622,9 @@ struct SweepFused {
         if (qd >= -1 && qd <= nd)
             b.put(DMN, (dm[o] + dm[o + SX] + dm[o + SY] + dm[o + SX + SY] + dm[o + 1] + dm[o + SX + 1] +
                         dm[o + SY + 1] + dm[o + SX + SY + 1]) * 0.125);
+        // (last: no load of an energy waits for this store)
+        if (own && i >= 1 && j >= 1 && k >= 1 && i <= g.nx && j <= g.ny && k <= g.nz)
+            w.rho[o] = dv(rho1[o] * cv1[o] + dm[o - d] - dm[o], dv.of(cv2[o]));
     }
 
     // SweepS7 at (i, j, k), first pass: the energy updates at the own points
@@ -1680,8 +1682,8 @@ struct SweepFused {
         const double o_v = v * dt * area;
         F.template set<DIR == 2>(dv, o_v >= 0.0, o_v, cv1[o + d], cv1[o], cv1[o + 2 * d], cvc1[o], cvc1[o + d], b.get(RVN, 0),
                                  b.get(RVN, 1), dmv);
-        const double f1 = F.carry_coherent(dv, c.f[SAMS_F_VX], o, d), f2 = F.carry_coherent(dv, c.f[SAMS_F_VY], o, d),
-                     f3 = F.carry_coherent(dv, c.f[SAMS_F_VZ], o, d);
+        const double *vx = c.f[SAMS_F_VX], *vy = c.f[SAMS_F_VY], *vz = c.f[SAMS_F_VZ];
+        const double f1 = F.carry(dv, vx, o, d), f2 = F.carry(dv, vy, o, d), f3 = F.carry(dv, vz, o, d);
         b.put(FM1, f1 * dmv);
         b.put(FM2, f2 * dmv);
         b.put(FM3, f3 * dmv);
