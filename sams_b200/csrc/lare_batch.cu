@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(kT, (MinBlocksBatch<Op, P2>::value))
 }
 
 template <bool GEO, bool P2>
-__global__ void __launch_bounds__(kT, 4)  // the split work at 4 blocks per SM, as k_visc_split
+__global__ void __launch_bounds__(kT, 4)  // tuned on n x n x 4 solves; k_visc_split has 3
     kb_visc(const Ctx *__restrict__ ctxs, const Tile *__restrict__ tiles, int ntiles, int tile_i)
 {
     __shared__ Ctx c;
@@ -148,12 +148,12 @@ __device__ __forceinline__ void for_blocks(const Ctx *ctxs, const SolveTiles *st
 
 #define KB_ARGS const Ctx *__restrict__ ctxs, const SolveTiles *__restrict__ st, const BlockRef *__restrict__ blocks, int n
 
-template <class P, int WHICH, bool GEO, bool P2>
+template <class P, bool GEO, bool P2>
 __global__ void __launch_bounds__(march::kMThreads, P::kMinBlocks) kb_cellnode(KB_ARGS, int arg)
 {
     extern __shared__ double ring[];
     for_blocks(ctxs, st, blocks, n, [&](const Ctx &c, const SolveTiles &t, int b) {
-        march::cellnode<P, GEO, P2>(c, t.cellnode[WHICH], b, arg >= 0 ? arg : c.p.resistive, ring);
+        march::cellnode<P, GEO, P2>(c, t.cellnode, b, arg >= 0 ? arg : c.p.resistive, ring);
     });
 }
 
@@ -617,7 +617,7 @@ static SolveTiles solve_tiles(const BatchSlot &s, double share, int sm_count)
     SolveTiles t{};
     const Geom &g = s.ctx.g;
     auto sm = [&](int per_sm) { return std::max(1, (int)(share * per_sm * sm_count)); };
-    t.cellnode[0] = march::march_tile(g.nz + 3, g.ny + 3, g.nx + 3, sm(march::PrepMarch::kMinBlocks));
+    t.cellnode = march::march_tile(g.nz + 3, g.ny + 3, g.nx + 3, sm(march::PrepMarch::kMinBlocks));
     t.pred = march::march_tile(g.nz + 1, g.ny + 1, g.nx + 1, sm(3));
     t.heat = march::march_tile(g.nz + 2, g.ny + 2, g.nx + 2, sm(march::kHeatMinBlocks));
     t.resist = march::march_tile(g.nz + 5, g.ny + 5, g.nx + 5, sm(5));
@@ -750,7 +750,7 @@ int Batch::rebuild()
         auto blocks = [&](int phase, long long n) {
             for (long long b = 0; b < n; ++b) lists[phase].push_back(BlockRef{(int)q, (int)b});
         };
-        blocks(P_CELLNODE, t.cellnode[0].blocks);
+        blocks(P_CELLNODE, t.cellnode.blocks);
         if (s.ctx.p.resistive) blocks(P_RESIST, t.resist.blocks);
         blocks(P_PRED, t.pred.blocks);
         blocks(P_HEAT, t.heat.blocks);
@@ -858,9 +858,9 @@ void Batch::launch_cellnode(int ctx, int arg)
 {
     const int ph = P_CELLNODE;
     const size_t smem = P::NR * kPlaneBytes;
-    if (has_geo_) { FUSED_LAUNCH((kb_cellnode<P, 0, true, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
-    else if (all_pow2_) { FUSED_LAUNCH((kb_cellnode<P, 0, false, true>), P::kMinBlocks, march::kMThreads, smem, arg); }
-    else { FUSED_LAUNCH((kb_cellnode<P, 0, false, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
+    if (has_geo_) { FUSED_LAUNCH((kb_cellnode<P, true, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
+    else if (all_pow2_) { FUSED_LAUNCH((kb_cellnode<P, false, true>), P::kMinBlocks, march::kMThreads, smem, arg); }
+    else { FUSED_LAUNCH((kb_cellnode<P, false, false>), P::kMinBlocks, march::kMThreads, smem, arg); }
 }
 
 void Batch::launch_resist(int ctx)

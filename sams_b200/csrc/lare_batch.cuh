@@ -1,8 +1,9 @@
 // lare_batch.cuh -- many independent LARE3D solves stepped together.
 //
-// Every phase of the step is ONE persistent launch over a worklist of tiles
-// drawn from all live solves (a tile = one solve, a slab of tile_i planes
-// along x, one chunk of 256 points of the (y, z) plane).  Each solve keeps its
+// Every phase of the step is ONE persistent launch over a worklist drawn from
+// all live solves: the blocks of each solve's own tiling (the fused phases), or
+// tiles of one solve, a slab of tile_i planes along x and a chunk of 256 points
+// of the (y, z) plane (the per-point phases).  Each solve keeps its
 // own state, scratch, metrics and device scalars, so each advances with its
 // own CFL timestep; the batch shares only the launches.  The whole batched
 // step is recorded once into a CUDA graph and replayed until the set of
@@ -36,7 +37,7 @@ struct BlockRef {
 
 // One solve's tilings of the fused phases and how its ghosts are filled.
 struct SolveTiles {
-    march::MarchTile cellnode[1], pred, heat, resist;
+    march::MarchTile cellnode, pred, heat, resist;
     march::WinTile ct[2], stage[2];
     march::ZTile ctz;
     int images[3];              // what the CT + mass kernels write of dm's ghosts, per sweep

@@ -147,13 +147,6 @@ enum ScratchId {
     S_CV1, S_B1X, S_B1Y, S_B1Z, S_PE, S_PI, S_FX, S_FY, S_FZ,
     NSCRATCH
 };
-// Resistive sub-step aliases (live between the CFL reduction and the
-// predictor, when cs, cs_v, cv1 and fx are free; pe holds the cell
-// electron pressure from before the Ohmic heating).
-#define S_FLUXX S_CS
-#define S_FLUXY S_CSV
-#define S_FLUXZ S_CV1
-#define S_CURLB S_FX
 // Remap aliases (the whole Lagrangian scratch is dead by then).
 #define S_R_CV1 S_CV1
 #define S_R_CV2 S_CS
@@ -210,7 +203,6 @@ struct RO {
 // 866 / 52 -> 767 / 48, corrector 597 / 38 -> 540 / 32; k_visc_split
 // (three blocks per SM) 1090 / 86 -> 1040 / 73.
 struct IeeeDiv {
-    static constexpr bool kFast = false;
     static constexpr bool bad = false;
     struct R {
         double d;
@@ -222,7 +214,6 @@ struct IeeeDiv {
     __host__ __device__ __forceinline__ void finite(double) {}
 };
 struct FastDiv {
-    static constexpr bool kFast = true;
     bool bad = false;
     using R = Rcp;
     __host__ __device__ __forceinline__ R of(double d)

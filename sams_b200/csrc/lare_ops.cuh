@@ -253,19 +253,21 @@ struct Alpha {
 
 // Viscous pressure and heating on cells, viscous forces on nodes and the
 // cell's CFL candidate (p_visc is consumed here and never stored).
-// Returns the candidate (DBL_MAX outside the CFL range).
 struct Visc {
     // (launched by k_visc_split and kb_visc, each with its own register cap)
     __host__ __device__ static void bounds(const Geom &g, int, int *lo, int *hi)
     {
         set_bounds(lo, hi, 0, g.nx + 1, 0, g.ny + 1, 0, g.nz + 1);
     }
-    // The cell's work in two halves, which the single-solve kernel
-    // (k_visc_split) gives to different threads: heat_forces is the viscous
+    // The cell's work in two halves, which the kernels give to different
+    // threads: heat_forces is the viscous
     // heating of cell (i, j, k) (lagran.cpp:283-326) and the viscous forces
     // on node (i, j, k) (:329-376); cfl is the cell's viscous pressure
     // (:303-305, with the three edge jumps it needs formed again, the same
-    // expressions) and its CFL candidate (set_dt, :380-443).
+    // expressions) and its CFL candidate (set_dt, :380-443).  nonfinite is set
+    // when a NaN or infinity shows up in the cell's viscous pressure, heating or
+    // CFL terms (the solve's state is no longer finite; the min itself would
+    // hide it, as LARE's min does).
     template <bool GEO, bool P2>
     __device__ __forceinline__ static void heat_forces(const Ctx &c, int i, int j, int k, bool &nonfinite)
     {
@@ -325,7 +327,7 @@ struct Visc {
         const double cv = (GEO && c.p.geometry) ? cv_at<GEO>(c, i, j, k) : dx * (dyp * dzp);
         c.s[S_VH][o] = By<P2, DV>(dv, cv, c.rc.cv)(dv, vh);
         if (i > g.nx || j > g.ny || k > g.nz) return;
-        // checked where run checks it: the cells of the CFL range
+        // checked in the cells of the CFL range, as in cfl
         if (!(GEO && c.p.geometry && i < 1) && !(fabs(vh) <= DBL_MAX)) nonfinite = true;
         double e1 = a1a[o + SY + 1] * dy * dz;
         double e2 = a1a[o + SX + SY + 1] * dy * dz;
@@ -425,16 +427,6 @@ struct Visc {
         const double chk = dt1 + dt2 + dt3 + dt4 + p_visc;
         if (!(fabs(chk) <= DBL_MAX)) nonfinite = true;
         return pmin(pmin(pmin(dt1, dt2), dt3), dt4);
-    }
-    // nonfinite is set when a NaN or infinity shows up in this cell's viscous
-    // pressure, heating or CFL terms (the solve's state is no longer finite;
-    // the min itself would hide it, as LARE's min does).
-    template <bool GEO, bool P2>
-    __device__ static double run(const Ctx &c, int, int i, int j, int k, bool &nonfinite)
-    {
-        heat_forces<GEO, P2>(c, i, j, k, nonfinite);
-        if (i > c.g.nx || j > c.g.ny || k > c.g.nz) return DBL_MAX;
-        return cfl<GEO, P2>(c, i, j, k, nonfinite);
     }
 };
 
@@ -846,7 +838,7 @@ struct Corr1 {
                     (vz[a] - vz[b]) * (vz1[a] - vz1[b]));
     }
     // The products of the x, y and z edges that end at node o, formed once
-    // per node by the marching kernel (k_edge_march).
+    // per node by the marching kernel (k_heat_march).
     __device__ __forceinline__ static void node_edges(const Ctx &c, int o, double *e)
     {
         e[0] = dd(c, o - c.g.sx, o);

@@ -116,7 +116,8 @@ private:
     void launch_heat();
     void launch_pred(int resistive);
     void launch_resist(bool last);
-    // true when the kernel also wrote dm's periodic ghost images along DIR
+    // true when the kernel also wrote dm's ghosts along DIR (periodic or
+    // zero-gradient ones)
     template <int DIR> bool launch_ctmass(int scale);
     int staging(double **out);
     void free_all();
