@@ -6,8 +6,8 @@
 //   1. admit queued requests in arrival order while their device footprint
 //      fits the budget and, when a cap is set, the interior cells of the
 //      running solves stay under it (allocate, upload the initial state);
-//   2. advance every running solve by one step: solves with long z lines
-//      (Solver::fused_path) each launch their own step graph on their own
+//   2. advance every running solve by one step: some, by the length of their
+//      z lines (Solver::own_stream), each launch their own step graph on their own
 //      stream, and all other solves advance together by one batched
 //      step (one graph launch; re-recorded when that set changes), on one
 //      more stream, so the steps of all running solves overlap on the GPU;
@@ -51,8 +51,8 @@ struct Request {
     int64_t done = 0;
     long long cells = 0;
     int slot = -1;                          // batch slot (batched solves)
-    std::unique_ptr<sams::Solver> solo;     // own solver (Solver::fused_path)
-    bool fused = false;
+    std::unique_ptr<sams::Solver> solo;     // own solver (Solver::own_stream)
+    bool own_stream = false;
     int status = SAMS_SERVE_QUEUED;
     bool cancel = false;  // set by sams_lare_serve_cancel while running
     long long bytes = 0;
@@ -97,7 +97,7 @@ struct sams_lare_server {
 int sams_lare_server::admit_one(Request *r)
 {
     int rc;
-    if (r->fused) {
+    if (r->own_stream) {
         r->solo.reset(new (std::nothrow) sams::Solver());
         if (!r->solo) return SAMS_ERR_NOMEM;
         rc = r->solo->init(r->p, r->bcs, device);
@@ -328,8 +328,8 @@ int sams_lare_serve_submit(sams_lare_server *s, const sams_lare_params *p, const
     for (int f = 0; f < SAMS_NFIELDS; ++f) r->ic[f] = ic[f];
     for (int q = 0; q < 9; ++q) r->out[q] = out ? out[q] : nullptr;
     r->nsteps = nsteps;
-    r->fused = sams::Solver::fused_path(*p);
-    r->bytes = r->fused ? sams::Solver::bytes_for(*p) : sams::Batch::bytes_for(*p);
+    r->own_stream = sams::Solver::own_stream(*p);
+    r->bytes = r->own_stream ? sams::Solver::bytes_for(*p) : sams::Batch::bytes_for(*p);
     r->cells = (long long)(p->nx * p->ny * p->nz);
     r->t_submit = Clock::now();
     std::lock_guard<std::mutex> lk(s->mu);
@@ -348,7 +348,7 @@ int sams_lare_serve_submit(sams_lare_server *s, const sams_lare_params *p, const
 int sams_lare_serve_solve_bytes(const sams_lare_params *p, int64_t *bytes)
 {
     if (!p || !bytes) return SAMS_ERR_INVALID;
-    *bytes = (int64_t)(sams::Solver::fused_path(*p) ? sams::Solver::bytes_for(*p) : sams::Batch::bytes_for(*p));
+    *bytes = (int64_t)(sams::Solver::own_stream(*p) ? sams::Solver::bytes_for(*p) : sams::Batch::bytes_for(*p));
     return SAMS_OK;
 }
 

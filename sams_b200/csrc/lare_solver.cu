@@ -298,7 +298,7 @@ long long Solver::bytes_for(const sams_lare_params &p)
     return (narr * nelem + staging + axes) * (long long)sizeof(double) + (long long)sizeof(Scalars) + 4096;
 }
 
-bool Solver::fused_path(const sams_lare_params &p) { return lanes_full(p.nz + 1, 31); }
+bool Solver::own_stream(const sams_lare_params &p) { return lanes_full(p.nz + 1, 31); }
 
 Solver::~Solver() { free_all(); }
 

@@ -59,10 +59,17 @@ public:
     // arrays, the host-transfer staging buffer, axes and metric tables (an
     // upper bound, for admission under a memory budget).
     static long long bytes_for(const sams_lare_params &p);
-    // Whether a server runs a solve of these parameters on a stream of its
-    // own (long z lines: large enough to fill much of the GPU) instead of in
-    // the batched step.
-    static bool fused_path(const sams_lare_params &p);
+    // Whether a server runs a solve of these parameters on a stream of its own
+    // instead of in the batched step: its nz + 1 nodes of a line fill at least
+    // three quarters of pieces of 31 (nz = 23..30, 46..61, 69 and up).  These
+    // were the z tiles of the marching kernels when the rule was made, and with
+    // it goes the footprint that sams_lare_serve_solve_bytes answers, so it has
+    // stayed while the tiles changed; nx and ny do not enter.  Time per step of
+    // solves on own streams over the same solves in one batched step: own side,
+    // six 60^3 0.84, four 96^3 0.84, two 128^3 0.78, but sixteen 16x16x24 1.59
+    // (one alone 0.79); batch side, eight 32^3 1.04, eight 40^3 0.98, four
+    // 256x256x4 1.13, but six 64^3 0.81, three 192x192x64 0.78.
+    static bool own_stream(const sams_lare_params &p);
     // One x slab of a larger grid: p.nx is the slab's own cell count, the
     // x axis and metric tables are those of the whole grid (slab.nx_global
     // cells over x_min..x_max) from the slab's offset on.

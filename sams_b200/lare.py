@@ -443,8 +443,8 @@ class Server:
     """Continuous-batching LARE3D server on one GPU (include/sams_lare.h,
     serving section).  Submitted solves are admitted as device memory within
     `budget_bytes` frees up, stepped together with every other running solve
-    (large ones on their own streams, small and thin ones in one batched
-    step), and their final state copied back when their step count is
+    (those with nz = 23..30, 46..61 or 69 and up on their own streams, the
+    others in one batched step), and their final state copied back when their step count is
     reached."""
 
     _prefix = "sams_lare_serve_"
