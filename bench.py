@@ -13,7 +13,8 @@ in HBM; `e2e` is the same solve through the C ABI from pinned host buffers
 every rank runs its own independent solve (replicas; the path does not shard
 within a solve), time = max over ranks.  `--impl reference` times the
 reference LARE3D CPU code (oracle/_ref/lare_ref_bench, built from the
-reference sources) on this host's cores for the same workload.
+reference sources) on this host's cores for the same workload, or says that
+it is unavailable where that build is not.
 """
 import argparse
 import json
@@ -256,6 +257,12 @@ def replica_throughput(world, cells, steps, ms):
 
 def run_reference_arm(args, world, rank):
     if rank != 0:
+        return
+    from oracle import lare_oracle as lo
+    if not os.path.exists(lo.reference_bench_binary()[0]):
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's CPU build (oracle/_ref/lare_ref_bench) is not here: "
+                                         "it is made from the reference's sources"}), flush=True)
         return
     w = workload(args)
     total = args.warmup + args.steps
