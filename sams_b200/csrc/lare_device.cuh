@@ -201,7 +201,8 @@ struct RO {
 // predictor 1451 / 154 -> 1233 / 129, x stages 1239 / 85 -> 1051 / 71, y stages
 // 1367 / 93 -> 1198 / 81, z stages 1367 / 116 -> 1257 / 86, edge viscosity
 // 866 / 52 -> 767 / 48, corrector 597 / 38 -> 540 / 32; k_visc_split
-// (three blocks per SM) 1090 / 86 -> 1040 / 73.
+// (three blocks per SM) 1090 / 86 -> 1040 / 73.  (The reciprocal's third Newton
+// step, added since, costs up to 2% of a kernel: predictor 1248 at 256^3.)
 struct IeeeDiv {
     static constexpr bool bad = false;
     struct R {
