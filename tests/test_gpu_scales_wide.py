@@ -1,5 +1,5 @@
 """Cell volumes and masses beyond the whole range of the branch-free division
-(2^-240..2^240, lare_div.cuh): its fall-back gives the checker's bits, as do
+(2^-240..2^240, lare_div.cuh): its fall-back gives the oracle's bits, as do
 scales that it takes on the straight path."""
 import pytest
 
@@ -21,5 +21,5 @@ def _thinnest_density(F, rng):
     ("rf", (9, 10, 11), 1.0, _thinnest_density),
 ])
 @pytest.mark.parametrize("batched", [False, True])
-def test_far_scales_match_checker(case, n, scale, change, batched, oracle_lib):
+def test_far_scales_match_oracle(case, n, scale, change, batched, oracle_lib):
     scales.test_fallback_matches_checker(case, n, scale, change, batched, oracle_lib)
